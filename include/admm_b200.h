@@ -112,7 +112,10 @@ typedef struct AdmmB200Desc {
      * through per-block sweep counters (falls back to 1 when the device cannot
      * hold all blocks at once or jacobi_iter < 2); 3 = two sweeps per launch,
      * one block per spatially compact tile of rows, the halo rows computed
-     * into shared memory.  All give identical bits. */
+     * into shared memory.  With 0, scenes whose matrix fits the shared memory of
+     * thread-block clusters and for which it is expected to be faster keep it there:
+     * one kernel for all sweeps (or all PCG iterations) of a global step, chosen by a
+     * rule on sizes.  All give identical bits (PCG: up to the order of its FP64 sums). */
     int32_t jacobi_mode;
     /* Broad phase of the DCD: 0 = default (2); 1 = LBVH (the reference's
      * structure, bvh_refit applies); 2 = uniform-grid spatial hash.  Both report
@@ -377,7 +380,8 @@ int  admm_b200_kernels_fallback(AdmmB200* h, int* n);
  * row-major nd x 3).  The substep counts as a step of the simulation. */
 int  admm_b200_record_global(AdmmB200* h, int iteration, float* b, float* x_cur, float* x_last, int nd);
 /* How the global step runs (jacobi_mode): persistent = 1 for the one-kernel
- * global step (blocks = its grid), 3 for two sweeps per launch over row tiles,
+ * global step (blocks = its grid), 3 for two sweeps per launch over row tiles, 4 for
+ * all sweeps in one launch with the matrix in shared memory (blocks = its grid),
  * 0 for one kernel per sweep; the autotuner's ms per global step with one
  * kernel per sweep and with the persistent kernel (0 when not timed). */
 int  admm_b200_global_mode(AdmmB200* h, int* persistent, int* blocks, float* ms_sweeps, float* ms_persist);

@@ -26,6 +26,7 @@
 #include "kernels.cuh"
 #include "lbvh.cuh"
 #include "learn.cuh"
+#include "resident.cuh"
 #include "scan_sort.cuh"
 #include "setup.hpp"
 
@@ -115,6 +116,10 @@ struct AdmmB200 {
     bool tiled = false;             // chosen mode: two sweeps per launch over row tiles
     TileSet ts;
     int tile_smem = 0;
+    // the global step resident in shared memory (resident.cuh), where the scene fits
+    ResidentDev res;
+    bool resident = false;
+    int res_smem = 0;               // dynamic shared memory of its kernels
     HostCsr hostA;                  // the global matrix on the host (admm_b200_system)
     std::vector<float> hostAdiag;
     float tune_ms_tiled = 0.f;
@@ -516,11 +521,95 @@ void launch_persist(AdmmB200* h, bool rhs, bool save_prev, int sweeps) {
     h->launch_counter++;
 }
 
+// The instantiation of a resident kernel for the plan's thread layout (fn: a macro of Q, TP, CLUSTER).
+#define RESIDENT_TP(fn, cl)                                                     \
+    switch (p.q * 16 + p.tp) {                                                  \
+        case 1 * 16 + 1: k = fn(1, 1, cl); break;                               \
+        case 1 * 16 + 2: k = fn(1, 2, cl); break;                               \
+        case 1 * 16 + 4: k = fn(1, 4, cl); break;                               \
+        case 1 * 16 + 8: k = fn(1, 8, cl); break;                               \
+        case 2 * 16 + 1: k = fn(2, 1, cl); break;                               \
+        case 2 * 16 + 2: k = fn(2, 2, cl); break;                               \
+        case 2 * 16 + 4: k = fn(2, 4, cl); break;                               \
+        case 4 * 16 + 1: k = fn(4, 1, cl); break;                               \
+        case 4 * 16 + 2: k = fn(4, 2, cl); break;                               \
+        default: k = fn(8, 1, cl); break;                                       \
+    }
+#define RESIDENT_PICK(fn)                  \
+    if (p.cluster > 1) {                   \
+        RESIDENT_TP(fn, true)              \
+    } else {                               \
+        RESIDENT_TP(fn, false)             \
+    }
+
+typedef void (*ResidentJacobiFn)(DevScene, ResidentDev, int);
+typedef void (*ResidentPcgFn)(DevScene, ResidentDev, PcgDev, int);
+typedef void (*ResidentLearnedFn)(DevScene, ResidentDev, LearnDev, const float4*, LearnCoef, int, int);
+
+ResidentJacobiFn resident_jacobi_fn(const ResidentDev& p) {
+    ResidentJacobiFn k = nullptr;
+#define FN(Q, TP, CL) k_resident_jacobi<Q, TP, CL>
+    RESIDENT_PICK(FN)
+#undef FN
+    return k;
+}
+
+ResidentPcgFn resident_pcg_fn(const ResidentDev& p) {
+    ResidentPcgFn k = nullptr;
+#define FN(Q, TP, CL) k_resident_pcg<Q, TP, CL>
+    RESIDENT_PICK(FN)
+#undef FN
+    return k;
+}
+
+ResidentLearnedFn resident_learned_fn(const ResidentDev& p) {
+    ResidentLearnedFn k = nullptr;
+#define FN(Q, TP, CL) k_resident_learned<Q, TP, CL>
+    RESIDENT_PICK(FN)
+#undef FN
+    return k;
+}
+
+// One launch of a resident kernel: its clusters, with programmatic dependent launch.
+template <typename... KArgs, typename... Args>
+void launch_resident(AdmmB200* h, void (*k)(KArgs...), int smem, Args&&... args) {
+    const ResidentDev& p = h->res;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.groups * p.cluster);
+    cfg.blockDim = dim3(p.threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->cstream;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (p.cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = p.cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (h->pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    LaunchTimer lt_(h, ADMM_KERNEL_JACOBI);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k, std::forward<Args>(args)...);
+    if (e != cudaSuccess && h->enqueue_rc == ADMM_OK)
+        h->enqueue_rc = fail(h, ADMM_ERR_CUDA, std::string("resident global step: ") + cudaGetErrorString(e));
+    h->launch_counter++;
+}
+
 void enqueue_jacobi(AdmmB200* h, int sweeps) {
     DevScene& s = h->s;
     const int vb = blocks(s.nd, kVertThreads);
     set_phase(h, ADMM_PHASE_JACOBI);
     if (sweeps <= 0) return;
+    if (h->resident && sweeps >= 2) {
+        launch_resident(h, resident_jacobi_fn(h->res), h->res_smem, s, h->res, sweeps);
+        return;
+    }
     if (h->persist && sweeps >= 2) {
         launch_persist(h, false, false, sweeps);
         return;
@@ -560,6 +649,10 @@ void enqueue_pcg(AdmmB200* h, int iters) {
     const int ga = blocks(s.A.nslices * 32, kVertThreads), gv = blocks(s.nd, kVertThreads);
     PcgDev& g = h->pcg;
     g.block = (h->global_solver == 2 && h->pcg_blocks) ? h->pcg_blocks : nullptr;
+    if (h->resident) {
+        launch_resident(h, resident_pcg_fn(h->res), h->res_smem, s, h->res, g, iters);
+        return;
+    }
 #define PCG_T(T)                                                                        \
     do {                                                                                \
         LAUNCH(k_pcg_init<T>, ga, kVertThreads, s, g);                                  \
@@ -605,7 +698,8 @@ void enqueue_learned_replacement(AdmmB200* h) {
 // condition (inside the residual-tolerance WHILE body the IF node is nested in it);
 // eagerly, the host reads the decision (one stream synchronisation per solve).
 void enqueue_learned_decide(AdmmB200* h, bool first) {
-    LearnDev& L = h->learn;
+    LearnDev L = h->learn;
+    if (h->resident) L.blocks = h->res.groups * h->res.cluster;  // its partials, one per CTA
     const int fi = first ? 1 : 0;
     cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
     cudaGraph_t g = nullptr;
@@ -685,6 +779,18 @@ void enqueue_learned(AdmmB200* h, bool save_prev, bool first) {
     }
 #undef RHSL_CASE
     set_phase(h, ADMM_PHASE_JACOBI);
+    if (h->resident) {
+        LearnCoef cf = {};
+        for (int k = 0; k < K; k++) {
+            cf.omega[k] = h->learn_omega[k];
+            cf.beta[k] = h->learn_beta[k];
+        }
+        LearnDev lr = L;
+        lr.blocks = h->res.groups * h->res.cluster;
+        launch_resident(h, resident_learned_fn(h->res), h->res_smem, s, h->res, lr, (const float4*)buf[s0], cf, K, ex);
+        enqueue_learned_decide(h, first);
+        return;
+    }
 #define LS_CASE(T)                                                                                         \
     for (int k = 0; k < K; k++) {                                                                          \
         const float4* src = buf[(s0 + k) % 3];                                                             \
@@ -855,6 +961,104 @@ int build_tiles_dev(AdmmB200* h, const HostCsr& A) {
         CK(cudaFuncSetAttribute(k_jacobi2<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
         CK(cudaFuncSetAttribute(k_jacobi2<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
         CK(cudaFuncSetAttribute(k_jacobi2<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    }
+    return ADMM_OK;
+}
+
+// Clusters of `size` CTAs with one CTA per SM that the device runs at once (7 of 16, 15 of 8, 33
+// of 4, 74 of 2 on a B200 with 148 SMs: a cluster lies within one GPC).
+int active_clusters(const void* kernel, int size, int smem, int* n) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(size);
+    cfg.blockDim = dim3(kResidentThreads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    *n = 0;
+    if (cudaOccupancyMaxActiveClusters(n, kernel, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        *n = 0;
+    }
+    return ADMM_OK;
+}
+
+// The resident plan (resident.hpp) for the lanes A was tuned to, where it is expected to beat a
+// launch per sweep.  Measured on a B200 (us per sweep of a substep's global step): resident
+// 0.85 + 2.2e-4 per entry of the largest CTA (32^2 cloth on 16 CTAs, 1536 entries: 1.2; 24 bodies
+// of 118 k rows on 7 x 16 CTAs, 14.7 k entries: 4.5; cube 20^3 on 16 CTAs, 8.1 k entries: 2.9; two
+// 128^2 sheets on 2 x 16, 18.6 k entries: 4.2); a launch per sweep 2.2 + 2.8e-6 per entry of A (2.3,
+// 5.9, 2.5 and 3.5 for the same scenes), an iteration of PCG 7.3 in two launches.  So the cloth
+// and the bodies run resident (within 10% the launches stay, which need no load of the plan, about
+// 5 us per global step), the cube and the sheets do not.
+int build_resident_plan(AdmmB200* h, const HostCsr& A, const std::vector<float>& diag) {
+    DevScene& s = h->s;
+    const bool pcg = h->global_solver == 1 || h->global_solver == 2;
+    const int passes = pcg ? h->pcg_iter : h->global_solver == 3 ? 8 : h->jac_iter;
+    if (s.nd <= 0 || passes < 2) return ADMM_OK;
+    const double nnz = (double)A.col.size(), launched = pcg ? 7.0 + 2.8e-6 * nnz : 2.2 + 2.8e-6 * nnz;
+    std::vector<float> pos(3 * (size_t)s.nd);
+    for (int i = 0; i < s.nd; i++) {
+        pos[3 * i] = h->x_init[i].x;
+        pos[3 * i + 1] = h->x_init[i].y;
+        pos[3 * i + 2] = h->x_init[i].z;
+    }
+    const ResidentOrder order = resident_order(A, s.nd, pos.data(), 3);
+    int smem_max = 0;
+    CK(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+    smem_max -= 2048;  // the kernels' static shared memory
+    struct Choice {
+        double us;
+        int cluster, groups;
+    };
+    std::vector<Choice> choices;
+    ResidentDev& p = h->res;
+    for (int c : {1, 2, 4, 8, 16}) {
+        p = ResidentDev{};
+        p.cluster = c;
+        p.q = s.A.lanes;
+        p.tp = 1;
+        const void* k = (const void*)resident_jacobi_fn(p);
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+        if (c > 8) CK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        int active = 0;
+        TRY(active_clusters(k, c, smem_max, &active));
+        if (active <= 0) continue;
+        const int groups = pcg ? 1 : std::min<int>((int)order.weight.size(), active);
+        const double us = 0.85 + 2.2e-4 * (double)resident_groups(order, groups) / c;
+        if (us * passes + 5.0 < 0.9 * launched * passes) choices.push_back({us, c, groups});
+    }
+    p = ResidentDev{};
+    std::sort(choices.begin(), choices.end(), [](const Choice& a, const Choice& b) { return a.us < b.us; });
+    for (const Choice& ch : choices) {
+        if ((double)order.total * 8.0 > (double)smem_max * ch.cluster * ch.groups) continue;  // cannot fit
+        const HostResident r = build_resident(A, diag, s.nd, s.A.lanes, order, ch.cluster, ch.groups);
+        const long long smem = resident_smem(r, 16 * (pcg ? kResidentPcgArrays : 2));
+        if (!r.ok || smem > smem_max) continue;
+        p.cluster = r.cluster;
+        p.groups = r.groups;
+        p.tp = r.tp;
+        p.q = r.q;
+        p.threads = r.threads;
+        p.max_own = (r.max_own + 3) / 4 * 4;
+        p.max_local = r.max_local;
+        ResidentCta* dc = nullptr;
+        unsigned char* db = nullptr;
+        TRY(dupload(h, &dc, r.cta.data(), r.cta.size()));
+        TRY(dupload(h, &db, r.blob.data(), r.blob.size()));
+        p.cta = dc;
+        p.blob = db;
+        h->res_smem = (int)smem;
+        for (const void* k : {(const void*)resident_jacobi_fn(p), (const void*)resident_learned_fn(p),
+                              (const void*)resident_pcg_fn(p)}) {
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+            if (p.cluster > 8) CK(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        }
+        h->resident = true;
+        return ADMM_OK;
     }
     return ADMM_OK;
 }
@@ -1653,6 +1857,7 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     if (d->pcg_iter < 0) return fail(h, ADMM_ERR_INVALID, "pcg_iter");
     h->global_solver = d->global_solver;
     h->pcg_iter = d->pcg_iter > 0 ? d->pcg_iter : std::max(1, d->jacobi_iter / 2);
+    if (d->jacobi_mode == 0) TRY(build_resident_plan(h, as.A, as.a_diag));
     {
         PcgDev& g = h->pcg;
         TRY(dalloc(h, &g.r, nd));
@@ -1680,8 +1885,9 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
         TRY(dalloc(h, &L.xl, nd));
         L.rblocks = blocks(s.R.nslices * 32, kVertThreads);
         TRY(dalloc(h, &L.ax, nd));
-        TRY(dalloc(h, &L.part, 3 * (size_t)L.blocks));
-        TRY(dalloc(h, &L.part_c, (size_t)L.blocks));
+        const size_t parts = std::max((size_t)L.blocks, (size_t)h->res.groups * h->res.cluster);
+        TRY(dalloc(h, &L.part, 3 * parts));
+        TRY(dalloc(h, &L.part_c, parts));
         TRY(dalloc(h, &L.stats, 4));
         TRY(dalloc(h, &L.fail, 1));
         TRY(dalloc(h, &L.warm, 1));
@@ -1692,10 +1898,10 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     }
     h->hostA = as.A;
     h->hostAdiag = as.a_diag;
-    TRY(build_persist_plan(h, as.A));
-    TRY(build_tiles_dev(h, as.A));
     h->persist = h->tiled = false;
-    if (h->jac_iter >= 2 && (d->global_solver == 0 || d->global_solver == 3)) {
+    if (!h->resident && h->jac_iter >= 2 && (d->global_solver == 0 || d->global_solver == 3)) {
+        if (d->jacobi_mode == 0 || d->jacobi_mode == 2) TRY(build_persist_plan(h, as.A));
+        if (d->jacobi_mode == 0 || d->jacobi_mode == 3) TRY(build_tiles_dev(h, as.A));
         if (d->jacobi_mode == 2 && h->persist_ok) {
             h->persist = true;
         } else if (d->jacobi_mode == 3) {
@@ -2600,8 +2806,8 @@ int admm_b200_record_global(AdmmB200* h, int iteration, float* b, float* x_cur, 
 
 int admm_b200_global_mode(AdmmB200* h, int* persistent, int* blocks, float* ms_sweeps, float* ms_persist) {
     if (!h) return ADMM_ERR_INVALID;
-    if (persistent) *persistent = h->persist ? 1 : h->tiled ? 3 : 0;
-    if (blocks) *blocks = h->persist ? h->pp.blocks : 0;
+    if (persistent) *persistent = h->resident ? 4 : h->persist ? 1 : h->tiled ? 3 : 0;
+    if (blocks) *blocks = h->resident ? h->res.groups * h->res.cluster : h->persist ? h->pp.blocks : 0;
     if (ms_sweeps) *ms_sweeps = h->tune_ms_sweeps;
     if (ms_persist) *ms_persist = h->tune_ms_persist;
     return ADMM_OK;

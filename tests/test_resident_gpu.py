@@ -1,0 +1,89 @@
+"""The global step resident in shared memory (csrc/resident.cuh) against the kernels it replaces
+(jacobi_mode 1: one kernel per sweep): the same bits for the Jacobi sweeps and the learned step,
+the same solution for conjugate gradients, whose FP64 sums are added in another order."""
+import numpy as np
+import pytest
+
+from parallel_admm_b200 import backend as B
+from parallel_admm_b200 import scene as S
+
+pytestmark = pytest.mark.gpu
+
+SCENES = {"cloth5": lambda: S.cloth_on_box(nx=5), "cloth33": lambda: S.cloth_on_box(nx=33),
+          "cloth46": lambda: S.cloth_on_box(nx=46), "cube3": lambda: S.cube_on_ground(n=3, drop=0.01),
+          "cube11": lambda: S.cube_on_ground(n=11, drop=0.01, rotate=True),
+          "bodies": lambda: S.batch_bodies(n_bodies=6, seed=3, vmax=3000)}
+
+
+def _pair(name, lanes, **kw):
+    sc = SCENES[name]()
+    hs = [B.Handle(sc, ell_lanes=lanes, jacobi_mode=m, **kw) for m in (1, 0)]
+    assert hs[0].global_mode()["mode"] == "sweeps"
+    assert hs[1].global_mode()["mode"] == "resident"
+    rng = np.random.default_rng(7)
+    x = sc.verts + rng.normal(scale=1e-3, size=sc.verts.shape).astype(np.float32)
+    v = rng.normal(scale=0.2, size=sc.verts.shape).astype(np.float32)
+    for h in hs:
+        h.set_state(x, v)
+    return hs
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("name", list(SCENES))
+def test_sweeps_bitwise(name, lanes):
+    a, b = _pair(name, lanes)
+    for h in (a, b):
+        h.pre_integration()
+        h.local_step()
+        h.global_step()
+    assert np.array_equal(a.read(B.BUF_X), b.read(B.BUF_X))
+    for sweeps in (1, 2, 3, 7):
+        a.jacobi(sweeps)
+        b.jacobi(sweeps)
+        assert np.array_equal(a.read(B.BUF_X), b.read(B.BUF_X)), sweeps
+
+
+@pytest.mark.parametrize("name", ["cloth33", "cube11", "bodies"])
+def test_substeps_bitwise(name):
+    a, b = _pair(name, 4)
+    for _ in range(4):
+        sa, sb = (h.step(1, allow=(B.ERR_CONTACT_OVERFLOW,)) for h in (a, b))
+        assert sa["n_contacts"] == sb["n_contacts"]
+        for p, q in zip(a.get_state(), b.get_state()):
+            assert np.array_equal(p, q)
+    assert b.kernels_per_step() < a.kernels_per_step()
+
+
+@pytest.mark.parametrize("tol", [0.0, 1e-4])
+@pytest.mark.parametrize("sweeps", [1, 5, 6, 7])
+def test_learned_bitwise(sweeps, tol):
+    # the schedule of sweep 6 steps backwards: its solves fail and are replaced
+    a, b = _pair("cloth33", 2, global_solver=3, residual_tol=tol)
+    omega = np.full(sweeps, -1.0 if sweeps == 6 else 0.9, np.float32)
+    beta = np.full(sweeps, 0.1, np.float32)
+    theta = np.full(a.n_dyn, 0.3, np.float32)
+    for h in (a, b):
+        h.set_learned(omega, beta, None, theta)
+    for _ in range(3):
+        for h in (a, b):
+            h.step(1, allow=(B.ERR_CONTACT_OVERFLOW,))
+        for p, q in zip(a.get_state(), b.get_state()):
+            assert np.array_equal(p, q)
+    assert a.learned_stats() == b.learned_stats()
+
+
+@pytest.mark.parametrize("name", ["cloth5", "cloth33", "cube11"])
+@pytest.mark.parametrize("solver", [1, 2])
+def test_pcg(name, solver):
+    a, b = _pair(name, 4, global_solver=solver, pcg_iter=25)
+    blocks = np.zeros((a.n_dyn, 9), np.float32)
+    blocks[:, [0, 4, 8]] = np.random.default_rng(2).uniform(0.5, 1.5, (a.n_dyn, 1)) / 10.0
+    blocks[:, [1, 3]] = 0.01
+    for h in (a, b):
+        if solver == 2:
+            h.set_preconditioner(blocks)
+        h.pre_integration()
+        h.local_step()
+        h.global_step()
+    x, y = a.read(B.BUF_X), b.read(B.BUF_X)
+    assert np.abs(x - y).max() <= 1e-5 * max(1.0, np.abs(x).max())
