@@ -5,13 +5,20 @@
 // counterpart; the network and loss are specified in the header of the CPU
 // restatement that the tests check these kernels against.
 //
-// Layout: every activation is a row-major FP32 matrix (rows = vertices or
-// directed edges of A's off-diagonal pattern, in CSR order).  Dense layers are
-// Z = X W^T + b with W row-major [out][in]; with bf16 set, the forward and
-// input-gradient passes use the weights rounded to BF16 (FP32 accumulation),
-// the master weights and Adam moments stay FP32.  Weight gradients are per-block
-// partial sums reduced in a fixed order, node sums over edges run in CSR order,
-// so a training step is deterministic.
+// Layout: every activation is a row-major FP32 matrix with a row per vertex; nothing of a
+// message's width is kept per edge but one bit per channel.  An edge layer
+// W [h_i, h_j, f_ij] + b of the message from j to i is W_r h_i + b (U), W_c h_j (V) and
+// W_f f_ij: U and V are products per vertex (14 edges per vertex on a tet lattice, so a
+// fourteenth of the work of a product per edge), and one pass over the edges adds the three,
+// applies the ReLU and averages.  Its gradient needs per vertex the sums of the message
+// gradients over its row (Gr) and over the reversed edges (Gc); the products with W and with
+// h follow per vertex.  (With an E x 130 input, an E x 64 output and an E x 130 gradient per
+// layer, forward took 1.18 ms on the 20^3 cube's graph, 9261 vertices and 103 k edges.)
+// Dense layers are Z = X W^T + b with W row-major [out][in]; with bf16 set, the forward and
+// input-gradient passes use the weights rounded to BF16 and the activations rounded to TF32
+// (FP32 accumulation), the sums Gr and Gc stay FP32; the master weights and Adam moments are
+// FP32.  Weight gradients are per-block partial sums reduced in a fixed order, node sums over
+// edges run in CSR order, so a training step is deterministic.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -34,7 +41,9 @@ constexpr int kFe = 2;        // edge features
 constexpr int kEdgeIn = 2 * kH + kFe;
 constexpr int kNodeIn = 2 * kH;
 constexpr int kOut = 7;       // head: lower-triangular factor of the block (6), warm-start coefficient (1)
-constexpr int kRowsPerBlockW = 2048;  // rows per partial of a weight gradient
+constexpr int kDwBlocks = 296;  // most partials of a weight gradient (2 x 148 SMs)
+
+constexpr int kTcRows = 128, kTcN = 64;
 
 __device__ __forceinline__ float wval(const float* W, int i, int bf16) {
     const float w = W[i];
@@ -68,22 +77,38 @@ __global__ void __launch_bounds__(256) k_dense_fwd(const float* __restrict__ X, 
     else if (act == 2) Y[(size_t)r * N + c] = res[(size_t)r * N + c] + fmaxf(acc, 0.f);
 }
 
+// Rows of one or two row-major [R][64] matrices (columns 0..63 from X0, 64.. from X1) rounded to
+// TF32 into the canonical layout, K = 64 or 128: eight rows by four 16-byte chunks per warp, so
+// that a warp reads 64-byte pieces of rows and writes without bank conflicts.
+__device__ __forceinline__ void stage_rows(unsigned char* As, const float* __restrict__ X0, const float* __restrict__ X1,
+                                           int row0, int R, int K) {
+    const int C = K / 4;
+    for (int i = threadIdx.x; i < kTcRows * C; i += blockDim.x) {
+        const int r = (i & 7) | ((i >> 5) & 15) << 3, c = ((i >> 3) & 3) | (i >> 9) << 2;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + r < R) v = *(const float4*)((c < 16 ? X0 : X1) + (size_t)(row0 + r) * kH + 4 * (c & 15));
+        *(float4*)(As + umma::core_offset(r, c, C)) = make_float4(umma::tf32_round(v.x), umma::tf32_round(v.y),
+                                                                  umma::tf32_round(v.z), umma::tf32_round(v.w));
+    }
+}
+
 // The same layer on the tensor cores (tcgen05, kind::tf32, FP32 accumulation in
 // tensor memory) for N = 64 outputs: one CTA of 4 warps per 128 rows.  The
-// rows of X and the weights (rounded to BF16 first when bf16 is set) are
-// rounded to TF32 and staged in shared memory in the canonical K-major layout,
+// rows of X (two [R][64] matrices side by side for K = 128) and the weights
+// (element (n, k) at W[n * ldw + blockIdx.y * 64 + k], rounded to BF16 first when bf16 is
+// set) are rounded to TF32 and staged in shared memory in the canonical K-major layout,
 // K padded with zeros to KP (a multiple of 8); thread 0 issues KP / 8 MMAs of
 // 128 x 64 x 8 into 64 TMEM columns and commits them to an mbarrier; each warp
 // then reads its 32 rows of the accumulator and applies bias and activation.
+// blockIdx.y > 0: another 64 input columns of the same weights into the next [R][64] output,
+// without bias (the two halves of an edge layer).
 // The wait for the MMAs is bounded: a wait that gives up sets err[0] and the
 // CTA releases its TMEM and leaves without writing.
-constexpr int kTcRows = 128, kTcN = 64;
-
-__global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ X, int R, int K, int KP,
-                                                      const float* __restrict__ W, const float* __restrict__ b,
-                                                      float* __restrict__ Z, float* __restrict__ Y,
-                                                      const float* __restrict__ res, int act, int bf16,
-                                                      int* __restrict__ err) {
+__global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ X, const float* __restrict__ X1, int R,
+                                                      int K, int KP, const float* __restrict__ W, int ldw,
+                                                      const float* __restrict__ b, float* __restrict__ Z,
+                                                      float* __restrict__ Y, const float* __restrict__ res, int act,
+                                                      int bf16, int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char tc_smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_base;
@@ -91,14 +116,18 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
     unsigned char* As = tc_smem;
     unsigned char* Bs = tc_smem + (size_t)kTcRows * KP * 4;
     const int row0 = blockIdx.x * kTcRows;
-    for (int i = threadIdx.x; i < kTcRows * KP; i += blockDim.x) {
-        const int m = i / KP, k = i % KP;
-        const float v = (row0 + m < R && k < K) ? X[(size_t)(row0 + m) * K + k] : 0.f;
-        *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
+    if (K % kH == 0) {
+        stage_rows(As, X, X1, row0, R, K);
+    } else {
+        for (int i = threadIdx.x; i < kTcRows * KP; i += blockDim.x) {
+            const int m = i / KP, k = i % KP;
+            const float v = (row0 + m < R && k < K) ? X[(size_t)(row0 + m) * K + k] : 0.f;
+            *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
+        }
     }
     for (int i = threadIdx.x; i < kTcN * KP; i += blockDim.x) {
         const int n = i / KP, k = i % KP;
-        const float v = k < K ? wval(W, n * K + k, bf16) : 0.f;
+        const float v = k < K ? wval(W, n * ldw + blockIdx.y * kH + k, bf16) : 0.f;
         *(float*)(Bs + umma::core_offset(n, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
     }
     umma::fence_operands();
@@ -123,6 +152,8 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
     const int row = row0 + warp * 32 + lane;
     if (ok) {
         const uint32_t tw = td + ((uint32_t)(warp * 32) << 16);
+        float* Zr = Z + ((size_t)blockIdx.y * R + row) * kTcN;
+        const bool bias = b && blockIdx.y == 0;
 #pragma unroll
         for (int c0 = 0; c0 < kTcN; c0 += 16) {
             uint32_t r[16];
@@ -130,12 +161,20 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
             umma::tmem_wait16(r);
             if (row < R) {
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
+                for (int j = 0; j < 16; j += 4) {
                     const int c = c0 + j;
-                    const float z = __uint_as_float(r[j]) + b[c];
-                    Z[(size_t)row * kTcN + c] = z;
-                    if (act == 1) Y[(size_t)row * kTcN + c] = fmaxf(z, 0.f);
-                    else if (act == 2) Y[(size_t)row * kTcN + c] = res[(size_t)row * kTcN + c] + fmaxf(z, 0.f);
+                    float z[4];
+#pragma unroll
+                    for (int t = 0; t < 4; t++) z[t] = __uint_as_float(r[j + t]) + (bias ? b[c + t] : 0.f);
+                    *(float4*)(Zr + c) = make_float4(z[0], z[1], z[2], z[3]);
+                    if (act) {
+                        float4 q = make_float4(fmaxf(z[0], 0.f), fmaxf(z[1], 0.f), fmaxf(z[2], 0.f), fmaxf(z[3], 0.f));
+                        if (act == 2) {
+                            const float4 e = *(const float4*)(res + (size_t)row * kTcN + c);
+                            q = make_float4(e.x + q.x, e.y + q.y, e.z + q.z, e.w + q.w);
+                        }
+                        *(float4*)(Y + (size_t)row * kTcN + c) = q;
+                    }
                 }
             }
         }
@@ -150,17 +189,18 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
     }
 }
 
-// The backward products on the tensor cores (bf16 set), the same tcgen05 path as
+// The input gradients on the tensor cores (bf16 set), the same tcgen05 path as
 // k_dense_fwd_tc: operands rounded to TF32 (the weights to BF16 first) and staged in
-// shared memory in the canonical K-major layout, MMAs of 128 x NP x 8 issued by one
-// thread into FP32 accumulators in tensor memory, an mbarrier per batch of MMAs
+// shared memory in the canonical K-major layout, MMAs of 128 x KP x 8 issued by one
+// thread into FP32 accumulators in tensor memory, one mbarrier
 // (bounded waits: a wait that gives up sets err[0], waits once more with a bound for the
 // MMAs in flight, releases the TMEM and leaves without writing).
 //
 // dX[R x K] = dZ[R x N] W[N x K]: one CTA of 4 warps per 128 rows; A = the rows of dZ
 // (reduction over N, padded to NP8 = 8 * ceil(N / 8)), B = W^T (row k holds W[., k]),
-// the MMA's N = KP (K padded to 16).
-constexpr int kTcCols = 256;  // TMEM columns of a backward CTA (KP <= 256)
+// the MMA's N = KP (K padded to 16).  Columns 0..63 of dX go to a row-major [R][64] matrix,
+// 64..127 to the next one.
+constexpr int kTcCols = 128;  // TMEM columns of a backward CTA (KP <= 128)
 
 // Every thread of the CTA waits (bounded); the result is the same in all threads (a
 // block-wide AND), so the warp-wide TMEM loads and the barriers after it stay convergent.
@@ -182,13 +222,17 @@ __global__ void __launch_bounds__(128) k_dense_dx_tc(const float* __restrict__ d
     unsigned char* As = tc_smem;
     unsigned char* Bs = tc_smem + (size_t)kTcRows * NP8 * 4;
     const int row0 = blockIdx.x * kTcRows;
-    for (int i = threadIdx.x; i < kTcRows * NP8; i += blockDim.x) {
-        const int m = i / NP8, k = i % NP8;
-        const float v = (row0 + m < R && k < N) ? dZ[(size_t)(row0 + m) * N + k] : 0.f;
-        *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
+    if (N == kH) {
+        stage_rows(As, dZ, dZ, row0, R, kH);
+    } else {
+        for (int i = threadIdx.x; i < kTcRows * NP8; i += blockDim.x) {
+            const int m = i / NP8, k = i % NP8;
+            const float v = (row0 + m < R && k < N) ? dZ[(size_t)(row0 + m) * N + k] : 0.f;
+            *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
+        }
     }
     for (int i = threadIdx.x; i < KP * NP8; i += blockDim.x) {
-        const int j = i / NP8, n = i % NP8;
+        const int j = i % KP, n = i / KP;
         const float v = (j < K && n < N) ? wval(W, n * K + j, bf16) : 0.f;
         *(float*)(Bs + umma::core_offset(j, n >> 2, C) + (n & 3) * 4) = umma::tf32_round(v);
     }
@@ -218,8 +262,11 @@ __global__ void __launch_bounds__(128) k_dense_dx_tc(const float* __restrict__ d
             umma::tmem_wait16(r);
             if (row < R) {
 #pragma unroll
-                for (int j = 0; j < 16; j++)
-                    if (c0 + j < K) dX[(size_t)row * K + c0 + j] = __uint_as_float(r[j]);
+                for (int j = 0; j < 16; j += 4)
+                    if (c0 + j < K)
+                        *(float4*)(dX + ((size_t)((c0 + j) / kH) * R + row) * kH + (c0 + j) % kH) =
+                            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                        __uint_as_float(r[j + 3]));
             }
         }
     }
@@ -231,85 +278,79 @@ __global__ void __launch_bounds__(128) k_dense_dx_tc(const float* __restrict__ d
     }
 }
 
-// Partials of dW[N x K] = dZ^T X and db[N] = sum_r dZ over rows [blockIdx * kRowsPerBlockW, ...):
-// part[block][n * K + k], part[block][N * K + n] (the layout of k_dense_dw).  The D
-// accumulator is 128 x KP with rows n < N (N <= 64; rows N.. are zero), columns k < K
-// and column K = the row sum (a column of ones appended to X gives db); the block's rows
-// go through in chunks of kDwChunk, one MMA batch and mbarrier phase per chunk.
-constexpr int kDwChunk = 64;
+// Products per vertex on the FP32 pipes (64 output columns): for FP32 weights, and for the sums
+// Gr and Gc, which TF32 would round.
+// C[R x 64] = A B (+ bias, act as k_dense_fwd; + add1 + add2), A = [A0 | A1] of row-major [R][64]
+// matrices (K = 64: A0 only), B(k, m) = W[m sm + (k % 64) sk + (k / 64) sx + blockIdx.y sy];
+// blockIdx.y > 0: the next [R][64] output, without bias.  256 threads per 64 rows, 4 x 4
+// outputs each.
+struct MatIndex {
+    int sm, sk, sx, sy;
+};
 
-__global__ void __launch_bounds__(128) k_dense_dw_tc(const float* __restrict__ dZ, const float* __restrict__ X, int R,
-                                                     int N, int K, int KP, float* __restrict__ part,
-                                                     int* __restrict__ err) {
-    extern __shared__ __align__(128) unsigned char tc_smem[];
-    __shared__ uint64_t mbar;
-    __shared__ uint32_t tmem_base;
-    constexpr int C = kDwChunk / 4;
-    unsigned char* As = tc_smem;
-    unsigned char* Bs = tc_smem + (size_t)kTcRows * kDwChunk * 4;
-    if (threadIdx.x == 0) umma::mbar_init(&mbar, 1);
-    if (threadIdx.x < 32) umma::tmem_alloc(&tmem_base, kTcCols);
-    umma::fence_before();
-    __syncthreads();
-    umma::fence_after();
-    const uint32_t td = tmem_base;
-    const int rbeg = blockIdx.x * kRowsPerBlockW, rend = min(R, rbeg + kRowsPerBlockW);
-    bool ok = true;
-    uint32_t phase = 0;
-    for (int rc = rbeg; rc < rend && ok; rc += kDwChunk) {
-        // operands of this chunk: A row n = dZ[rc.., n], B row k = X[rc.., k] (row K: ones)
-        for (int i = threadIdx.x; i < kTcRows * kDwChunk; i += blockDim.x) {
-            const int n = i / kDwChunk, r = i % kDwChunk;
-            const float v = (n < N && rc + r < rend) ? dZ[(size_t)(rc + r) * N + n] : 0.f;
-            *(float*)(As + umma::core_offset(n, r >> 2, C) + (r & 3) * 4) = umma::tf32_round(v);
-        }
-        for (int i = threadIdx.x; i < KP * kDwChunk; i += blockDim.x) {
-            const int k = i / kDwChunk, r = i % kDwChunk;
-            float v = 0.f;
-            if (rc + r < rend) v = k < K ? X[(size_t)(rc + r) * K + k] : (k == K ? 1.f : 0.f);
-            *(float*)(Bs + umma::core_offset(k, r >> 2, C) + (r & 3) * 4) = umma::tf32_round(v);
-        }
-        umma::fence_operands();
-        umma::fence_before();
-        __syncthreads();
-        umma::fence_after();
-        if (threadIdx.x == 0) {
-            const uint32_t idesc = umma::idesc_tf32(kTcRows, KP);
-            const uint32_t a0 = umma::smem_u32(As), b0 = umma::smem_u32(Bs);
-            for (int k = 0; k < kDwChunk / 8; k++)
-                umma::mma_tf32(td, umma::smem_desc(a0 + 256u * k, C), umma::smem_desc(b0 + 256u * k, C), idesc,
-                               (rc > rbeg || k > 0) ? 1u : 0u);
-            umma::commit(&mbar);
-        }
-        ok = tc_wait_or_fail(&mbar, phase, err);
-        phase ^= 1u;
-        umma::fence_after();
-        __syncthreads();  // the next chunk overwrites the operands
+template <int K>
+__global__ void __launch_bounds__(256) k_gemm(const float* __restrict__ A0, const float* __restrict__ A1, int R,
+                                              const float* __restrict__ W, MatIndex ix, const float* __restrict__ b,
+                                              float* __restrict__ Z, float* __restrict__ Y,
+                                              const float* __restrict__ res, int act, const float* __restrict__ add1,
+                                              const float* __restrict__ add2, int bf16) {
+    extern __shared__ __align__(16) float gsm[];
+    constexpr int LA = K + 4, LB = 68;
+    float* As = gsm;            // [64][LA]
+    float* Bs = gsm + 64 * LA;  // [K][LB]
+    const int row0 = blockIdx.x * 64;
+    for (int i = threadIdx.x; i < 64 * (K / 4); i += 256) {
+        const int r = i / (K / 4), c = i % (K / 4);
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row0 + r < R) v = *(const float4*)((c < 16 ? A0 : A1) + (size_t)(row0 + r) * kH + 4 * (c & 15));
+        *(float4*)(As + r * LA + 4 * c) = v;
     }
-    const int nout = N * K + N;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = warp * 32 + lane;
-    if (ok && rbeg < rend) {
-        const uint32_t tw = td + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < KP; c0 += 16) {
-            uint32_t r[16];
-            umma::tmem_load16(tw + c0, r);
-            umma::tmem_wait16(r);
-            if (n < N) {
+    for (int i = threadIdx.x; i < K * 64; i += 256) {
+        const int k = ix.sk == 1 ? i % K : i / 64, m = ix.sk == 1 ? i / K : i % 64;  // consecutive threads: consecutive weights
+        Bs[k * LB + m] = wval(W, m * ix.sm + (k & 63) * ix.sk + (k >> 6) * ix.sx + (int)blockIdx.y * ix.sy, bf16);
+    }
+    __syncthreads();
+    const int r0 = threadIdx.x / 16 * 4, c0 = threadIdx.x % 16 * 4;
+    float acc[4][4] = {};
+#pragma unroll 4
+    for (int k = 0; k < K; k += 4) {
+        float4 a[4], w[4];
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int k = c0 + j;
-                    if (k < K) part[(size_t)blockIdx.x * nout + n * K + k] = __uint_as_float(r[j]);
-                    else if (k == K) part[(size_t)blockIdx.x * nout + N * K + n] = __uint_as_float(r[j]);
-                }
+        for (int i = 0; i < 4; i++) a[i] = *(const float4*)(As + (r0 + i) * LA + k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = *(const float4*)(Bs + (k + j) * LB + c0);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                acc[i][0] = fmaf(av[j], w[j].x, acc[i][0]);
+                acc[i][1] = fmaf(av[j], w[j].y, acc[i][1]);
+                acc[i][2] = fmaf(av[j], w[j].z, acc[i][2]);
+                acc[i][3] = fmaf(av[j], w[j].w, acc[i][3]);
             }
         }
     }
-    umma::fence_before();
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        umma::fence_after();
-        umma::tmem_dealloc(td, kTcCols);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int row = row0 + r0 + i;
+        if (row >= R) break;
+        const size_t at = (size_t)row * kH + c0;
+        float4 z = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        if (b && blockIdx.y == 0) z = make_float4(z.x + b[c0], z.y + b[c0 + 1], z.z + b[c0 + 2], z.w + b[c0 + 3]);
+        if (add1) {
+            const float4 p = *(const float4*)(add1 + at), q = *(const float4*)(add2 + at);
+            z = make_float4((p.x + q.x) + z.x, (p.y + q.y) + z.y, (p.z + q.z) + z.z, (p.w + q.w) + z.w);
+        }
+        *(float4*)(Z + (size_t)blockIdx.y * R * kH + at) = z;
+        if (act) {
+            float4 q = make_float4(fmaxf(z.x, 0.f), fmaxf(z.y, 0.f), fmaxf(z.z, 0.f), fmaxf(z.w, 0.f));
+            if (act == 2) {
+                const float4 e = *(const float4*)(res + at);
+                q = make_float4(e.x + q.x, e.y + q.y, e.z + q.z, e.w + q.w);
+            }
+            *(float4*)(Y + at) = q;
+        }
     }
 }
 
@@ -335,81 +376,128 @@ __global__ void __launch_bounds__(256) k_dense_dx(const float* __restrict__ dZ, 
     }
 }
 
-// Per-block partials of dW[N x K] = dZ^T X and db[N] = sum_r dZ over rows
-// [blockIdx * kRowsPerBlockW, ...): part[block][N * K + N].
-__global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, const float* __restrict__ X, int R,
-                                                  int N, int K, float* __restrict__ part) {
-    __shared__ float Ds[32 * 64];
-    __shared__ float Xs[32 * kEdgeIn];
-    const int nout = N * K + N;
-    float acc[40];
-    const int per = (nout + blockDim.x - 1) / blockDim.x;  // <= 40 for N*K+N <= 10240
-#pragma unroll
-    for (int j = 0; j < 40; j++) acc[j] = 0.f;
-    const int rbeg = blockIdx.x * kRowsPerBlockW, rend = min(R, rbeg + kRowsPerBlockW);
-    for (int rc = rbeg; rc < rend; rc += 32) {
-        const int nr = min(32, rend - rc);
+// Per-block partials of dW[N x K] = dZ^T X (N <= 64, K <= KT) and db[N] = sum_r dZ over the
+// block's rows: part[block][n * K + k], part[block][N * K + n].  X = [X0 | X1] of row-major
+// [R][64] matrices for K = 64 or 128, else X0 [R][K].  round_z / round_x: to TF32, the operands
+// of a tensor-core product.  A block takes `per` consecutive rows, 64 at a time through shared
+// memory, a thread 4 x KT / 16 outputs.
+template <int KT>
+__global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, const float* __restrict__ X0,
+                                                  const float* __restrict__ X1, int R, int per, int N, int K,
+                                                  int round_z, int round_x, float* __restrict__ part) {
+    extern __shared__ __align__(16) float gsm[];
+    constexpr int LZ = 68, LX = KT + 4;
+    float* Zs = gsm;            // [64][LZ]
+    float* Xs = gsm + 64 * LZ;  // [64][LX]
+    const int c0 = threadIdx.x / 16 * 4, k0 = threadIdx.x % 16 * 4;
+    float acc[KT / 64][4][4] = {};
+    float bias = 0.f;
+    const int rbeg = blockIdx.x * per, rend = min(R, rbeg + per);
+    for (int rc = rbeg; rc < rend; rc += 64) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 32 * N; i += blockDim.x) Ds[i] = (i / N) < nr ? dZ[(size_t)(rc + i / N) * N + i % N] : 0.f;
-        for (int i = threadIdx.x; i < 32 * K; i += blockDim.x) Xs[i] = (i / K) < nr ? X[(size_t)(rc + i / K) * K + i % K] : 0.f;
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < 40; j++) {
-            if (j >= per) break;
-            const int o = threadIdx.x + j * blockDim.x;
-            if (o >= nout) break;
-            float a = acc[j];
-            if (o < N * K) {
-                const int c = o / K, k = o % K;
-                for (int r = 0; r < nr; r++) a = fmaf(Ds[r * N + c], Xs[r * K + k], a);
-            } else {
-                const int c = o - N * K;
-                for (int r = 0; r < nr; r++) a += Ds[r * N + c];
-            }
-            acc[j] = a;
+        for (int i = threadIdx.x; i < 64 * 64; i += 256) {
+            const int r = i / 64, c = i % 64;
+            float v = (rc + r < rend && c < N) ? dZ[(size_t)(rc + r) * N + c] : 0.f;
+            if (round_z) v = umma::tf32_round(v);
+            Zs[r * LZ + c] = v;
         }
-    }
+        for (int i = threadIdx.x; i < 64 * KT; i += 256) {
+            const int r = i / KT, k = i % KT;
+            float v = 0.f;
+            if (rc + r < rend && k < K)
+                v = K % 64 == 0 ? (k < 64 ? X0 : X1)[(size_t)(rc + r) * kH + k % 64] : X0[(size_t)(rc + r) * K + k];
+            if (round_x) v = umma::tf32_round(v);
+            Xs[r * LX + k] = v;
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int r = 0; r < 64; r++) {
+            const float4 z = *(const float4*)(Zs + r * LZ + c0);
+            const float zv[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
-    for (int j = 0; j < 40; j++) {
-        if (j >= per) break;
-        const int o = threadIdx.x + j * blockDim.x;
-        if (o < nout) part[(size_t)blockIdx.x * nout + o] = acc[j];
+            for (int h = 0; h < KT / 64; h++) {
+                const float4 x = *(const float4*)(Xs + r * LX + 64 * h + k0);
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    acc[h][i][0] = fmaf(zv[i], x.x, acc[h][i][0]);
+                    acc[h][i][1] = fmaf(zv[i], x.y, acc[h][i][1]);
+                    acc[h][i][2] = fmaf(zv[i], x.z, acc[h][i][2]);
+                    acc[h][i][3] = fmaf(zv[i], x.w, acc[h][i][3]);
+                }
+            }
+        }
+        if (threadIdx.x < 64)
+            for (int r = 0; r < 64; r++) bias += Zs[r * LZ + threadIdx.x];
     }
+    float* out = part + (size_t)blockIdx.x * (N * K + N);
+#pragma unroll
+    for (int h = 0; h < KT / 64; h++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                if (c0 + i < N && 64 * h + k0 + j < K) out[(c0 + i) * K + 64 * h + k0 + j] = acc[h][i][j];
+    if (threadIdx.x < (unsigned)N) out[N * K + threadIdx.x] = bias;
 }
 
-// grad[o] += sum_b part[b][o] (fixed order).
-__global__ void k_reduce_parts(const float* __restrict__ part, int nparts, int nout, float* __restrict__ grad) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nout) return;
+// Partials summed in a fixed order, output o = n * K + k to grad[wo + n * ldw + k] and the last N
+// to grad[bo + n] (bo < 0: dropped).  A block sums 64 outputs, four threads each.
+__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nparts, int N, int K,
+                                                      float* __restrict__ grad, int wo, int ldw, int bo) {
+    __shared__ float sh[256];
+    const int nout = N * K + N, o = blockIdx.x * 64 + threadIdx.x % 64;
     float a = 0.f;
-    for (int b = 0; b < nparts; b++) a += part[(size_t)b * nout + o];
-    grad[o] += a;
+    if (o < nout)
+#pragma unroll 8
+        for (int b = threadIdx.x / 64; b < nparts; b += 4) a += part[(size_t)b * nout + o];
+    sh[threadIdx.x] = a;
+    __syncthreads();
+    if (threadIdx.x >= 64 || o >= nout) return;
+    a = (sh[threadIdx.x] + sh[threadIdx.x + 64]) + (sh[threadIdx.x + 128] + sh[threadIdx.x + 192]);
+    if (o < N * K) grad[wo + o / K * ldw + o % K] += a;
+    else if (bo >= 0) grad[bo + o - N * K] += a;
 }
 
-// inp[e] = [h[row(e)], h[col(e)], ef[e]]
-__global__ void k_edge_input(const float* __restrict__ h, const float* __restrict__ ef, const int* __restrict__ rows,
-                             const int* __restrict__ col, int E, float* __restrict__ inp) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t / kEdgeIn), k = (int)(t % kEdgeIn);
-    if (e >= E) return;
-    float v;
-    if (k < kH) v = h[(size_t)rows[e] * kH + k];
-    else if (k < 2 * kH) v = h[(size_t)col[e] * kH + k - kH];
-    else v = ef[(size_t)e * kFe + k - 2 * kH];
-    inp[t] = v;
-}
-
-// nin[i] = [h[i], mean_{e in row i} relu(zm[e])]  (agg stored in the second half)
-__global__ void k_node_input(const float* __restrict__ h, const float* __restrict__ zm, const int* __restrict__ start,
-                             int n, float* __restrict__ nin) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kH, c = t % kH;
+// The edge layer from its per-vertex halves: agg_i = mean over the edges e = (i, j) of row i of
+// relu(U_i + V_j + W_f f_e), and per edge one bit per channel, set where the message's argument is
+// positive (bits: the four ballots of the row's 16 lanes, lane l holding channels 4 l .. 4 l + 3).
+// 16 lanes per vertex; U and V are the two halves of UV.  Bound by the gathers of V (256 B per
+// edge, from L2).
+__global__ void __launch_bounds__(256) k_edge_agg(const float* __restrict__ UV, const float* __restrict__ We,
+                                                  const float* __restrict__ ef, const int* __restrict__ start,
+                                                  const int* __restrict__ col, int n, float* __restrict__ agg,
+                                                  uint2* __restrict__ bits, int bf16) {
+    const int lane = threadIdx.x & 15, i = (blockIdx.x * blockDim.x + threadIdx.x) / 16;
     if (i >= n) return;
-    float a = 0.f;
+    const unsigned gm = 0xffffu << (threadIdx.x & 16);
+    const int shift = threadIdx.x & 16;
+    const float4* V = (const float4*)(UV + (size_t)n * kH) + lane;
+    const float4 u = ((const float4*)UV)[(size_t)i * 16 + lane];
+    float w0[4], w1[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        w0[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH, bf16);
+        w1[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH + 1, bf16);
+    }
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
     const int b = start[i], e1 = start[i + 1];
-    for (int e = b; e < e1; e++) a += fmaxf(zm[(size_t)e * kH + c], 0.f);
-    nin[(size_t)i * kNodeIn + c] = h[(size_t)i * kH + c];
-    nin[(size_t)i * kNodeIn + kH + c] = a / (float)max(e1 - b, 1);
+#pragma unroll 4
+    for (int e = b; e < e1; e++) {
+        const float4 v = V[(size_t)col[e] * 16];
+        float2 f = ((const float2*)ef)[e];
+        if (bf16) f = make_float2(umma::tf32_round(f.x), umma::tf32_round(f.y));
+        const float z[4] = {fmaf(f.y, w1[0], fmaf(f.x, w0[0], u.x + v.x)), fmaf(f.y, w1[1], fmaf(f.x, w0[1], u.y + v.y)),
+                            fmaf(f.y, w1[2], fmaf(f.x, w0[2], u.z + v.z)), fmaf(f.y, w1[3], fmaf(f.x, w0[3], u.w + v.w))};
+        unsigned m[4];
+#pragma unroll
+        for (int t = 0; t < 4; t++) {
+            a[t] += fmaxf(z[t], 0.f);
+            m[t] = (__ballot_sync(gm, z[t] > 0.f) >> shift) & 0xffffu;
+        }
+        if (lane == 0) bits[e] = make_uint2(m[0] | m[1] << 16, m[2] | m[3] << 16);
+    }
+    const float d = (float)max(e1 - b, 1);
+    ((float4*)agg)[(size_t)i * 16 + lane] = make_float4(a[0] / d, a[1] / d, a[2] / d, a[3] / d);
 }
 
 // B_i = L_i L_i^T / a_ii from the head output o_i (L: exp of o0..2 clamped to
@@ -543,28 +631,69 @@ __global__ void k_relu_mask(const float* __restrict__ g, const float* __restrict
     if (t < m) d[t] = z[t] > 0.f ? g[t] : 0.f;
 }
 
-// gzm[e] = gnin[row(e)][64 + c] / deg(row(e)) * (zm[e] > 0)   (gradient of the averaged messages)
-__global__ void k_edge_grad(const float* __restrict__ gnin, const float* __restrict__ zm, const int* __restrict__ rows,
-                            const int* __restrict__ start, int E, float* __restrict__ gzm) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t / kH), c = (int)(t % kH);
-    if (e >= E) return;
-    const int i = rows[e];
-    gzm[t] = zm[t] > 0.f ? gnin[(size_t)i * kNodeIn + kH + c] / (float)max(start[i + 1] - start[i], 1) : 0.f;
+// q_i = g_i / deg_i: the gradient that vertex i's mean hands to each of its messages (rounded to
+// TF32 with bf16 set, as the operand of a tensor-core product).
+__global__ void k_mean_grad(const float* __restrict__ g, const int* __restrict__ start, int n, float* __restrict__ q,
+                            int bf16) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kH;
+    if (i >= n) return;
+    const float v = g[t] / (float)max(start[i + 1] - start[i], 1);
+    q[t] = bf16 ? umma::tf32_round(v) : v;
 }
 
-// gh[i] = gh_next[i] + gnin[i][c] + sum_{e in row i} ginp[e][c] + sum_{e in row i} ginp[rev(e)][64 + c]
-__global__ void k_node_grad(const float* __restrict__ gh_next, const float* __restrict__ gnin, const float* __restrict__ ginp,
-                            const int* __restrict__ start, const int* __restrict__ rev, int n, float* __restrict__ gh) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / kH, c = t % kH;
-    if (i >= n) return;
-    float a = gh_next[(size_t)i * kH + c] + gnin[(size_t)i * kNodeIn + c];
-    for (int e = start[i]; e < start[i + 1]; e++) {
-        a += ginp[(size_t)e * kEdgeIn + c];
-        a += ginp[(size_t)rev[e] * kEdgeIn + kH + c];
+// The message gradients q_i (where their bit is set) of the edges e = (i, j), summed per vertex:
+// Gr_i over row i, Gc_i over the reversed edges of row i; and the block partials of
+// sum_e gradient f_e^T (2 columns) and sum_e gradient (part[block][c * 2 + k],
+// part[block][128 + c], the layout of k_dense_dw for K = 2).  16 lanes per vertex, a block takes
+// vertices in steps of the grid.
+__global__ void __launch_bounds__(256) k_edge_grad(const float* __restrict__ q, const uint2* __restrict__ bits,
+                                                   const float* __restrict__ ef, const int* __restrict__ start,
+                                                   const int* __restrict__ col, const int* __restrict__ rev, int n,
+                                                   float* __restrict__ Gr, float* __restrict__ Gc,
+                                                   float* __restrict__ part, int bf16) {
+    __shared__ float sh[16][12 * 16];
+    const int lane = threadIdx.x & 15, grp = threadIdx.x / 16;
+    float pe[4][2] = {}, pb[4] = {};
+    for (int i = blockIdx.x * 16 + grp; i < n; i += gridDim.x * 16) {
+        const float4 qi4 = ((const float4*)q)[(size_t)i * 16 + lane];
+        const float qi[4] = {qi4.x, qi4.y, qi4.z, qi4.w};
+        float gr[4] = {0.f, 0.f, 0.f, 0.f}, gc[4] = {0.f, 0.f, 0.f, 0.f};
+        const int e1 = start[i + 1];
+#pragma unroll 2
+        for (int e = start[i]; e < e1; e++) {
+            const uint2 m = bits[e], mr = bits[rev[e]];
+            const float4 qj4 = ((const float4*)q)[(size_t)col[e] * 16 + lane];
+            const float qj[4] = {qj4.x, qj4.y, qj4.z, qj4.w};
+            float2 f = ((const float2*)ef)[e];
+            if (bf16) f = make_float2(umma::tf32_round(f.x), umma::tf32_round(f.y));
+#pragma unroll
+            for (int t = 0; t < 4; t++) {
+                const unsigned w = t < 2 ? m.x : m.y, wr = t < 2 ? mr.x : mr.y;
+                const int at = lane + (t & 1) * 16;
+                const float g = (w >> at) & 1u ? qi[t] : 0.f;
+                gr[t] += g;
+                if ((wr >> at) & 1u) gc[t] += qj[t];
+                pe[t][0] = fmaf(g, f.x, pe[t][0]);
+                pe[t][1] = fmaf(g, f.y, pe[t][1]);
+            }
+        }
+        ((float4*)Gr)[(size_t)i * 16 + lane] = make_float4(gr[0], gr[1], gr[2], gr[3]);
+        ((float4*)Gc)[(size_t)i * 16 + lane] = make_float4(gc[0], gc[1], gc[2], gc[3]);
+#pragma unroll
+        for (int t = 0; t < 4; t++) pb[t] += gr[t];
     }
-    gh[(size_t)i * kH + c] = a;
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+        sh[grp][(4 * lane + t) * 2] = pe[t][0];
+        sh[grp][(4 * lane + t) * 2 + 1] = pe[t][1];
+        sh[grp][128 + 4 * lane + t] = pb[t];
+    }
+    __syncthreads();
+    if (threadIdx.x < 192) {
+        float a = 0.f;
+        for (int k = 0; k < 16; k++) a += sh[k][threadIdx.x];
+        part[(size_t)blockIdx.x * 192 + threadIdx.x] = a;
+    }
 }
 
 __global__ void k_adam(float* __restrict__ th, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
@@ -585,14 +714,15 @@ inline int nblk(size_t n, int t) { return (int)((n + t - 1) / t); }
 struct AdmmGnn {
     int n = 0, E = 0, P = 0, bf16 = 1, steps = 0;
     std::vector<void*> allocs, gallocs;  // parameters and optimiser state; per-graph buffers
-    int *start = nullptr, *col = nullptr, *rows = nullptr, *rev = nullptr;
+    int *start = nullptr, *col = nullptr, *rev = nullptr;
     float *val = nullptr, *adiag = nullptr, *x = nullptr, *ef = nullptr;
     float *theta = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     float *z0 = nullptr, *h[4] = {nullptr, nullptr, nullptr, nullptr};
-    float *inp[3] = {nullptr, nullptr, nullptr}, *zm[3] = {nullptr, nullptr, nullptr};
-    float *nin[3] = {nullptr, nullptr, nullptr}, *zn[3] = {nullptr, nullptr, nullptr};
+    float *uv = nullptr, *agg[3] = {nullptr, nullptr, nullptr}, *zn[3] = {nullptr, nullptr, nullptr};
+    uint2* bits[3] = {nullptr, nullptr, nullptr};  // per edge: which channels of its message are positive
     float *o = nullptr, *B = nullptr;
-    float *gh = nullptr, *gh2 = nullptr, *gz = nullptr, *ginp = nullptr, *gnin = nullptr, *go = nullptr, *gB = nullptr;
+    float *gh = nullptr, *gh2 = nullptr, *gz = nullptr, *gnin = nullptr, *go = nullptr, *gB = nullptr;
+    float *q = nullptr, *gr = nullptr, *gc = nullptr;
     float *part = nullptr, *r = nullptr, *zv = nullptr, *res = nullptr, *gzv = nullptr;
     double *dots = nullptr, *scal = nullptr;
     int* derr = nullptr;    // set by a tensor-core layer whose bounded wait gave up
@@ -639,60 +769,83 @@ int galloc(AdmmGnn* g, T** p, size_t count, bool graph) {
         if (r_) return r_;       \
     } while (0)
 
-// With BF16 weights the 64-output layers run on the tensor cores, the others
-// (and every layer with FP32 weights) on the SIMT kernel.
+constexpr size_t gemm_smem(int K) { return sizeof(float) * (size_t)(64 * (K + 4) + K * 68); }
+constexpr size_t dw_smem(int KT) { return sizeof(float) * (size_t)(64 * 68 + 64 * (KT + 4)); }
+
+// A layer of 64 outputs on [R][64] inputs X (and X1 beside it for K = 128): `halves` products with
+// consecutive 64 input columns of the weights (k_dense_fwd_tc), on the tensor cores with BF16
+// weights, else on the FP32 pipes.
+void dense64(AdmmGnn* g, const float* X, const float* X1, int R, int K, int halves, int wo, int ldw, int bo, float* Z,
+             float* Y, const float* res, int act) {
+    if (g->bf16) {
+        const size_t sm = sizeof(float) * (size_t)(kTcRows + kTcN) * K;
+        k_dense_fwd_tc<<<dim3(nblk(R, kTcRows), halves), 128, sm, g->st>>>(X, X1, R, K, K, g->theta + wo, ldw,
+                                                                          g->theta + bo, Z, Y, res, act, g->bf16, g->derr);
+        return;
+    }
+    const MatIndex ix = {ldw, 1, kH, kH};
+    const dim3 grid(nblk(R, 64), halves);
+    if (K == kH)
+        k_gemm<kH><<<grid, 256, gemm_smem(kH), g->st>>>(X, X1, R, g->theta + wo, ix, g->theta + bo, Z, Y, res, act,
+                                                        nullptr, nullptr, 0);
+    else
+        k_gemm<2 * kH><<<grid, 256, gemm_smem(2 * kH), g->st>>>(X, X1, R, g->theta + wo, ix, g->theta + bo, Z, Y, res,
+                                                                act, nullptr, nullptr, 0);
+}
+
+// The input layer and the head: few inputs or outputs.
 void dense_fwd(AdmmGnn* g, const float* X, int R, int K, int wo, int bo, int N, float* Z, float* Y, const float* res,
                int act) {
     if (g->bf16 && N == kTcN && R > 0) {
         const int KP = (K + 7) / 8 * 8;
         const size_t sm = sizeof(float) * (size_t)(kTcRows + kTcN) * KP;
-        k_dense_fwd_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(X, R, K, KP, g->theta + wo, g->theta + bo, Z, Y, res, act,
-                                                            g->bf16, g->derr);
+        k_dense_fwd_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(X, X, R, K, KP, g->theta + wo, K, g->theta + bo, Z, Y, res,
+                                                            act, g->bf16, g->derr);
         return;
     }
     const size_t sm = sizeof(float) * (size_t)(N * K + 4 * K);
     k_dense_fwd<<<nblk(R, 4), 256, sm, g->st>>>(X, R, K, g->theta + wo, g->theta + bo, N, Z, Y, res, act, g->bf16);
 }
 
-// With BF16 weights the backward products run on the tensor cores (N <= 64 outputs of the
-// layer, K + 1 <= 256 inputs plus the bias column), else on the SIMT kernels.
-void dense_bwd(AdmmGnn* g, const float* dZ, const float* X, int R, int K, int wo, int N, float* dX) {
-    const int KP = (K + 1 + 15) / 16 * 16;
-    if (g->bf16 && N <= kTcN && KP <= kTcCols && R > 0) {
+// dX = dZ W (K = 64 or 128 columns, in [R][64] matrices one after the other): on the tensor cores
+// with BF16 weights.
+void dense_dx(AdmmGnn* g, const float* dZ, int R, int K, int wo, int N, float* dX) {
+    if (g->bf16) {
         const int NP8 = (N + 7) / 8 * 8;
-        if (dX) {
-            const int KPx = (K + 15) / 16 * 16;
-            const size_t sm = std::max<size_t>(sizeof(float) * (size_t)(kTcRows + KPx) * NP8, 100 * 1024);
-            k_dense_dx_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(dZ, R, N, NP8, g->theta + wo, K, KPx, dX, g->bf16,
-                                                              g->derr);
-        }
-        const int nparts = nblk(R, kRowsPerBlockW), nout = N * K + N;
-        const size_t sm = std::max<size_t>(sizeof(float) * (size_t)(kTcRows + KP) * kDwChunk, 100 * 1024);
-        k_dense_dw_tc<<<nparts, 128, sm, g->st>>>(dZ, X, R, N, K, KP, g->part, g->derr);
-        k_reduce_parts<<<nblk(nout, 256), 256, 0, g->st>>>(g->part, nparts, nout, g->grad + wo);
-        return;
-    }
-    if (dX) {
+        // at least 52 KB: no more than the four CTAs per SM that TMEM's 512 columns hold
+        const size_t sm = std::max<size_t>(sizeof(float) * (size_t)(kTcRows + K) * NP8, 52 * 1024);
+        k_dense_dx_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(dZ, R, N, NP8, g->theta + wo, K, K, dX, g->bf16, g->derr);
+    } else if (N == kH) {
+        const MatIndex ix = {1, K, 0, kH};
+        k_gemm<kH><<<dim3(nblk(R, 64), K / kH), 256, gemm_smem(kH), g->st>>>(dZ, dZ, R, g->theta + wo, ix, nullptr, dX,
+                                                                            nullptr, nullptr, 0, nullptr, nullptr, 0);
+    } else {
         const size_t sm = sizeof(float) * (size_t)(N * K + 4 * N);
-        k_dense_dx<<<nblk(R, 4), 256, sm, g->st>>>(dZ, R, N, g->theta + wo, K, dX, g->bf16);
+        k_dense_dx<<<nblk(R, 4), 256, sm, g->st>>>(dZ, R, N, g->theta + wo, K, dX, 0);
     }
-    const int nparts = nblk(R, kRowsPerBlockW), nout = N * K + N;
-    k_dense_dw<<<nparts, 256, 0, g->st>>>(dZ, X, R, N, K, g->part);
-    // the bias follows its weight in the parameter vector
-    k_reduce_parts<<<nblk(nout, 256), 256, 0, g->st>>>(g->part, nparts, nout, g->grad + wo);
+}
+
+// grad[wo + n ldw + k] += (dZ^T X)[n][k], grad[bo + n] += sum_r dZ[r][n] (bo < 0: none).
+void dense_dw(AdmmGnn* g, const float* dZ, const float* X0, const float* X1, int R, int K, int wo, int ldw, int bo, int N,
+              int round_z, int round_x) {
+    const int per = std::max(64, (nblk(R, kDwBlocks) + 63) / 64 * 64), nparts = nblk(R, per);
+    if (K <= kH) k_dense_dw<kH><<<nparts, 256, dw_smem(kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
+    else k_dense_dw<2 * kH><<<nparts, 256, dw_smem(2 * kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
+    k_reduce_parts<<<nblk(N * K + N, 64), 256, 0, g->st>>>(g->part, nparts, N, K, g->grad, wo, ldw, bo);
 }
 
 void forward(AdmmGnn* g) {
     const Off f = offsets();
-    dense_fwd(g, g->x, g->n, kFin, f.W0, f.b0, kH, g->z0, g->h[0], nullptr, 1);
+    const int n = g->n;
+    dense_fwd(g, g->x, n, kFin, f.W0, f.b0, kH, g->z0, g->h[0], nullptr, 1);
     for (int l = 0; l < 3; l++) {
-        k_edge_input<<<nblk((size_t)g->E * kEdgeIn, 256), 256, 0, g->st>>>(g->h[l], g->ef, g->rows, g->col, g->E, g->inp[l]);
-        dense_fwd(g, g->inp[l], g->E, kEdgeIn, f.We[l], f.be[l], kH, g->zm[l], nullptr, nullptr, 0);
-        k_node_input<<<nblk((size_t)g->n * kH, 256), 256, 0, g->st>>>(g->h[l], g->zm[l], g->start, g->n, g->nin[l]);
-        dense_fwd(g, g->nin[l], g->n, kNodeIn, f.Wn[l], f.bn[l], kH, g->zn[l], g->h[l + 1], g->h[l], 2);
+        dense64(g, g->h[l], g->h[l], n, kH, 2, f.We[l], kEdgeIn, f.be[l], g->uv, nullptr, nullptr, 0);
+        k_edge_agg<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(g->uv, g->theta + f.We[l], g->ef, g->start, g->col, n,
+                                                                g->agg[l], g->bits[l], g->bf16);
+        dense64(g, g->h[l], g->agg[l], n, kNodeIn, 1, f.Wn[l], kNodeIn, f.bn[l], g->zn[l], g->h[l + 1], g->h[l], 2);
     }
-    dense_fwd(g, g->h[3], g->n, kH, f.Wo, f.bo, kOut, g->o, nullptr, nullptr, 0);
-    k_blocks<<<nblk(g->n, 256), 256, 0, g->st>>>(g->o, g->adiag, g->n, g->B);
+    dense_fwd(g, g->h[3], n, kH, f.Wo, f.bo, kOut, g->o, nullptr, nullptr, 0);
+    k_blocks<<<nblk(n, 256), 256, 0, g->st>>>(g->o, g->adiag, n, g->B);
 }
 
 // ADMM_ERR_TIMEOUT once a tensor-core layer gave up waiting for its MMAs (the
@@ -735,7 +888,10 @@ int admm_gnn_create(int bf16, AdmmGnn** out) {
     cudaFuncSetAttribute(k_dense_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     cudaFuncSetAttribute(k_dense_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     cudaFuncSetAttribute(k_dense_dx_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_dense_dw_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_gemm<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(kH));
+    cudaFuncSetAttribute(k_gemm<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(2 * kH));
+    cudaFuncSetAttribute(k_dense_dw<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dw_smem(kH));
+    cudaFuncSetAttribute(k_dense_dw<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dw_smem(2 * kH));
     *out = g;
     return ADMM_OK;
 }
@@ -751,9 +907,7 @@ int admm_gnn_set_graph(AdmmGnn* g, int n, int n_edges, const int32_t* start, con
     g->gallocs.clear();
     g->n = n;
     g->E = n_edges;
-    std::vector<int> rows(n_edges), rev(n_edges, 0);
-    for (int i = 0; i < n; i++)
-        for (int e = start[i]; e < start[i + 1]; e++) rows[e] = i;
+    std::vector<int> rev(n_edges, 0);
     for (int i = 0; i < n; i++)  // reverse edge: (j -> i) in row j, binary search (columns sorted)
         for (int e = start[i]; e < start[i + 1]; e++) {
             const int j = col[e];
@@ -774,21 +928,21 @@ int admm_gnn_set_graph(AdmmGnn* g, int n, int n_edges, const int32_t* start, con
     auto ga = [&](auto** p, size_t cnt) -> int { return galloc(g, p, cnt, true); };
     const size_t H = kH, N = n, Ee = n_edges;
     int rc = ADMM_OK;
-    if ((rc = up(&g->start, start, N + 1)) || (rc = up(&g->col, col, Ee)) || (rc = up(&g->rows, rows.data(), Ee)) ||
+    if ((rc = up(&g->start, start, N + 1)) || (rc = up(&g->col, col, Ee)) ||
         (rc = up(&g->rev, rev.data(), Ee)) || (rc = up(&g->val, val, Ee)) || (rc = up(&g->adiag, adiag, N)) ||
         (rc = up(&g->x, node_feat, N * kFin)) || (rc = up(&g->ef, edge_feat, Ee * kFe)) || (rc = ga(&g->z0, N * H)) ||
         (rc = ga(&g->o, N * kOut)) || (rc = ga(&g->B, N * 9)) || (rc = ga(&g->gh, N * H)) || (rc = ga(&g->gh2, N * H)) ||
-        (rc = ga(&g->gz, std::max(Ee, N) * H)) || (rc = ga(&g->ginp, Ee * kEdgeIn)) || (rc = ga(&g->gnin, N * kNodeIn)) ||
+        (rc = ga(&g->gz, N * H)) || (rc = ga(&g->gnin, N * kNodeIn)) || (rc = ga(&g->uv, 2 * N * H)) ||
+        (rc = ga(&g->q, N * H)) || (rc = ga(&g->gr, N * H)) || (rc = ga(&g->gc, N * H)) ||
         (rc = ga(&g->go, N * kOut)) || (rc = ga(&g->gB, N * 9)) ||
-        (rc = ga(&g->part, (size_t)nblk(std::max(n_edges, n), kRowsPerBlockW) * (kH * kEdgeIn + kH))) ||
+        (rc = ga(&g->part, (size_t)kDwBlocks * (kH * kNodeIn + kH))) ||
         (rc = ga(&g->r, N * 3)) || (rc = ga(&g->zv, N * 3)) || (rc = ga(&g->res, N * 3)) || (rc = ga(&g->gzv, N * 3)) ||
         (rc = ga(&g->dots, 1024)) || (rc = ga(&g->scal, 4)))
         return rc;
     for (int l = 0; l < 4; l++) GTRY(ga(&g->h[l], N * H));
     for (int l = 0; l < 3; l++) {
-        GTRY(ga(&g->inp[l], Ee * kEdgeIn));
-        GTRY(ga(&g->zm[l], Ee * H));
-        GTRY(ga(&g->nin[l], N * kNodeIn));
+        GTRY(ga(&g->agg[l], N * H));
+        GTRY(ga(&g->bits[l], Ee));
         GTRY(ga(&g->zn[l], N * H));
     }
     return cudaGetLastError() == cudaSuccess ? ADMM_OK : ADMM_ERR_CUDA;
@@ -912,19 +1066,29 @@ namespace {
 // The backward pass from the head gradient go (dL/do) into g->grad.
 void backward_from_head(AdmmGnn* g) {
     const Off f = offsets();
-    const int n = g->n, E = g->E;
-    dense_bwd(g, g->go, g->h[3], n, kH, f.Wo, kOut, g->gh);          // gh = dL/dh3
+    const int n = g->n;
+    const int tc = g->bf16;
+    const size_t nh = (size_t)n * kH;
+    dense_dx(g, g->go, n, kH, f.Wo, kOut, g->gh);  // gh = dL/dh3
+    dense_dw(g, g->go, g->h[3], g->h[3], n, kH, f.Wo, kH, f.bo, kOut, tc, tc);
     for (int l = 2; l >= 0; l--) {
-        const size_t nh = (size_t)n * kH;
-        k_relu_mask<<<nblk(nh, 256), 256, 0, g->st>>>(g->gh, g->zn[l], nh, g->gz);   // gzn
-        dense_bwd(g, g->gz, g->nin[l], n, kNodeIn, f.Wn[l], kH, g->gnin);
-        k_edge_grad<<<nblk((size_t)E * kH, 256), 256, 0, g->st>>>(g->gnin, g->zm[l], g->rows, g->start, E, g->gz);  // gzm
-        dense_bwd(g, g->gz, g->inp[l], E, kEdgeIn, f.We[l], kH, g->ginp);
-        k_node_grad<<<nblk(nh, 256), 256, 0, g->st>>>(g->gh, g->gnin, g->ginp, g->start, g->rev, n, g->gh2);
+        k_relu_mask<<<nblk(nh, 256), 256, 0, g->st>>>(g->gh, g->zn[l], nh, g->gz);  // gzn
+        dense_dx(g, g->gz, n, kNodeIn, f.Wn[l], kH, g->gnin);
+        dense_dw(g, g->gz, g->h[l], g->agg[l], n, kNodeIn, f.Wn[l], kNodeIn, f.bn[l], kH, tc, tc);
+        k_mean_grad<<<nblk(nh, 256), 256, 0, g->st>>>(g->gnin + nh, g->start, n, g->q, tc);
+        const int eb = std::min(nblk(n, 16), kDwBlocks);
+        k_edge_grad<<<eb, 256, 0, g->st>>>(g->q, g->bits[l], g->ef, g->start, g->col, g->rev, n, g->gr, g->gc, g->part, tc);
+        k_reduce_parts<<<nblk(3 * kH, 64), 256, 0, g->st>>>(g->part, eb, kH, kFe, g->grad, f.We[l] + 2 * kH, kEdgeIn, f.be[l]);
+        dense_dw(g, g->gr, g->h[l], g->h[l], n, kH, f.We[l], kEdgeIn, -1, kH, 0, tc);
+        dense_dw(g, g->gc, g->h[l], g->h[l], n, kH, f.We[l] + kH, kEdgeIn, -1, kH, 0, tc);
+        // gh <- gh + (h half of gnin) + Gr W_r + Gc W_c
+        const MatIndex ix = {1, kEdgeIn, kH, 0};
+        k_gemm<2 * kH><<<nblk(n, 64), 256, gemm_smem(2 * kH), g->st>>>(g->gr, g->gc, n, g->theta + f.We[l], ix, nullptr,
+                                                                      g->gh2, nullptr, nullptr, 0, g->gh, g->gnin, tc);
         std::swap(g->gh, g->gh2);
     }
-    k_relu_mask<<<nblk((size_t)n * kH, 256), 256, 0, g->st>>>(g->gh, g->z0, (size_t)n * kH, g->gz);
-    dense_bwd(g, g->gz, g->x, n, kFin, f.W0, kH, nullptr);
+    k_relu_mask<<<nblk(nh, 256), 256, 0, g->st>>>(g->gh, g->z0, nh, g->gz);
+    dense_dw(g, g->gz, g->x, g->x, n, kFin, f.W0, kFin, f.b0, kH, tc, tc);
 }
 
 }  // namespace

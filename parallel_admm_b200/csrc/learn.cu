@@ -17,8 +17,8 @@
 //
 // Also a conjugate-gradient solve of A x* = b (the converged solution of a
 // sample).  One thread per row over a CSR copy of A (off-diagonal part plus
-// diagonal); the per-sweep dot products are FP64 block partials summed in a
-// fixed order, so a gradient is deterministic.  The FP64 restatement that the
+// diagonal), all samples of a batch in one launch; the dot products are FP64 block partials
+// summed in a fixed order on the device, so a gradient is deterministic.  The FP64 restatement that the
 // tests check these kernels against is in the oracle directory.
 #include <cuda_runtime.h>
 
@@ -32,8 +32,9 @@
 
 namespace {
 
-constexpr int kT = 256;
-constexpr int kParts = 296;  // blocks of the reduction kernels (2 x 148 SMs)
+constexpr int kT = 128;
+constexpr int kParts = 592;  // most blocks of the reduction kernels (4 x 148 SMs)
+constexpr int kCgChunk = 32;  // CG iterations queued between two looks at their state
 constexpr int kMaxK = 32;
 
 inline int nblk(size_t n, int t) { return (int)((n + t - 1) / t); }
@@ -43,6 +44,7 @@ __device__ __forceinline__ void row_spmv(const int* __restrict__ start, const in
                                          const float* __restrict__ val, const float* __restrict__ diag,
                                          const float* __restrict__ v, int i, float out[3]) {
     float a0 = diag[i] * v[3 * i], a1 = diag[i] * v[3 * i + 1], a2 = diag[i] * v[3 * i + 2];
+#pragma unroll 4
     for (int e = start[i]; e < start[i + 1]; e++) {
         const int j = col[e];
         const float w = val[e];
@@ -55,120 +57,10 @@ __device__ __forceinline__ void row_spmv(const int* __restrict__ start, const in
     out[2] = a2;
 }
 
-// x0 = xc + theta (xc - xl)
-__global__ void k_t_init(const float* __restrict__ xc, const float* __restrict__ xl, const float* __restrict__ th, int n,
-                         float* __restrict__ x0) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int c = 0; c < 3; c++) x0[3 * i + c] = fmaf(th[i], xc[3 * i + c] - xl[3 * i + c], xc[3 * i + c]);
-}
-
-// r_k = b - A x_k; x_{k+1} = x_k + omega m r_k + beta (x_k - x_{k-1})
-__global__ void k_t_sweep(const int* __restrict__ start, const int* __restrict__ col, const float* __restrict__ val,
-                          const float* __restrict__ diag, const float* __restrict__ m, const float* __restrict__ b,
-                          const float* __restrict__ xk, const float* __restrict__ xkm1, int n, float omega, float beta,
-                          float* __restrict__ rk, float* __restrict__ xk1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float ax[3];
-    row_spmv(start, col, val, diag, xk, i, ax);
-    for (int c = 0; c < 3; c++) {
-        const int q = 3 * i + c;
-        const float r = b[q] - ax[c];
-        rk[q] = r;
-        xk1[q] = fmaf(omega * m[i], r, fmaf(beta, xk[q] - xkm1[q], xk[q]));
-    }
-}
-
-// e = x - xs
-__global__ void k_t_diff(const float* __restrict__ x, const float* __restrict__ xs, size_t cnt, float* __restrict__ e) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < cnt) e[t] = x[t] - xs[t];
-}
-
-// ae = A e, block partials of e . A e
-__global__ void k_t_anorm2(const int* __restrict__ start, const int* __restrict__ col, const float* __restrict__ val,
-                           const float* __restrict__ diag, const float* __restrict__ e, int n, float* __restrict__ ae,
-                           double* __restrict__ part) {
-    __shared__ double sh[kT];
-    double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float a[3];
-        row_spmv(start, col, val, diag, e, i, a);
-        for (int c = 0; c < 3; c++) {
-            ae[3 * i + c] = a[c];
-            acc += (double)a[c] * (double)e[3 * i + c];
-        }
-    }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// block partials of v . v
-__global__ void k_t_sq(const float* __restrict__ v, size_t cnt, double* __restrict__ part) {
-    __shared__ double sh[kT];
-    double acc = 0.0;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += (size_t)gridDim.x * blockDim.x)
-        acc += (double)v[t] * (double)v[t];
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// g = s1 a (+ s2 c when c is given)
-__global__ void k_t_seed(float* __restrict__ g, const float* __restrict__ a, const float* __restrict__ c, size_t cnt,
-                         double s1, double s2) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cnt) return;
-    double v = (double)a[t] * s1;
-    if (c) v += (double)c[t] * s2;
-    g[t] = (float)v;
-}
-
-// One adjoint step k: gk = (1 + beta_k) g1 - omega_k A (m g1) - beta_{k+1} g2 (g2 may be
-// null); partials of g1 . m r_k and g1 . (x_k - x_{k-1}); gm_i += omega_k g1_i . r_k,i.
-__global__ void k_t_adjoint(const int* __restrict__ start, const int* __restrict__ col, const float* __restrict__ val,
-                            const float* __restrict__ diag, const float* __restrict__ m, const float* __restrict__ g1,
-                            const float* __restrict__ g2, const float* __restrict__ rk, const float* __restrict__ xk,
-                            const float* __restrict__ xkm1, int n, float omega, float beta_k, float beta_k1,
-                            float* __restrict__ gk, float* __restrict__ gm, double* __restrict__ part_o,
-                            double* __restrict__ part_b) {
-    __shared__ double sh[2 * kT];
-    double ao = 0.0, ab = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        // A (m g1) row i
-        float a0 = diag[i] * m[i] * g1[3 * i], a1 = diag[i] * m[i] * g1[3 * i + 1], a2 = diag[i] * m[i] * g1[3 * i + 2];
-        for (int e = start[i]; e < start[i + 1]; e++) {
-            const int j = col[e];
-            const float w = val[e] * m[j];
-            a0 = fmaf(w, g1[3 * j], a0);
-            a1 = fmaf(w, g1[3 * j + 1], a1);
-            a2 = fmaf(w, g1[3 * j + 2], a2);
-        }
-        const float amg[3] = {a0, a1, a2};
-        float gmi = 0.f;
-        for (int c = 0; c < 3; c++) {
-            const int q = 3 * i + c;
-            float g = fmaf(1.f + beta_k, g1[q], -omega * amg[c]);
-            if (g2) g = fmaf(-beta_k1, g2[q], g);
-            gk[q] = g;
-            ao += (double)g1[q] * (double)m[i] * (double)rk[q];
-            ab += (double)g1[q] * ((double)xk[q] - (double)xkm1[q]);
-            gmi = fmaf(g1[q], rk[q], gmi);
-        }
-        gm[i] = fmaf(omega, gmi, gm[i]);
-    }
-    sh[threadIdx.x] = ao;
-    sh[kT + threadIdx.x] = ab;
+// Block sum of two doubles (fixed order) into out0[0], out1[0] by thread 0; sh: 2 x kT.
+__device__ __forceinline__ void block_sum2(double a, double b, double* sh, double* out0, double* out1) {
+    sh[threadIdx.x] = a;
+    sh[kT + threadIdx.x] = b;
     __syncthreads();
     for (int o = blockDim.x / 2; o > 0; o >>= 1) {
         if ((int)threadIdx.x < o) {
@@ -178,99 +70,301 @@ __global__ void k_t_adjoint(const int* __restrict__ start, const int* __restrict
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        part_o[blockIdx.x] = sh[0];
-        part_b[blockIdx.x] = sh[kT];
+        *out0 = sh[0];
+        if (out1) *out1 = sh[kT];
     }
 }
 
-// gth_i += g0_i . (xc - xl)_i
-__global__ void k_t_theta(const float* __restrict__ g0, const float* __restrict__ xc, const float* __restrict__ xl, int n,
-                          float* __restrict__ gth) {
+// The kernels of a loss and its gradient take all samples of a batch at once: blockIdx.y is the
+// sample, its vectors at sample * n3.  Everything between the upload and the download stays on
+// the device (with the sums read back by the host, a sample of K = 6 sweeps waited 8 times).
+struct TrainMat {
+    const int *start, *col;
+    const float *val, *diag;
+    int n;
+    size_t n3;
+};
+
+// ae = A (x - xs); block partials of (x - xs) . A (x - xs) and of |A (x - xs)|^2 into
+// part[sample][0 / 1][block].  x0 (first pass): x0 = xc + theta (xc - xl), xc = x.
+__global__ void __launch_bounds__(kT) k_t_error(TrainMat M, const float* __restrict__ x, const float* __restrict__ xs,
+                                                const float* __restrict__ xl, const float* __restrict__ th,
+                                                float* __restrict__ x0, float* __restrict__ ae,
+                                                double* __restrict__ part) {
+    __shared__ double sh[2 * kT];
+    const size_t off = blockIdx.y * M.n3;
+    x += off;
+    xs += off;
+    double e2 = 0.0, r2 = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
+        const float e[3] = {x[3 * i] - xs[3 * i], x[3 * i + 1] - xs[3 * i + 1], x[3 * i + 2] - xs[3 * i + 2]};
+        float a[3] = {M.diag[i] * e[0], M.diag[i] * e[1], M.diag[i] * e[2]};
+#pragma unroll 4
+        for (int k = M.start[i]; k < M.start[i + 1]; k++) {
+            const int j = M.col[k];
+            const float w = M.val[k];
+            for (int c = 0; c < 3; c++) a[c] = fmaf(w, x[3 * j + c] - xs[3 * j + c], a[c]);
+        }
+        for (int c = 0; c < 3; c++) {
+            ae[off + 3 * i + c] = a[c];
+            e2 += (double)a[c] * (double)e[c];
+            r2 += (double)a[c] * (double)a[c];
+            if (x0) x0[off + 3 * i + c] = fmaf(th[i], x[3 * i + c] - xl[off + 3 * i + c], x[3 * i + c]);
+        }
+    }
+    double* p = part + (size_t)blockIdx.y * 2 * gridDim.x;
+    block_sum2(e2, r2, sh, p + blockIdx.x, p + gridDim.x + blockIdx.x);
+}
+
+// r_k = b - A x_k; x_{k+1} = x_k + omega m r_k + beta (x_k - x_{k-1})
+__global__ void __launch_bounds__(kT) k_t_sweep(TrainMat M, const float* __restrict__ m, const float* __restrict__ b,
+                                                const float* __restrict__ xk, const float* __restrict__ xkm1,
+                                                float omega, float beta, float* __restrict__ rk,
+                                                float* __restrict__ xk1) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float a = 0.f;
-    for (int c = 0; c < 3; c++) a = fmaf(g0[3 * i + c], xc[3 * i + c] - xl[3 * i + c], a);
-    gth[i] += a;
+    if (i >= M.n) return;
+    const size_t off = blockIdx.y * M.n3;
+    float ax[3];
+    row_spmv(M.start, M.col, M.val, M.diag, xk + off, i, ax);
+    for (int c = 0; c < 3; c++) {
+        const size_t q = off + 3 * i + c;
+        const float r = b[q] - ax[c];
+        rk[q] = r;
+        xk1[q] = fmaf(omega * m[i], r, fmaf(beta, xk[q] - xkm1[q], xk[q]));
+    }
+}
+
+// Sum of n partials in a fixed order, the same in every thread of the block; sh: 2 x kT.
+__device__ __forceinline__ double parts_sum(const double* __restrict__ p, int n, double* sh) {
+    double a = 0.0;
+    for (int k = threadIdx.x; k < n; k += blockDim.x) a += p[k];
+    __shared__ double total;
+    __syncthreads();
+    block_sum2(a, 0.0, sh, &total, nullptr);
+    __syncthreads();
+    return total;
+}
+
+// Per sample (blockIdx.x): scal = E_c, R_c, E_K, R_K from the partials of the two k_t_error passes.
+__global__ void __launch_bounds__(kT) k_t_scalars(const double* __restrict__ pc, const double* __restrict__ pK, int nb,
+                                                  double* __restrict__ scal) {
+    __shared__ double sh[2 * kT];
+    const size_t at = (size_t)blockIdx.x * 2 * nb;
+    for (int k = 0; k < 4; k++) {
+        const double v = parts_sum((k < 2 ? pc : pK) + at + (k & 1) * nb, nb, sh);
+        if (threadIdx.x == 0) scal[4 * blockIdx.x + k] = v;
+    }
+}
+
+// The adjoint's seed g_K = 2 A e_K / (E_c nsamp) (+ mu 2 A A e_K / (R_c nsamp)); a sample whose x_c is
+// the solution (E_c = 0) is left out.
+__global__ void __launch_bounds__(kT) k_t_seed(TrainMat M, const float* __restrict__ ae, const double* __restrict__ scal,
+                                               double mu, int nsamp, float* __restrict__ g) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M.n) return;
+    const size_t off = blockIdx.y * M.n3;
+    const double Ec = scal[4 * blockIdx.y], Rc = scal[4 * blockIdx.y + 1];
+    const bool used = Ec > 0.0, res = mu > 0.0 && Rc > 0.0;
+    float a2[3] = {0.f, 0.f, 0.f};
+    if (used && res) row_spmv(M.start, M.col, M.val, M.diag, ae + off, i, a2);
+    for (int c = 0; c < 3; c++) {
+        const size_t q = off + 3 * i + c;
+        double v = used ? (double)ae[q] * (2.0 / (Ec * nsamp)) : 0.0;
+        if (used && res) v += (double)a2[c] * (mu * 2.0 / (Rc * nsamp));
+        g[q] = (float)v;
+    }
+}
+
+// One adjoint step k: gk = (1 + beta_k) g1 - omega_k A (m g1) - beta_{k+1} g2 (g2 may be
+// null); partials of g1 . m r_k and g1 . (x_k - x_{k-1}) into part[0 / 1][sample][block];
+// gm_i (+)= omega_k g1_i . r_k,i per sample (first: set).
+__global__ void __launch_bounds__(kT) k_t_adjoint(TrainMat M, const float* __restrict__ m, const double* __restrict__ scal,
+                                                  const float* __restrict__ g1, const float* __restrict__ g2,
+                                                  const float* __restrict__ rk, const float* __restrict__ xk,
+                                                  const float* __restrict__ xkm1, float omega, float beta_k,
+                                                  float beta_k1, int first, float* __restrict__ gk,
+                                                  float* __restrict__ gm, double* __restrict__ part) {
+    __shared__ double sh[2 * kT];
+    const size_t off = blockIdx.y * M.n3;
+    const bool used = scal[4 * blockIdx.y] > 0.0;
+    double ao = 0.0, ab = 0.0;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < M.n) {
+        float gmi = 0.f;
+        if (used) {
+            const float* g = g1 + off;
+            // A (m g1) row i
+            float a0 = M.diag[i] * m[i] * g[3 * i], a1 = M.diag[i] * m[i] * g[3 * i + 1],
+                  a2 = M.diag[i] * m[i] * g[3 * i + 2];
+#pragma unroll 4
+            for (int e = M.start[i]; e < M.start[i + 1]; e++) {
+                const int j = M.col[e];
+                const float w = M.val[e] * m[j];
+                a0 = fmaf(w, g[3 * j], a0);
+                a1 = fmaf(w, g[3 * j + 1], a1);
+                a2 = fmaf(w, g[3 * j + 2], a2);
+            }
+            const float amg[3] = {a0, a1, a2};
+            for (int c = 0; c < 3; c++) {
+                const size_t q = off + 3 * i + c;
+                const float gi = g1[q], ri = rk[q];
+                float v = fmaf(1.f + beta_k, gi, -omega * amg[c]);
+                if (g2) v = fmaf(-beta_k1, g2[q], v);
+                gk[q] = v;
+                ao += (double)gi * (double)m[i] * (double)ri;
+                ab += (double)gi * ((double)xk[q] - (double)xkm1[q]);
+                gmi = fmaf(gi, ri, gmi);
+            }
+        } else {
+            for (int c = 0; c < 3; c++) gk[off + 3 * i + c] = 0.f;
+        }
+        const size_t at = (size_t)blockIdx.y * M.n + i;
+        gm[at] = fmaf(omega, gmi, first ? 0.f : gm[at]);
+    }
+    const size_t at = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    block_sum2(ao, ab, sh, part + at, part + (size_t)gridDim.y * gridDim.x + at);
+}
+
+// gm_i += the samples' gm_i, gth_i += sum over the samples of g0_i . (xc - xl)_i; the last blocks:
+// the sums over all partials of dL/domega_k (block -> 2 k) and dL/dbeta_k (2 k + 1) onto coef.
+__global__ void __launch_bounds__(kT) k_t_collect(TrainMat M, const double* __restrict__ scal, const float* __restrict__ g0,
+                                                  const float* __restrict__ xc, const float* __restrict__ xl,
+                                                  const float* __restrict__ gms, int S, int row_blocks,
+                                                  const double* __restrict__ part, int parts, float* __restrict__ gm,
+                                                  float* __restrict__ gth, double* __restrict__ coef) {
+    __shared__ double sh[2 * kT];
+    if ((int)blockIdx.x >= row_blocks) {
+        const int k = blockIdx.x - row_blocks;
+        const double v = parts_sum(part + (size_t)k * parts, parts, sh);
+        if (threadIdx.x == 0) coef[k] += v;
+        return;
+    }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M.n) return;
+    float a = gm[i], t = gth[i];
+    for (int s = 0; s < S; s++) {
+        a += gms[(size_t)s * M.n + i];
+        if (!(scal[4 * s] > 0.0)) continue;
+        float d = 0.f;
+        for (int c = 0; c < 3; c++) {
+            const size_t q = s * M.n3 + 3 * i + c;
+            d = fmaf(g0[q], xc[q] - xl[q], d);
+        }
+        t += d;
+    }
+    gm[i] = a;
+    gth[i] = t;
 }
 
 // ---- conjugate gradients (diag(A) preconditioned) for the converged solution ----
-// r = b - A x, z = r / a, p = z; part = r . z
-__global__ void k_cg_init(const int* __restrict__ start, const int* __restrict__ col, const float* __restrict__ val,
-                          const float* __restrict__ diag, const float* __restrict__ b, const float* __restrict__ x, int n,
-                          float* __restrict__ r, float* __restrict__ p, double* __restrict__ part) {
-    __shared__ double sh[kT];
+// Two launches per iteration, the scalars on the device: every block of a kernel sums the
+// partials that the kernel before it left.  Once the iteration has ended (done), the kernels
+// still queued do nothing.
+struct CgState {
+    double rz0, rz, pq;  // (r, z) at the start, now; (p, A p)
+    int iters, done;
+};
+
+// r = b - A x, z = r / a; part = r . z
+__global__ void __launch_bounds__(kT) k_cg_init(TrainMat M, const float* __restrict__ b, const float* __restrict__ x,
+                                                float* __restrict__ r, float* __restrict__ z, double* __restrict__ part) {
+    __shared__ double sh[2 * kT];
     double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
         float a[3];
-        row_spmv(start, col, val, diag, x, i, a);
+        row_spmv(M.start, M.col, M.val, M.diag, x, i, a);
         for (int c = 0; c < 3; c++) {
             const int q = 3 * i + c;
-            const float rr = b[q] - a[c];
+            const float rr = b[q] - a[c], zz = rr / M.diag[i];
             r[q] = rr;
-            p[q] = rr / diag[i];
-            acc += (double)rr * (double)(rr / diag[i]);
+            z[q] = zz;
+            acc += (double)rr * (double)zz;
         }
     }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    block_sum2(acc, 0.0, sh, part + blockIdx.x, nullptr);
 }
 
-// q = A p, part = p . q
-__global__ void k_cg_q(const int* __restrict__ start, const int* __restrict__ col, const float* __restrict__ val,
-                       const float* __restrict__ diag, const float* __restrict__ p, int n, float* __restrict__ q,
-                       double* __restrict__ part) {
-    __shared__ double sh[kT];
+// Entry q of the direction z + beta p (p null: z).
+__device__ __forceinline__ float cg_direction(const float* __restrict__ z, const float* __restrict__ p, int q,
+                                              double beta) {
+    return p ? (float)((double)z[q] + beta * (double)p[q]) : z[q];
+}
+
+// Iteration `it`: rz = the sum of the partials of the last kernel; ends here once rz has dropped
+// by rel_tol^2, or is 0; else p_new = z + (rz / rz_old) p and q = A p_new (the neighbours' p_new
+// computed from their z and p), part = p_new . q.
+__global__ void __launch_bounds__(kT) k_cg_q(TrainMat M, const float* __restrict__ z, const float* __restrict__ p,
+                                             int nparts, const double* __restrict__ parts_in, double rel_tol2, int it,
+                                             const CgState* __restrict__ old, CgState* __restrict__ cur,
+                                             float* __restrict__ pn, float* __restrict__ q, double* __restrict__ part) {
+    __shared__ double sh[2 * kT];
+    const CgState s0 = *old;
+    const double rz = s0.done ? s0.rz : parts_sum(parts_in, nparts, sh);
+    const double rz0 = it == 0 ? rz : s0.rz0;
+    const bool done = s0.done || !(rz > rel_tol2 * rz0 && rz > 0.0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        CgState c = s0;
+        c.rz0 = rz0;
+        c.rz = rz;
+        c.done = done;
+        *cur = c;
+    }
+    if (done) return;
+    const double beta = it == 0 ? 0.0 : rz / s0.rz;
+    const float* pp = it == 0 ? nullptr : p;
     double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float a[3];
-        row_spmv(start, col, val, diag, p, i, a);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x) {
+        float pi[3], a[3];
         for (int c = 0; c < 3; c++) {
+            pi[c] = cg_direction(z, pp, 3 * i + c, beta);
+            a[c] = M.diag[i] * pi[c];
+        }
+#pragma unroll 4
+        for (int e = M.start[i]; e < M.start[i + 1]; e++) {
+            const int j = M.col[e];
+            const float w = M.val[e];
+            for (int c = 0; c < 3; c++) a[c] = fmaf(w, cg_direction(z, pp, 3 * j + c, beta), a[c]);
+        }
+        for (int c = 0; c < 3; c++) {
+            pn[3 * i + c] = pi[c];
             q[3 * i + c] = a[c];
-            acc += (double)a[c] * (double)p[3 * i + c];
+            acc += (double)a[c] * (double)pi[c];
         }
     }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+    block_sum2(acc, 0.0, sh, part + blockIdx.x, nullptr);
 }
 
-// x += alpha p, r -= alpha q; part = r . r/a (new rz)
-__global__ void k_cg_xr(const float* __restrict__ diag, const float* __restrict__ p, const float* __restrict__ q, int n,
-                        double alpha, float* __restrict__ x, float* __restrict__ r, double* __restrict__ part) {
-    __shared__ double sh[kT];
+// alpha = rz / (p . q) (ends the iteration when p . q is not positive); x += alpha p, r -= alpha q;
+// z = r / a, part = r . z (the new rz)
+__global__ void __launch_bounds__(kT) k_cg_xr(TrainMat M, const float* __restrict__ p, const float* __restrict__ q,
+                                              int nparts, const double* __restrict__ parts_in,
+                                              const CgState* __restrict__ old, CgState* __restrict__ cur,
+                                              float* __restrict__ x, float* __restrict__ r, float* __restrict__ z,
+                                              double* __restrict__ part) {
+    __shared__ double sh[2 * kT];
+    const CgState s0 = *old;
+    const double pq = s0.done ? 1.0 : parts_sum(parts_in, nparts, sh);
+    const bool done = s0.done || !(pq > 0.0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        CgState c = s0;
+        c.done = done;
+        if (!done) c.iters = s0.iters + 1;
+        *cur = c;
+    }
+    if (done) return;
+    const double alpha = s0.rz / pq;
     double acc = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.n; i += gridDim.x * blockDim.x)
         for (int c = 0; c < 3; c++) {
             const int k = 3 * i + c;
             x[k] = (float)((double)x[k] + alpha * (double)p[k]);
             const float rr = (float)((double)r[k] - alpha * (double)q[k]);
+            const float zz = rr / M.diag[i];
             r[k] = rr;
-            acc += (double)rr * (double)(rr / diag[i]);
+            z[k] = zz;
+            acc += (double)rr * (double)zz;
         }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// p = r / a + beta p
-__global__ void k_cg_p(const float* __restrict__ diag, const float* __restrict__ r, int n, double beta,
-                       float* __restrict__ p) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    for (int c = 0; c < 3; c++) p[3 * i + c] = (float)((double)(r[3 * i + c] / diag[i]) + beta * (double)p[3 * i + c]);
+    block_sum2(acc, 0.0, sh, part + blockIdx.x, nullptr);
 }
 
 }  // namespace
@@ -280,15 +374,14 @@ struct AdmmLearn {
     std::vector<void*> allocs;
     int *start = nullptr, *col = nullptr;
     float *val = nullptr, *diag = nullptr, *m = nullptr, *th = nullptr;
-    float *b = nullptr, *xc = nullptr, *xl = nullptr, *xs = nullptr;
-    float* X = nullptr;  // [(kMaxK + 1) * 3n] iterates
-    float* Rk = nullptr; // [kMaxK * 3n] residuals
-    float *g[3] = {nullptr, nullptr, nullptr}, *e = nullptr, *ae = nullptr;
-    float* a2e = nullptr;  // A A e for the residual term
-    double mu = 0.0;       // weight of the residual term
     float *gm = nullptr, *gth = nullptr;
-    float *cr = nullptr, *cp = nullptr, *cq = nullptr;
-    double* part = nullptr;  // [3 * kParts]
+    double* coef = nullptr;  // [2 kMaxK] dL/domega_k, dL/dbeta_k interleaved
+    double mu = 0.0;         // weight of the residual term
+    // workspaces, grown to the largest call: a batch's vectors; the partials and scalars
+    float* work = nullptr;
+    size_t work_floats = 0;
+    double* dwork = nullptr;
+    size_t dwork_doubles = 0;
     cudaStream_t st = nullptr;
 };
 
@@ -303,16 +396,22 @@ int lalloc(AdmmLearn* L, T** p, size_t count) {
     return ADMM_OK;
 }
 
-int sum_parts(AdmmLearn* L, const double* dev, int k, double* out) {
-    std::vector<double> h(k);
-    if (cudaMemcpyAsync(h.data(), dev, sizeof(double) * k, cudaMemcpyDeviceToHost, L->st) != cudaSuccess)
-        return ADMM_ERR_CUDA;
-    if (cudaStreamSynchronize(L->st) != cudaSuccess) return ADMM_ERR_CUDA;
-    double s = 0.0;
-    for (int i = 0; i < k; i++) s += h[i];
-    *out = s;
+// At least `count` elements at *p (their contents are lost when it grows).
+template <class T>
+int grow(T** p, size_t* have, size_t count) {
+    if (*have >= count) return ADMM_OK;
+    cudaFree(*p);
+    *p = nullptr;
+    *have = 0;
+    if (cudaMalloc((void**)p, count * sizeof(T)) != cudaSuccess) {
+        cudaGetLastError();
+        return ADMM_ERR_OOM;
+    }
+    *have = count;
     return ADMM_OK;
 }
+
+TrainMat matrix_of(const AdmmLearn* L) { return {L->start, L->col, L->val, L->diag, L->n, 3 * (size_t)L->n}; }
 
 }  // namespace
 
@@ -328,17 +427,10 @@ int admm_learn_create(int n, const int32_t* start, const int32_t* col, const flo
     if (!L) return ADMM_ERR_OOM;
     L->n = n;
     L->nnz = nnz;
-    const size_t N3 = 3 * (size_t)n;
     int rc = ADMM_OK;
     if ((rc = lalloc(L, &L->start, n + 1)) || (rc = lalloc(L, &L->col, nnz)) || (rc = lalloc(L, &L->val, nnz)) ||
         (rc = lalloc(L, &L->diag, n)) || (rc = lalloc(L, &L->m, n)) || (rc = lalloc(L, &L->th, n)) ||
-        (rc = lalloc(L, &L->b, N3)) || (rc = lalloc(L, &L->xc, N3)) || (rc = lalloc(L, &L->xl, N3)) ||
-        (rc = lalloc(L, &L->xs, N3)) || (rc = lalloc(L, &L->X, (kMaxK + 1) * N3)) ||
-        (rc = lalloc(L, &L->Rk, kMaxK * N3)) || (rc = lalloc(L, &L->g[0], N3)) || (rc = lalloc(L, &L->g[1], N3)) ||
-        (rc = lalloc(L, &L->g[2], N3)) || (rc = lalloc(L, &L->e, N3)) || (rc = lalloc(L, &L->ae, N3)) ||
-        (rc = lalloc(L, &L->a2e, N3)) ||
-        (rc = lalloc(L, &L->gm, n)) || (rc = lalloc(L, &L->gth, n)) || (rc = lalloc(L, &L->cr, N3)) ||
-        (rc = lalloc(L, &L->cp, N3)) || (rc = lalloc(L, &L->cq, N3)) || (rc = lalloc(L, &L->part, 3 * kParts))) {
+        (rc = lalloc(L, &L->gm, n)) || (rc = lalloc(L, &L->gth, n)) || (rc = lalloc(L, &L->coef, 2 * kMaxK))) {
         admm_learn_destroy(L);
         return rc;
     }
@@ -367,6 +459,8 @@ void admm_learn_destroy(AdmmLearn* L) {
         cudaStreamDestroy(L->st);
     }
     for (void* p : L->allocs) cudaFree(p);
+    cudaFree(L->work);
+    cudaFree(L->dwork);
     delete L;
 }
 
@@ -377,91 +471,79 @@ int admm_learn_loss_grad(AdmmLearn* L, int K, const float* omega, const float* b
         return ADMM_ERR_INVALID;
     const int n = L->n;
     const size_t N3 = 3 * (size_t)n;
-    const int gb = nblk(n, kT);
+    const TrainMat M = matrix_of(L);
+    const int gb = nblk(n, kT), ge = std::min(gb, kParts);
     cudaStream_t st = L->st;
+    // samples per batch: 2 K + 9 vectors each, at most 2 GiB together (one at least)
+    const size_t per = (size_t)(2 * K + 9) * N3 + n;
+    const int most = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nsamp, ((size_t)2 << 30) / (4 * per), 32768}));
+    if (int rc = grow(&L->work, &L->work_floats, per * most)) return rc;
+    if (int rc = grow(&L->dwork, &L->dwork_doubles, (size_t)most * (4 + 4 * (size_t)ge + 2 * (size_t)K * gb))) return rc;
     cudaMemcpyAsync(L->m, m, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(L->th, theta, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(L->gm, 0, sizeof(float) * n, st);
     cudaMemsetAsync(L->gth, 0, sizeof(float) * n, st);
-    std::vector<double> go(K, 0.0), gbt(K, 0.0);
+    cudaMemsetAsync(L->coef, 0, sizeof(double) * 2 * kMaxK, st);
     double total = 0.0;
     int used = 0;
+    std::vector<double> hs;
+    for (int s0 = 0; s0 < nsamp; s0 += most) {
+        const int S = std::min(most, nsamp - s0);
+        const size_t SN = S * N3, bytes = sizeof(float) * SN, off = (size_t)s0 * N3;
+        float* w = L->work;
+        auto take = [&](size_t cnt) {
+            float* p = w;
+            w += cnt;
+            return p;
+        };
+        float *db = take(SN), *dxc = take(SN), *dxl = take(SN), *dxs = take(SN);
+        float *X = take((K + 1) * SN), *Rk = take(K * SN), *ae = take(SN);
+        float* g[3] = {take(SN), take(SN), take(SN)};
+        float* gms = take((size_t)S * n);
+        double *scal = L->dwork, *pc = scal + 4 * (size_t)S, *pK = pc + 2 * (size_t)S * ge, *pa = pK + 2 * (size_t)S * ge;
+        cudaMemcpyAsync(dxc, xc + off, bytes, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(dxs, xs + off, bytes, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(dxl, xl + off, bytes, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(db, b + off, bytes, cudaMemcpyHostToDevice, st);
+        // E_c = (xc - x*)^T A (xc - x*), R_c = |A (xc - x*)|^2 = |b - A xc|^2, and x_0
+        k_t_error<<<dim3(ge, S), kT, 0, st>>>(M, dxc, dxs, dxl, L->th, X, ae, pc);
+        for (int k = 0; k < K; k++)
+            k_t_sweep<<<dim3(gb, S), kT, 0, st>>>(M, L->m, db, X + k * SN, X + (k > 0 ? k - 1 : 0) * SN, omega[k],
+                                                  k > 0 ? beta[k] : 0.f, Rk + k * SN, X + (k + 1) * SN);
+        k_t_error<<<dim3(ge, S), kT, 0, st>>>(M, X + K * SN, dxs, nullptr, nullptr, nullptr, ae, pK);
+        k_t_scalars<<<S, kT, 0, st>>>(pc, pK, ge, scal);
+        // adjoint from g_K, g_k in g[k % 3]
+        k_t_seed<<<dim3(gb, S), kT, 0, st>>>(M, ae, scal, L->mu, nsamp, g[K % 3]);
+        for (int k = K - 1; k >= 0; k--)
+            k_t_adjoint<<<dim3(gb, S), kT, 0, st>>>(M, L->m, scal, g[(k + 1) % 3], k + 2 <= K ? g[(k + 2) % 3] : nullptr,
+                                                    Rk + k * SN, X + k * SN, X + (k > 0 ? k - 1 : 0) * SN, omega[k],
+                                                    k > 0 ? beta[k] : 0.f, k + 1 < K ? beta[k + 1] : 0.f, k == K - 1,
+                                                    g[k % 3], gms, pa + 2 * (size_t)k * S * gb);
+        k_t_collect<<<gb + 2 * K, kT, 0, st>>>(M, scal, g[0], dxc, dxl, gms, S, gb, pa, S * gb, L->gm, L->gth, L->coef);
+        const size_t have = hs.size();
+        hs.resize(have + 4 * (size_t)S);
+        if (cudaMemcpyAsync(hs.data() + have, scal, sizeof(double) * 4 * S, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return ADMM_ERR_CUDA;
+    }
     for (int s = 0; s < nsamp; s++) {
-        const size_t off = (size_t)s * N3;
-        cudaMemcpyAsync(L->b, b + off, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(L->xc, xc + off, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(L->xl, xl + off, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(L->xs, xs + off, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-        // E_c = (xc - x*)^T A (xc - x*)
-        k_t_diff<<<nblk(N3, kT), kT, 0, st>>>(L->xc, L->xs, N3, L->e);
-        k_t_anorm2<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->e, n, L->ae, L->part);
-        double Ec = 0.0;
-        if (int rc = sum_parts(L, L->part, kParts, &Ec)) return rc;
+        const double Ec = hs[4 * s], Rc = hs[4 * s + 1], EK = hs[4 * s + 2], RK = hs[4 * s + 3];
         if (!(Ec > 0.0)) continue;
         used++;
-        // R_c = |A (xc - x*)|^2 = |b - A xc|^2
-        double Rc = 0.0;
-        if (L->mu > 0.0) {
-            k_t_sq<<<kParts, kT, 0, st>>>(L->ae, N3, L->part);
-            if (int rc = sum_parts(L, L->part, kParts, &Rc)) return rc;
-        }
-        // forward
-        k_t_init<<<gb, kT, 0, st>>>(L->xc, L->xl, L->th, n, L->X);
-        for (int k = 0; k < K; k++) {
-            const float* xk = L->X + k * N3;
-            const float* xkm1 = L->X + (k > 0 ? k - 1 : 0) * N3;
-            k_t_sweep<<<gb, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->m, L->b, xk, xkm1, n, omega[k],
-                                         k > 0 ? beta[k] : 0.f, L->Rk + k * N3, L->X + (k + 1) * N3);
-        }
-        k_t_diff<<<nblk(N3, kT), kT, 0, st>>>(L->X + K * N3, L->xs, N3, L->e);
-        k_t_anorm2<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->e, n, L->ae, L->part);
-        double EK = 0.0;
-        if (int rc = sum_parts(L, L->part, kParts, &EK)) return rc;
         total += EK / Ec;
-        // adjoint: g_K = 2 A e_K / (E_c nsamp) (+ mu 2 A A e_K / (R_c nsamp)), in g[K % 3]
-        const double sc = 2.0 / (Ec * nsamp);
-        float* gK = L->g[K % 3];
-        if (L->mu > 0.0 && Rc > 0.0) {
-            double RK = 0.0;
-            k_t_sq<<<kParts, kT, 0, st>>>(L->ae, N3, L->part);
-            if (int rc = sum_parts(L, L->part, kParts, &RK)) return rc;
-            total += L->mu * RK / Rc;
-            k_t_anorm2<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->ae, n, L->a2e, L->part);
-            k_t_seed<<<nblk(N3, kT), kT, 0, st>>>(gK, L->ae, L->a2e, N3, sc, L->mu * 2.0 / (Rc * nsamp));
-        } else {
-            k_t_seed<<<nblk(N3, kT), kT, 0, st>>>(gK, L->ae, nullptr, N3, sc, 0.0);
-        }
-        for (int k = K - 1; k >= 0; k--) {
-            const float* g1 = L->g[(k + 1) % 3];
-            const float* g2 = k + 2 <= K ? L->g[(k + 2) % 3] : nullptr;
-            const float bk1 = k + 1 < K ? beta[k + 1] : 0.f;
-            const float* xk = L->X + k * N3;
-            const float* xkm1 = L->X + (k > 0 ? k - 1 : 0) * N3;
-            k_t_adjoint<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->m, g1, g2, L->Rk + k * N3, xk,
-                                               xkm1, n, omega[k], k > 0 ? beta[k] : 0.f, bk1, L->g[k % 3], L->gm,
-                                               L->part, L->part + kParts);
-            std::vector<double> h(2 * kParts);
-            cudaMemcpyAsync(h.data(), L->part, sizeof(double) * 2 * kParts, cudaMemcpyDeviceToHost, st);
-            if (cudaStreamSynchronize(st) != cudaSuccess) return ADMM_ERR_CUDA;
-            double so = 0.0, sb = 0.0;
-            for (int i = 0; i < kParts; i++) {
-                so += h[i];
-                sb += h[kParts + i];
-            }
-            go[k] += so;
-            if (k > 0) gbt[k] += sb;
-        }
-        k_t_theta<<<gb, kT, 0, st>>>(L->g[0], L->xc, L->xl, n, L->gth);
+        if (L->mu > 0.0 && Rc > 0.0) total += L->mu * RK / Rc;
     }
-    if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) return ADMM_ERR_CUDA;
+    double coef[2 * kMaxK];
+    if (cudaMemcpyAsync(coef, L->coef, sizeof(double) * 2 * K, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        (g_m && cudaMemcpyAsync(g_m, L->gm, sizeof(float) * n, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
+        (g_theta && cudaMemcpyAsync(g_theta, L->gth, sizeof(float) * n, cudaMemcpyDeviceToHost, st) != cudaSuccess) ||
+        cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
+        return ADMM_ERR_CUDA;
     if (loss) *loss = used ? total / nsamp : 0.0;
     if (g_omega)
-        for (int k = 0; k < K; k++) g_omega[k] = (float)go[k];
+        for (int k = 0; k < K; k++) g_omega[k] = (float)coef[2 * k];
     if (g_beta)
-        for (int k = 0; k < K; k++) g_beta[k] = (float)gbt[k];
-    if (g_m && cudaMemcpy(g_m, L->gm, sizeof(float) * n, cudaMemcpyDeviceToHost) != cudaSuccess) return ADMM_ERR_CUDA;
-    if (g_theta && cudaMemcpy(g_theta, L->gth, sizeof(float) * n, cudaMemcpyDeviceToHost) != cudaSuccess)
-        return ADMM_ERR_CUDA;
+        for (int k = 0; k < K; k++) g_beta[k] = k > 0 ? (float)coef[2 * k + 1] : 0.f;
     return ADMM_OK;
 }
 
@@ -475,28 +557,35 @@ int admm_learn_solve(AdmmLearn* L, const float* b, float* x, double rel_tol, int
     if (!L || !b || !x || max_iter < 0) return ADMM_ERR_INVALID;
     const int n = L->n;
     const size_t N3 = 3 * (size_t)n;
+    const TrainMat M = matrix_of(L);
+    const int ge = std::min(nblk(n, kT), kParts);
     cudaStream_t st = L->st;
-    cudaMemcpyAsync(L->b, b, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(L->xs, x, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
-    k_cg_init<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->b, L->xs, n, L->cr, L->cp, L->part);
-    double rz = 0.0;
-    if (int rc = sum_parts(L, L->part, kParts, &rz)) return rc;
-    const double rz0 = rz;
-    int it = 0;
-    for (; it < max_iter && rz > rel_tol * rel_tol * rz0 && rz > 0.0; it++) {
-        k_cg_q<<<kParts, kT, 0, st>>>(L->start, L->col, L->val, L->diag, L->cp, n, L->cq, L->part);
-        double pq = 0.0;
-        if (int rc = sum_parts(L, L->part, kParts, &pq)) return rc;
-        if (!(pq > 0.0)) break;
-        const double alpha = rz / pq;
-        k_cg_xr<<<kParts, kT, 0, st>>>(L->diag, L->cp, L->cq, n, alpha, L->xs, L->cr, L->part);
-        double rzn = 0.0;
-        if (int rc = sum_parts(L, L->part, kParts, &rzn)) return rc;
-        k_cg_p<<<nblk(n, kT), kT, 0, st>>>(L->diag, L->cr, n, rzn / rz, L->cp);
-        rz = rzn;
+    if (int rc = grow(&L->work, &L->work_floats, 7 * N3)) return rc;
+    constexpr size_t kState = sizeof(CgState) / sizeof(double);
+    static_assert(sizeof(CgState) % sizeof(double) == 0, "the states lie in the double workspace");
+    if (int rc = grow(&L->dwork, &L->dwork_doubles, 2 * kState + 2 * (size_t)ge)) return rc;
+    float *db = L->work, *dx = db + N3, *r = dx + N3, *z = r + N3, *q = z + N3, *p[2] = {q + N3, q + 2 * N3};
+    CgState* state[2] = {(CgState*)L->dwork, (CgState*)(L->dwork + kState)};
+    double* part[2] = {L->dwork + 2 * kState, L->dwork + 2 * kState + ge};
+    cudaMemsetAsync(state[0], 0, sizeof(CgState), st);
+    cudaMemcpyAsync(db, b, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(dx, x, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
+    k_cg_init<<<ge, kT, 0, st>>>(M, db, dx, r, z, part[0]);
+    CgState now = {};
+    for (int it = 0; it < max_iter && !now.done;) {
+        for (const int end = std::min(max_iter, it + kCgChunk); it < end; it++) {
+            k_cg_q<<<ge, kT, 0, st>>>(M, z, p[it & 1], ge, part[0], rel_tol * rel_tol, it, state[0], state[1],
+                                      p[(it + 1) & 1], q, part[1]);
+            k_cg_xr<<<ge, kT, 0, st>>>(M, p[(it + 1) & 1], q, ge, part[1], state[1], state[0], dx, r, z, part[0]);
+        }
+        if (cudaMemcpyAsync(&now, state[0], sizeof(now), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return ADMM_ERR_CUDA;
     }
-    if (cudaMemcpy(x, L->xs, sizeof(float) * N3, cudaMemcpyDeviceToHost) != cudaSuccess) return ADMM_ERR_CUDA;
-    if (iters) *iters = it;
+    if (cudaMemcpyAsync(x, dx, sizeof(float) * N3, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return ADMM_ERR_CUDA;
+    if (iters) *iters = now.iters;
     return cudaGetLastError() == cudaSuccess ? ADMM_OK : ADMM_ERR_CUDA;
 }
 
