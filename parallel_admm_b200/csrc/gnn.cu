@@ -41,7 +41,7 @@ constexpr int kFe = 2;        // edge features
 constexpr int kEdgeIn = 2 * kH + kFe;
 constexpr int kNodeIn = 2 * kH;
 constexpr int kOut = 7;       // head: lower-triangular factor of the block (6), warm-start coefficient (1)
-constexpr int kDwBlocks = 296;  // most partials of a weight gradient (2 x 148 SMs)
+constexpr int kDwBlocks = 592;  // most partials of a weight gradient (4 x 148 SMs)
 
 constexpr int kTcRows = 128, kTcN = 64;
 
@@ -77,13 +77,18 @@ __global__ void __launch_bounds__(256) k_dense_fwd(const float* __restrict__ X, 
     else if (act == 2) Y[(size_t)r * N + c] = res[(size_t)r * N + c] + fmaxf(acc, 0.f);
 }
 
+constexpr int kTcThreads = 256;  // a warp per 32 rows and half of the output columns
+
 // Rows of one or two row-major [R][64] matrices (columns 0..63 from X0, 64.. from X1) rounded to
-// TF32 into the canonical layout, K = 64 or 128: eight rows by four 16-byte chunks per warp, so
-// that a warp reads 64-byte pieces of rows and writes without bank conflicts.
+// TF32 into the canonical layout: eight rows by four 16-byte chunks per warp, so that a warp
+// reads 64-byte pieces of rows and writes without bank conflicts.
+template <int K>
 __device__ __forceinline__ void stage_rows(unsigned char* As, const float* __restrict__ X0, const float* __restrict__ X1,
-                                           int row0, int R, int K) {
-    const int C = K / 4;
-    for (int i = threadIdx.x; i < kTcRows * C; i += blockDim.x) {
+                                           int row0, int R) {
+    constexpr int C = K / 4;
+#pragma unroll
+    for (int u = 0; u < kTcRows * C / kTcThreads; u++) {
+        const int i = threadIdx.x + u * kTcThreads;
         const int r = (i & 7) | ((i >> 5) & 15) << 3, c = ((i >> 3) & 3) | (i >> 9) << 2;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (row0 + r < R) v = *(const float4*)((c < 16 ? X0 : X1) + (size_t)(row0 + r) * kH + 4 * (c & 15));
@@ -92,43 +97,66 @@ __device__ __forceinline__ void stage_rows(unsigned char* As, const float* __res
     }
 }
 
+// The accumulator (128 rows, N columns of TMEM at td) to f(row, column, four values): warp w
+// reads rows 32 (w % 4) .. + 31 of half w / 4 of the columns.
+template <int N, class F>
+__device__ __forceinline__ void read_rows(uint32_t td, int row0, F f) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = warp & 3;
+    const int row = row0 + q * 32 + lane;
+    const uint32_t tw = td + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+    for (int u = 0; u < N / 32; u++) {
+        const int c0 = (warp >> 2) * (N / 2) + 16 * u;
+        uint32_t r[16];
+        umma::tmem_load16(tw + c0, r);
+        umma::tmem_wait16(r);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4)
+            f(row, c0 + j, make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
+                                       __uint_as_float(r[j + 3])));
+    }
+}
+
 // The same layer on the tensor cores (tcgen05, kind::tf32, FP32 accumulation in
-// tensor memory) for N = 64 outputs: one CTA of 4 warps per 128 rows.  The
-// rows of X (two [R][64] matrices side by side for K = 128) and the weights
-// (element (n, k) at W[n * ldw + blockIdx.y * 64 + k], rounded to BF16 first when bf16 is
-// set) are rounded to TF32 and staged in shared memory in the canonical K-major layout,
-// K padded with zeros to KP (a multiple of 8); thread 0 issues KP / 8 MMAs of
-// 128 x 64 x 8 into 64 TMEM columns and commits them to an mbarrier; each warp
-// then reads its 32 rows of the accumulator and applies bias and activation.
+// tensor memory) for 64 outputs: one CTA per 128 rows.  The
+// rows of X (K = 64 or 128: one or two [R][64] matrices side by side; K = 8: [R][Kin] padded with
+// zeros) and the weights (element (n, k) at W[n * ldw + blockIdx.y * 64 + k], rounded to BF16
+// first) are rounded to TF32 and staged in shared memory in the canonical K-major layout;
+// thread 0 issues K / 8 MMAs of 128 x 64 x 8 into 64 TMEM columns and commits them to an
+// mbarrier; the warps then read the accumulator and apply bias and activation.
 // blockIdx.y > 0: another 64 input columns of the same weights into the next [R][64] output,
-// without bias (the two halves of an edge layer).
+// without bias (the two halves of an edge layer).  Bound by the latency of staging: with K and the
+// loads' trip counts known to the compiler, 64 -> 19 us for 28 k rows and K = 64 (cold caches).
 // The wait for the MMAs is bounded: a wait that gives up sets err[0] and the
 // CTA releases its TMEM and leaves without writing.
-__global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ X, const float* __restrict__ X1, int R,
-                                                      int K, int KP, const float* __restrict__ W, int ldw,
-                                                      const float* __restrict__ b, float* __restrict__ Z,
-                                                      float* __restrict__ Y, const float* __restrict__ res, int act,
-                                                      int bf16, int* __restrict__ err) {
+template <int K>
+__global__ void __launch_bounds__(kTcThreads) k_dense_fwd_tc(const float* __restrict__ X, const float* __restrict__ X1,
+                                                             int R, int Kin, const float* __restrict__ W, int ldw,
+                                                             const float* __restrict__ b, float* __restrict__ Z,
+                                                             float* __restrict__ Y, const float* __restrict__ res,
+                                                             int act, int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char tc_smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_base;
-    const int C = KP / 4;  // 16-byte K chunks per row
+    constexpr int C = K / 4;  // 16-byte K chunks per row
     unsigned char* As = tc_smem;
-    unsigned char* Bs = tc_smem + (size_t)kTcRows * KP * 4;
+    unsigned char* Bs = tc_smem + (size_t)kTcRows * K * 4;
     const int row0 = blockIdx.x * kTcRows;
     if (K % kH == 0) {
-        stage_rows(As, X, X1, row0, R, K);
+        stage_rows<(K % kH == 0 ? K : kH)>(As, X, X1, row0, R);
     } else {
-        for (int i = threadIdx.x; i < kTcRows * KP; i += blockDim.x) {
-            const int m = i / KP, k = i % KP;
-            const float v = (row0 + m < R && k < K) ? X[(size_t)(row0 + m) * K + k] : 0.f;
+#pragma unroll
+        for (int u = 0; u < kTcRows * K / kTcThreads; u++) {
+            const int i = threadIdx.x + u * kTcThreads, m = i / K, k = i % K;
+            const float v = (row0 + m < R && k < Kin) ? X[(size_t)(row0 + m) * Kin + k] : 0.f;
             *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
         }
     }
-    for (int i = threadIdx.x; i < kTcN * KP; i += blockDim.x) {
-        const int n = i / KP, k = i % KP;
-        const float v = k < K ? wval(W, n * ldw + blockIdx.y * kH + k, bf16) : 0.f;
-        *(float*)(Bs + umma::core_offset(n, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
+#pragma unroll 16
+    for (int u = 0; u < kTcN * K / kTcThreads; u++) {
+        const int i = threadIdx.x + u * kTcThreads, n = i / K, k = i % K;
+        const float v = k < Kin ? wval(W, n * ldw + blockIdx.y * kH + k, 1) : 0.f;
+        *(float*)(Bs + umma::core_offset(n, k >> 2, C) + (k & 3) * 4) = v;  // BF16 is exact in TF32
     }
     umma::fence_operands();
     if (threadIdx.x == 0) umma::mbar_init(&mbar, 1);
@@ -140,7 +168,7 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
     if (threadIdx.x == 0) {
         const uint32_t idesc = umma::idesc_tf32(kTcRows, kTcN);
         const uint32_t a0 = umma::smem_u32(As), b0 = umma::smem_u32(Bs);
-        for (int k = 0; k < KP / 8; k++)  // 8 TF32 values of K = two 16-byte chunks per MMA
+        for (int k = 0; k < K / 8; k++)  // 8 TF32 values of K = two 16-byte chunks per MMA
             umma::mma_tf32(td, umma::smem_desc(a0 + 256u * k, C), umma::smem_desc(b0 + 256u * k, C), idesc, k > 0);
         umma::commit(&mbar);
     }
@@ -148,36 +176,20 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
     if (!ok) umma::mbar_wait(&mbar, 0, 1 << 22);  // the MMAs in flight, once more with a bound
     ok = __syncthreads_and(ok) != 0;              // uniform: the TMEM loads below are warp-wide
     umma::fence_after();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = row0 + warp * 32 + lane;
     if (ok) {
-        const uint32_t tw = td + ((uint32_t)(warp * 32) << 16);
-        float* Zr = Z + ((size_t)blockIdx.y * R + row) * kTcN;
         const bool bias = b && blockIdx.y == 0;
-#pragma unroll
-        for (int c0 = 0; c0 < kTcN; c0 += 16) {
-            uint32_t r[16];
-            umma::tmem_load16(tw + c0, r);
-            umma::tmem_wait16(r);
-            if (row < R) {
-#pragma unroll
-                for (int j = 0; j < 16; j += 4) {
-                    const int c = c0 + j;
-                    float z[4];
-#pragma unroll
-                    for (int t = 0; t < 4; t++) z[t] = __uint_as_float(r[j + t]) + (bias ? b[c + t] : 0.f);
-                    *(float4*)(Zr + c) = make_float4(z[0], z[1], z[2], z[3]);
-                    if (act) {
-                        float4 q = make_float4(fmaxf(z[0], 0.f), fmaxf(z[1], 0.f), fmaxf(z[2], 0.f), fmaxf(z[3], 0.f));
-                        if (act == 2) {
-                            const float4 e = *(const float4*)(res + (size_t)row * kTcN + c);
-                            q = make_float4(e.x + q.x, e.y + q.y, e.z + q.z, e.w + q.w);
-                        }
-                        *(float4*)(Y + (size_t)row * kTcN + c) = q;
-                    }
-                }
+        read_rows<kTcN>(td, row0, [&](int row, int c, float4 v) {
+            if (row >= R) return;
+            if (bias) v = make_float4(v.x + b[c], v.y + b[c + 1], v.z + b[c + 2], v.w + b[c + 3]);
+            *(float4*)(Z + ((size_t)blockIdx.y * R + row) * kTcN + c) = v;
+            if (!act) return;
+            float4 q = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+            if (act == 2) {
+                const float4 e = *(const float4*)(res + (size_t)row * kTcN + c);
+                q = make_float4(e.x + q.x, e.y + q.y, e.z + q.z, e.w + q.w);
             }
-        }
+            *(float4*)(Y + (size_t)row * kTcN + c) = q;
+        });
     } else if (threadIdx.x == 0) {
         atomicExch(err, 1);
     }
@@ -196,85 +208,68 @@ __global__ void __launch_bounds__(128) k_dense_fwd_tc(const float* __restrict__ 
 // (bounded waits: a wait that gives up sets err[0], waits once more with a bound for the
 // MMAs in flight, releases the TMEM and leaves without writing).
 //
-// dX[R x K] = dZ[R x N] W[N x K]: one CTA of 4 warps per 128 rows; A = the rows of dZ
-// (reduction over N, padded to NP8 = 8 * ceil(N / 8)), B = W^T (row k holds W[., k]),
-// the MMA's N = KP (K padded to 16).  Columns 0..63 of dX go to a row-major [R][64] matrix,
-// 64..127 to the next one.
-constexpr int kTcCols = 128;  // TMEM columns of a backward CTA (KP <= 128)
-
-// Every thread of the CTA waits (bounded); the result is the same in all threads (a
-// block-wide AND), so the warp-wide TMEM loads and the barriers after it stay convergent.
-__device__ __forceinline__ bool tc_wait_or_fail(uint64_t* mbar, uint32_t parity, int* err) {
-    bool ok = umma::mbar_wait(mbar, parity, 1 << 22);
-    if (!ok) umma::mbar_wait(mbar, parity, 1 << 22);  // the MMAs in flight, once more with a bound
-    ok = __syncthreads_and(ok) != 0;
-    if (!ok && threadIdx.x == 0) atomicExch(err, 1);
-    return ok;
-}
-
-__global__ void __launch_bounds__(128) k_dense_dx_tc(const float* __restrict__ dZ, int R, int N, int NP8,
-                                                     const float* __restrict__ W, int K, int KP,
-                                                     float* __restrict__ dX, int bf16, int* __restrict__ err) {
+// dX[R x K] = dZ[R x N] W[N x K]: one CTA per 128 rows; A = the rows of dZ (reduction over N,
+// NP = 64 or, for the head, 8: N padded with zeros), B = W^T (row k holds W[., k]), the MMA's N = K
+// (64 or 128).  Columns 0..63 of dX go to a row-major [R][64] matrix, 64..127 to the next one.
+template <int NP, int K>
+__global__ void __launch_bounds__(kTcThreads) k_dense_dx_tc(const float* __restrict__ dZ, int R, int N,
+                                                            const float* __restrict__ W, float* __restrict__ dX,
+                                                            int* __restrict__ err) {
     extern __shared__ __align__(128) unsigned char tc_smem[];
     __shared__ uint64_t mbar;
     __shared__ uint32_t tmem_base;
-    const int C = NP8 / 4;
+    constexpr int C = NP / 4;
     unsigned char* As = tc_smem;
-    unsigned char* Bs = tc_smem + (size_t)kTcRows * NP8 * 4;
+    unsigned char* Bs = tc_smem + (size_t)kTcRows * NP * 4;
     const int row0 = blockIdx.x * kTcRows;
-    if (N == kH) {
-        stage_rows(As, dZ, dZ, row0, R, kH);
+    if (NP == kH) {
+        stage_rows<kH>(As, dZ, dZ, row0, R);
     } else {
-        for (int i = threadIdx.x; i < kTcRows * NP8; i += blockDim.x) {
-            const int m = i / NP8, k = i % NP8;
+#pragma unroll
+        for (int u = 0; u < kTcRows * NP / kTcThreads; u++) {
+            const int i = threadIdx.x + u * kTcThreads, m = i / NP, k = i % NP;
             const float v = (row0 + m < R && k < N) ? dZ[(size_t)(row0 + m) * N + k] : 0.f;
             *(float*)(As + umma::core_offset(m, k >> 2, C) + (k & 3) * 4) = umma::tf32_round(v);
         }
     }
-    for (int i = threadIdx.x; i < KP * NP8; i += blockDim.x) {
-        const int j = i % KP, n = i / KP;
-        const float v = (j < K && n < N) ? wval(W, n * K + j, bf16) : 0.f;
-        *(float*)(Bs + umma::core_offset(j, n >> 2, C) + (n & 3) * 4) = umma::tf32_round(v);
+#pragma unroll 16
+    for (int u = 0; u < (K * NP + kTcThreads - 1) / kTcThreads; u++) {
+        const int i = threadIdx.x + u * kTcThreads, j = i % K, n = i / K;
+        if (n < NP) {
+            const float v = n < N ? wval(W, n * K + j, 1) : 0.f;
+            *(float*)(Bs + umma::core_offset(j, n >> 2, C) + (n & 3) * 4) = v;
+        }
     }
     umma::fence_operands();
     if (threadIdx.x == 0) umma::mbar_init(&mbar, 1);
-    if (threadIdx.x < 32) umma::tmem_alloc(&tmem_base, kTcCols);
+    if (threadIdx.x < 32) umma::tmem_alloc(&tmem_base, K);
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t td = tmem_base;
     if (threadIdx.x == 0) {
-        const uint32_t idesc = umma::idesc_tf32(kTcRows, KP);
+        const uint32_t idesc = umma::idesc_tf32(kTcRows, K);
         const uint32_t a0 = umma::smem_u32(As), b0 = umma::smem_u32(Bs);
-        for (int k = 0; k < NP8 / 8; k++)
+        for (int k = 0; k < NP / 8; k++)
             umma::mma_tf32(td, umma::smem_desc(a0 + 256u * k, C), umma::smem_desc(b0 + 256u * k, C), idesc, k > 0);
         umma::commit(&mbar);
     }
-    const bool ok = tc_wait_or_fail(&mbar, 0, err);
+    bool ok = umma::mbar_wait(&mbar, 0, 1 << 22);
+    if (!ok) umma::mbar_wait(&mbar, 0, 1 << 22);
+    ok = __syncthreads_and(ok) != 0;
     umma::fence_after();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = row0 + warp * 32 + lane;
     if (ok) {
-        const uint32_t tw = td + ((uint32_t)(warp * 32) << 16);
-        for (int c0 = 0; c0 < KP; c0 += 16) {
-            uint32_t r[16];
-            umma::tmem_load16(tw + c0, r);
-            umma::tmem_wait16(r);
-            if (row < R) {
-#pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                    if (c0 + j < K)
-                        *(float4*)(dX + ((size_t)((c0 + j) / kH) * R + row) * kH + (c0 + j) % kH) =
-                            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                                        __uint_as_float(r[j + 3]));
-            }
-        }
+        read_rows<K>(td, row0, [&](int row, int c, float4 v) {
+            if (row < R) *(float4*)(dX + ((size_t)(c / kH) * R + row) * kH + c % kH) = v;
+        });
+    } else if (threadIdx.x == 0) {
+        atomicExch(err, 1);
     }
     umma::fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {
         umma::fence_after();
-        umma::tmem_dealloc(td, kTcCols);
+        umma::tmem_dealloc(td, K);
     }
 }
 
@@ -380,7 +375,12 @@ __global__ void __launch_bounds__(256) k_dense_dx(const float* __restrict__ dZ, 
 // block's rows: part[block][n * K + k], part[block][N * K + n].  X = [X0 | X1] of row-major
 // [R][64] matrices for K = 64 or 128, else X0 [R][K].  round_z / round_x: to TF32, the operands
 // of a tensor-core product.  A block takes `per` consecutive rows, 64 at a time through shared
-// memory, a thread 4 x KT / 16 outputs.
+// memory, a thread 4 x KT / 16 outputs.  blockIdx.y > 0: the next [R][64] matrix of dZ, into the
+// partials after the first one's.
+__device__ __forceinline__ float4 round4(float4 v, int on) {
+    return on ? make_float4(umma::tf32_round(v.x), umma::tf32_round(v.y), umma::tf32_round(v.z), umma::tf32_round(v.w)) : v;
+}
+
 template <int KT>
 __global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, const float* __restrict__ X0,
                                                   const float* __restrict__ X1, int R, int per, int N, int K,
@@ -392,22 +392,38 @@ __global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, 
     const int c0 = threadIdx.x / 16 * 4, k0 = threadIdx.x % 16 * 4;
     float acc[KT / 64][4][4] = {};
     float bias = 0.f;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    dZ += (size_t)blockIdx.y * R * kH;
     const int rbeg = blockIdx.x * per, rend = min(R, rbeg + per);
     for (int rc = rbeg; rc < rend; rc += 64) {
         __syncthreads();
-        for (int i = threadIdx.x; i < 64 * 64; i += 256) {
-            const int r = i / 64, c = i % 64;
-            float v = (rc + r < rend && c < N) ? dZ[(size_t)(rc + r) * N + c] : 0.f;
-            if (round_z) v = umma::tf32_round(v);
-            Zs[r * LZ + c] = v;
+        if (N == 64) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int i = threadIdx.x + 256 * u, r = i / 16, c = i % 16 * 4;
+                const float4 v = rc + r < rend ? *(const float4*)(dZ + (size_t)(rc + r) * kH + c) : zero;
+                *(float4*)(Zs + r * LZ + c) = round4(v, round_z);
+            }
+        } else {
+            for (int i = threadIdx.x; i < 64 * 64; i += 256) {
+                const int r = i / 64, c = i % 64;
+                const float v = (rc + r < rend && c < N) ? dZ[(size_t)(rc + r) * N + c] : 0.f;
+                Zs[r * LZ + c] = round_z ? umma::tf32_round(v) : v;
+            }
         }
-        for (int i = threadIdx.x; i < 64 * KT; i += 256) {
-            const int r = i / KT, k = i % KT;
-            float v = 0.f;
-            if (rc + r < rend && k < K)
-                v = K % 64 == 0 ? (k < 64 ? X0 : X1)[(size_t)(rc + r) * kH + k % 64] : X0[(size_t)(rc + r) * K + k];
-            if (round_x) v = umma::tf32_round(v);
-            Xs[r * LX + k] = v;
+        if (K % 64 == 0) {
+#pragma unroll
+            for (int u = 0; u < KT / 16; u++) {
+                const int i = threadIdx.x + 256 * u, r = i / (KT / 4), k = i % (KT / 4) * 4;
+                const float4 v = rc + r < rend ? *(const float4*)((k < 64 ? X0 : X1) + (size_t)(rc + r) * kH + k % 64) : zero;
+                *(float4*)(Xs + r * LX + k) = round4(v, round_x);
+            }
+        } else {
+            for (int i = threadIdx.x; i < 64 * KT; i += 256) {
+                const int r = i / KT, k = i % KT;
+                const float v = (rc + r < rend && k < K) ? X0[(size_t)(rc + r) * K + k] : 0.f;
+                Xs[r * LX + k] = round_x ? umma::tf32_round(v) : v;
+            }
         }
         __syncthreads();
 #pragma unroll 4
@@ -426,10 +442,12 @@ __global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, 
                 }
             }
         }
-        if (threadIdx.x < 64)
+        if (threadIdx.x < 64) {
+#pragma unroll 16
             for (int r = 0; r < 64; r++) bias += Zs[r * LZ + threadIdx.x];
+        }
     }
-    float* out = part + (size_t)blockIdx.x * (N * K + N);
+    float* out = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (N * K + N);
 #pragma unroll
     for (int h = 0; h < KT / 64; h++)
 #pragma unroll
@@ -441,28 +459,34 @@ __global__ void __launch_bounds__(256) k_dense_dw(const float* __restrict__ dZ, 
 }
 
 // Partials summed in a fixed order, output o = n * K + k to grad[wo + n * ldw + k] and the last N
-// to grad[bo + n] (bo < 0: dropped).  A block sums 64 outputs, four threads each.
-__global__ void __launch_bounds__(256) k_reduce_parts(const float* __restrict__ part, int nparts, int N, int K,
-                                                      float* __restrict__ grad, int wo, int ldw, int bo) {
-    __shared__ float sh[256];
-    const int nout = N * K + N, o = blockIdx.x * 64 + threadIdx.x % 64;
+// to grad[bo + n] (bo < 0: dropped).  A block sums 32 outputs, 32 threads each; blockIdx.y > 0: the
+// next nparts partials, to weights 64 columns further.
+__global__ void __launch_bounds__(1024) k_reduce_parts(const float* __restrict__ part, int nparts, int N, int K,
+                                                       float* __restrict__ grad, int wo, int ldw, int bo) {
+    __shared__ float sh[32][33];
+    const int nout = N * K + N, tx = threadIdx.x & 31, ty = threadIdx.x >> 5, o = blockIdx.x * 32 + tx;
+    part += (size_t)blockIdx.y * nparts * nout;
     float a = 0.f;
     if (o < nout)
 #pragma unroll 8
-        for (int b = threadIdx.x / 64; b < nparts; b += 4) a += part[(size_t)b * nout + o];
-    sh[threadIdx.x] = a;
+        for (int b = ty; b < nparts; b += 32) a += part[(size_t)b * nout + o];
+    sh[tx][ty] = a;
     __syncthreads();
-    if (threadIdx.x >= 64 || o >= nout) return;
-    a = (sh[threadIdx.x] + sh[threadIdx.x + 64]) + (sh[threadIdx.x + 128] + sh[threadIdx.x + 192]);
-    if (o < N * K) grad[wo + o / K * ldw + o % K] += a;
-    else if (bo >= 0) grad[bo + o - N * K] += a;
+    a = sh[ty][tx];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
+    const int q = blockIdx.x * 32 + ty;
+    if (tx != 0 || q >= nout) return;
+    if (q < N * K) grad[wo + blockIdx.y * kH + q / K * ldw + q % K] += a;
+    else if (bo >= 0) grad[bo + q - N * K] += a;
 }
 
 // The edge layer from its per-vertex halves: agg_i = mean over the edges e = (i, j) of row i of
 // relu(U_i + V_j + W_f f_e), and per edge one bit per channel, set where the message's argument is
 // positive (bits: the four ballots of the row's 16 lanes, lane l holding channels 4 l .. 4 l + 3).
 // 16 lanes per vertex; U and V are the two halves of UV.  Bound by the gathers of V (256 B per
-// edge, from L2).
+// edge, from L2).  BITS = false: without the bits, which only the gradient reads.
+template <bool BITS>
 __global__ void __launch_bounds__(256) k_edge_agg(const float* __restrict__ UV, const float* __restrict__ We,
                                                   const float* __restrict__ ef, const int* __restrict__ start,
                                                   const int* __restrict__ col, int n, float* __restrict__ agg,
@@ -488,13 +512,14 @@ __global__ void __launch_bounds__(256) k_edge_agg(const float* __restrict__ UV, 
         if (bf16) f = make_float2(umma::tf32_round(f.x), umma::tf32_round(f.y));
         const float z[4] = {fmaf(f.y, w1[0], fmaf(f.x, w0[0], u.x + v.x)), fmaf(f.y, w1[1], fmaf(f.x, w0[1], u.y + v.y)),
                             fmaf(f.y, w1[2], fmaf(f.x, w0[2], u.z + v.z)), fmaf(f.y, w1[3], fmaf(f.x, w0[3], u.w + v.w))};
-        unsigned m[4];
 #pragma unroll
-        for (int t = 0; t < 4; t++) {
-            a[t] += fmaxf(z[t], 0.f);
-            m[t] = (__ballot_sync(gm, z[t] > 0.f) >> shift) & 0xffffu;
+        for (int t = 0; t < 4; t++) a[t] += fmaxf(z[t], 0.f);
+        if (BITS) {
+            unsigned m[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) m[t] = (__ballot_sync(gm, z[t] > 0.f) >> shift) & 0xffffu;
+            if (lane == 0) bits[e] = make_uint2(m[0] | m[1] << 16, m[2] | m[3] << 16);
         }
-        if (lane == 0) bits[e] = make_uint2(m[0] | m[1] << 16, m[2] | m[3] << 16);
     }
     const float d = (float)max(e1 - b, 1);
     ((float4*)agg)[(size_t)i * 16 + lane] = make_float4(a[0] / d, a[1] / d, a[2] / d, a[3] / d);
@@ -510,18 +535,48 @@ __device__ __forceinline__ void lower_of(const float* o, float L[9]) {
     L[6] = o[4]; L[7] = o[5]; L[8] = expf(clamp8(o[2]));
 }
 
-__global__ void k_blocks(const float* __restrict__ o, const float* __restrict__ adiag, int n, float* __restrict__ B) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float L[9];
-    lower_of(o + (size_t)i * kOut, L);
+// The head o = W h + b (7 outputs) and what is made of it: B, and the learned global step's outputs
+// m_i = trace(B_i) / 3 (the isotropic part of the block: the system is A (x) I3),
+// theta_i = clamp(o_i6, -1, 1).  64 rows per block, an output (row, c) per thread at a time.
+__global__ void __launch_bounds__(256) k_head(const float* __restrict__ h, const float* __restrict__ W,
+                                              const float* __restrict__ b, const float* __restrict__ adiag, int n,
+                                              float* __restrict__ o, float* __restrict__ B, float* __restrict__ m,
+                                              float* __restrict__ th, int bf16) {
+    __shared__ __align__(16) float Hs[64][68];
+    __shared__ float Ws[kOut][kH];
+    __shared__ float Os[64][kOut];
+    const int row0 = blockIdx.x * 64;
+    for (int i = threadIdx.x; i < kOut * kH; i += 256) Ws[i / kH][i % kH] = wval(W, i, bf16);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = threadIdx.x + 256 * u, r = i / 16, c = i % 16 * 4;
+        *(float4*)&Hs[r][c] = row0 + r < n ? *(const float4*)(h + (size_t)(row0 + r) * kH + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 64 * kOut; i += 256) {
+        const int r = i % 64, c = i / 64;
+        float acc = b[c];
+#pragma unroll 16
+        for (int k = 0; k < kH; k++) acc = fmaf(Hs[r][k], Ws[c][k], acc);
+        Os[r][c] = acc;
+        if (row0 + r < n) o[(size_t)(row0 + r) * kOut + c] = acc;
+    }
+    __syncthreads();
+    const int i = row0 + threadIdx.x;
+    if (threadIdx.x >= 64 || i >= n) return;
+    float L[9], d = 0.f;
+    lower_of(Os[threadIdx.x], L);
     const float ia = 1.f / adiag[i];
     for (int r = 0; r < 3; r++)
         for (int c = 0; c < 3; c++) {
             float a = 0.f;
             for (int k = 0; k < 3; k++) a = fmaf(L[3 * r + k], L[3 * c + k], a);
-            B[(size_t)i * 9 + 3 * r + c] = a * ia;
+            a *= ia;
+            B[(size_t)i * 9 + 3 * r + c] = a;
+            if (r == c) d += a;
         }
+    m[i] = d * (1.f / 3.f);
+    th[i] = fminf(fmaxf(Os[threadIdx.x][6], -1.f), 1.f);
 }
 
 // out = A v  (A = diag + CSR off-diagonal), v and out [n x 3]
@@ -605,16 +660,6 @@ __global__ void k_head_grad(const float* __restrict__ gB, const float* __restric
     g[4] = gL[6];
     g[5] = gL[7];
     g[6] = (gth && fabsf(oi[6]) < 1.f) ? gth[i] : 0.f;
-}
-
-// m_i = trace(B_i) / 3 (the isotropic part of the block: the system is A (x) I3),
-// theta_i = clamp(o_i6, -1, 1).
-__global__ void k_outputs(const float* __restrict__ B, const float* __restrict__ o, int n, float* __restrict__ m,
-                          float* __restrict__ th) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    m[i] = (B[(size_t)i * 9] + B[(size_t)i * 9 + 4] + B[(size_t)i * 9 + 8]) * (1.f / 3.f);
-    th[i] = fminf(fmaxf(o[(size_t)i * kOut + 6], -1.f), 1.f);
 }
 
 // gB_i = (gm_i / 3) I
@@ -722,7 +767,8 @@ struct AdmmGnn {
     uint2* bits[3] = {nullptr, nullptr, nullptr};  // per edge: which channels of its message are positive
     float *o = nullptr, *B = nullptr;
     float *gh = nullptr, *gh2 = nullptr, *gz = nullptr, *gnin = nullptr, *go = nullptr, *gB = nullptr;
-    float *q = nullptr, *gr = nullptr, *gc = nullptr;
+    float *q = nullptr, *grc = nullptr;  // message gradients per vertex; Gr then Gc
+    float *om = nullptr, *oth = nullptr;  // outputs m, theta
     float *part = nullptr, *r = nullptr, *zv = nullptr, *res = nullptr, *gzv = nullptr;
     double *dots = nullptr, *scal = nullptr;
     int* derr = nullptr;    // set by a tensor-core layer whose bounded wait gave up
@@ -771,81 +817,80 @@ int galloc(AdmmGnn* g, T** p, size_t count, bool graph) {
 
 constexpr size_t gemm_smem(int K) { return sizeof(float) * (size_t)(64 * (K + 4) + K * 68); }
 constexpr size_t dw_smem(int KT) { return sizeof(float) * (size_t)(64 * 68 + 64 * (KT + 4)); }
+constexpr size_t fwd_smem(int K) { return sizeof(float) * (size_t)(kTcRows + kTcN) * K; }
+// no more CTAs per SM than TMEM's 512 columns hold: four of 128 columns, eight of 64
+constexpr size_t dx_smem(int NP, int K) {
+    const size_t need = sizeof(float) * (size_t)(kTcRows + K) * NP, least = K > 64 ? 52 * 1024 : 26 * 1024;
+    return need > least ? need : least;
+}
 
 // A layer of 64 outputs on [R][64] inputs X (and X1 beside it for K = 128): `halves` products with
 // consecutive 64 input columns of the weights (k_dense_fwd_tc), on the tensor cores with BF16
 // weights, else on the FP32 pipes.
 void dense64(AdmmGnn* g, const float* X, const float* X1, int R, int K, int halves, int wo, int ldw, int bo, float* Z,
              float* Y, const float* res, int act) {
+    const float *W = g->theta + wo, *b = g->theta + bo;
     if (g->bf16) {
-        const size_t sm = sizeof(float) * (size_t)(kTcRows + kTcN) * K;
-        k_dense_fwd_tc<<<dim3(nblk(R, kTcRows), halves), 128, sm, g->st>>>(X, X1, R, K, K, g->theta + wo, ldw,
-                                                                          g->theta + bo, Z, Y, res, act, g->bf16, g->derr);
+        const dim3 grid(nblk(R, kTcRows), halves);
+        if (K == kH)
+            k_dense_fwd_tc<kH><<<grid, kTcThreads, fwd_smem(kH), g->st>>>(X, X1, R, K, W, ldw, b, Z, Y, res, act, g->derr);
+        else
+            k_dense_fwd_tc<2 * kH><<<grid, kTcThreads, fwd_smem(2 * kH), g->st>>>(X, X1, R, K, W, ldw, b, Z, Y, res, act, g->derr);
         return;
     }
     const MatIndex ix = {ldw, 1, kH, kH};
     const dim3 grid(nblk(R, 64), halves);
-    if (K == kH)
-        k_gemm<kH><<<grid, 256, gemm_smem(kH), g->st>>>(X, X1, R, g->theta + wo, ix, g->theta + bo, Z, Y, res, act,
-                                                        nullptr, nullptr, 0);
-    else
-        k_gemm<2 * kH><<<grid, 256, gemm_smem(2 * kH), g->st>>>(X, X1, R, g->theta + wo, ix, g->theta + bo, Z, Y, res,
-                                                                act, nullptr, nullptr, 0);
-}
-
-// The input layer and the head: few inputs or outputs.
-void dense_fwd(AdmmGnn* g, const float* X, int R, int K, int wo, int bo, int N, float* Z, float* Y, const float* res,
-               int act) {
-    if (g->bf16 && N == kTcN && R > 0) {
-        const int KP = (K + 7) / 8 * 8;
-        const size_t sm = sizeof(float) * (size_t)(kTcRows + kTcN) * KP;
-        k_dense_fwd_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(X, X, R, K, KP, g->theta + wo, K, g->theta + bo, Z, Y, res,
-                                                            act, g->bf16, g->derr);
-        return;
-    }
-    const size_t sm = sizeof(float) * (size_t)(N * K + 4 * K);
-    k_dense_fwd<<<nblk(R, 4), 256, sm, g->st>>>(X, R, K, g->theta + wo, g->theta + bo, N, Z, Y, res, act, g->bf16);
+    if (K == kH) k_gemm<kH><<<grid, 256, gemm_smem(kH), g->st>>>(X, X1, R, W, ix, b, Z, Y, res, act, nullptr, nullptr, 0);
+    else k_gemm<2 * kH><<<grid, 256, gemm_smem(2 * kH), g->st>>>(X, X1, R, W, ix, b, Z, Y, res, act, nullptr, nullptr, 0);
 }
 
 // dX = dZ W (K = 64 or 128 columns, in [R][64] matrices one after the other): on the tensor cores
 // with BF16 weights.
 void dense_dx(AdmmGnn* g, const float* dZ, int R, int K, int wo, int N, float* dX) {
+    const float* W = g->theta + wo;
     if (g->bf16) {
-        const int NP8 = (N + 7) / 8 * 8;
-        // at least 52 KB: no more than the four CTAs per SM that TMEM's 512 columns hold
-        const size_t sm = std::max<size_t>(sizeof(float) * (size_t)(kTcRows + K) * NP8, 52 * 1024);
-        k_dense_dx_tc<<<nblk(R, kTcRows), 128, sm, g->st>>>(dZ, R, N, NP8, g->theta + wo, K, K, dX, g->bf16, g->derr);
+        const int grid = nblk(R, kTcRows);
+        if (N == kH) k_dense_dx_tc<kH, 2 * kH><<<grid, kTcThreads, dx_smem(kH, 2 * kH), g->st>>>(dZ, R, N, W, dX, g->derr);
+        else k_dense_dx_tc<8, kH><<<grid, kTcThreads, dx_smem(8, kH), g->st>>>(dZ, R, N, W, dX, g->derr);
     } else if (N == kH) {
         const MatIndex ix = {1, K, 0, kH};
-        k_gemm<kH><<<dim3(nblk(R, 64), K / kH), 256, gemm_smem(kH), g->st>>>(dZ, dZ, R, g->theta + wo, ix, nullptr, dX,
-                                                                            nullptr, nullptr, 0, nullptr, nullptr, 0);
+        k_gemm<kH><<<dim3(nblk(R, 64), K / kH), 256, gemm_smem(kH), g->st>>>(dZ, dZ, R, W, ix, nullptr, dX, nullptr,
+                                                                            nullptr, 0, nullptr, nullptr, 0);
     } else {
         const size_t sm = sizeof(float) * (size_t)(N * K + 4 * N);
-        k_dense_dx<<<nblk(R, 4), 256, sm, g->st>>>(dZ, R, N, g->theta + wo, K, dX, 0);
+        k_dense_dx<<<nblk(R, 4), 256, sm, g->st>>>(dZ, R, N, W, K, dX, 0);
     }
 }
 
-// grad[wo + n ldw + k] += (dZ^T X)[n][k], grad[bo + n] += sum_r dZ[r][n] (bo < 0: none).
+// grad[wo + n ldw + k] += (dZ^T X)[n][k], grad[bo + n] += sum_r dZ[r][n] (bo < 0: none); halves = 2:
+// also the next [R][64] matrix of dZ, to weights 64 columns further.
 void dense_dw(AdmmGnn* g, const float* dZ, const float* X0, const float* X1, int R, int K, int wo, int ldw, int bo, int N,
-              int round_z, int round_x) {
+              int round_z, int round_x, int halves = 1) {
     const int per = std::max(64, (nblk(R, kDwBlocks) + 63) / 64 * 64), nparts = nblk(R, per);
-    if (K <= kH) k_dense_dw<kH><<<nparts, 256, dw_smem(kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
-    else k_dense_dw<2 * kH><<<nparts, 256, dw_smem(2 * kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
-    k_reduce_parts<<<nblk(N * K + N, 64), 256, 0, g->st>>>(g->part, nparts, N, K, g->grad, wo, ldw, bo);
+    const dim3 grid(nparts, halves);
+    if (K <= kH) k_dense_dw<kH><<<grid, 256, dw_smem(kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
+    else k_dense_dw<2 * kH><<<grid, 256, dw_smem(2 * kH), g->st>>>(dZ, X0, X1, R, per, N, K, round_z, round_x, g->part);
+    k_reduce_parts<<<dim3(nblk(N * K + N, 32), halves), 1024, 0, g->st>>>(g->part, nparts, N, K, g->grad, wo, ldw, bo);
 }
 
-void forward(AdmmGnn* g) {
+// bits: keep what the gradient needs.  The outputs m and theta go to g->om and g->oth.
+void forward(AdmmGnn* g, bool bits) {
     const Off f = offsets();
     const int n = g->n;
-    dense_fwd(g, g->x, n, kFin, f.W0, f.b0, kH, g->z0, g->h[0], nullptr, 1);
+    if (g->bf16)
+        k_dense_fwd_tc<8><<<nblk(n, kTcRows), kTcThreads, fwd_smem(8), g->st>>>(
+            g->x, g->x, n, kFin, g->theta + f.W0, kFin, g->theta + f.b0, g->z0, g->h[0], nullptr, 1, g->derr);
+    else
+        k_dense_fwd<<<nblk(n, 4), 256, sizeof(float) * (kH * kFin + 4 * kFin), g->st>>>(
+            g->x, n, kFin, g->theta + f.W0, g->theta + f.b0, kH, g->z0, g->h[0], nullptr, 1, 0);
     for (int l = 0; l < 3; l++) {
         dense64(g, g->h[l], g->h[l], n, kH, 2, f.We[l], kEdgeIn, f.be[l], g->uv, nullptr, nullptr, 0);
-        k_edge_agg<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(g->uv, g->theta + f.We[l], g->ef, g->start, g->col, n,
-                                                                g->agg[l], g->bits[l], g->bf16);
+        (bits ? k_edge_agg<true> : k_edge_agg<false>)<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(
+            g->uv, g->theta + f.We[l], g->ef, g->start, g->col, n, g->agg[l], g->bits[l], g->bf16);
         dense64(g, g->h[l], g->agg[l], n, kNodeIn, 1, f.Wn[l], kNodeIn, f.bn[l], g->zn[l], g->h[l + 1], g->h[l], 2);
     }
-    dense_fwd(g, g->h[3], n, kH, f.Wo, f.bo, kOut, g->o, nullptr, nullptr, 0);
-    k_blocks<<<nblk(n, 256), 256, 0, g->st>>>(g->o, g->adiag, n, g->B);
+    k_head<<<nblk(n, 64), 256, 0, g->st>>>(g->h[3], g->theta + f.Wo, g->theta + f.bo, g->adiag, n, g->o, g->B, g->om,
+                                           g->oth, g->bf16);
 }
 
 // ADMM_ERR_TIMEOUT once a tensor-core layer gave up waiting for its MMAs (the
@@ -884,10 +929,9 @@ int admm_gnn_create(int bf16, AdmmGnn** out) {
         admm_gnn_destroy(g);
         return ADMM_ERR_CUDA;
     }
-    cudaFuncSetAttribute(k_dense_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(k_dense_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    cudaFuncSetAttribute(k_dense_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_dense_dx_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_dense_fwd_tc<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(kH));
+    cudaFuncSetAttribute(k_dense_fwd_tc<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(2 * kH));
+    cudaFuncSetAttribute(k_dense_dx_tc<kH, 2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dx_smem(kH, 2 * kH));
     cudaFuncSetAttribute(k_gemm<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(kH));
     cudaFuncSetAttribute(k_gemm<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(2 * kH));
     cudaFuncSetAttribute(k_dense_dw<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dw_smem(kH));
@@ -933,9 +977,9 @@ int admm_gnn_set_graph(AdmmGnn* g, int n, int n_edges, const int32_t* start, con
         (rc = up(&g->x, node_feat, N * kFin)) || (rc = up(&g->ef, edge_feat, Ee * kFe)) || (rc = ga(&g->z0, N * H)) ||
         (rc = ga(&g->o, N * kOut)) || (rc = ga(&g->B, N * 9)) || (rc = ga(&g->gh, N * H)) || (rc = ga(&g->gh2, N * H)) ||
         (rc = ga(&g->gz, N * H)) || (rc = ga(&g->gnin, N * kNodeIn)) || (rc = ga(&g->uv, 2 * N * H)) ||
-        (rc = ga(&g->q, N * H)) || (rc = ga(&g->gr, N * H)) || (rc = ga(&g->gc, N * H)) ||
+        (rc = ga(&g->q, N * H)) || (rc = ga(&g->grc, 2 * N * H)) || (rc = ga(&g->om, N)) || (rc = ga(&g->oth, N)) ||
         (rc = ga(&g->go, N * kOut)) || (rc = ga(&g->gB, N * 9)) ||
-        (rc = ga(&g->part, (size_t)kDwBlocks * (kH * kNodeIn + kH))) ||
+        (rc = ga(&g->part, (size_t)std::min(kDwBlocks, nblk(N, 64)) * 2 * (kH * kNodeIn + kH))) ||
         (rc = ga(&g->r, N * 3)) || (rc = ga(&g->zv, N * 3)) || (rc = ga(&g->res, N * 3)) || (rc = ga(&g->gzv, N * 3)) ||
         (rc = ga(&g->dots, 1024)) || (rc = ga(&g->scal, 4)))
         return rc;
@@ -980,7 +1024,7 @@ int admm_gnn_get_params(AdmmGnn* g, float* theta, int P) {
 int admm_gnn_forward(AdmmGnn* g, float* blocks9) {
     if (!g || g->n <= 0) return ADMM_ERR_INVALID;
     if (g->failed) return ADMM_ERR_STATE;
-    forward(g);
+    forward(g, false);
     if (blocks9 && cudaMemcpyAsync(blocks9, g->B, sizeof(float) * 9 * (size_t)g->n, cudaMemcpyDeviceToHost, g->st) != cudaSuccess)
         return ADMM_ERR_CUDA;
     if (cudaStreamSynchronize(g->st) != cudaSuccess) return ADMM_ERR_CUDA;
@@ -995,7 +1039,7 @@ int admm_gnn_loss_grad(AdmmGnn* g, const float* R, int K, double* loss, float* g
     if (!g || g->n <= 0 || !R || K <= 0) return ADMM_ERR_INVALID;
     if (g->failed) return ADMM_ERR_STATE;
     const int n = g->n;
-    forward(g);
+    forward(g, true);
     cudaMemsetAsync(g->grad, 0, sizeof(float) * g->P, g->st);
     cudaMemsetAsync(g->gB, 0, sizeof(float) * 9 * (size_t)n, g->st);
     double total = 0.0;
@@ -1031,10 +1075,9 @@ int admm_gnn_loss_grad(AdmmGnn* g, const float* R, int K, double* loss, float* g
 int admm_gnn_outputs(AdmmGnn* g, float* m, float* theta) {
     if (!g || g->n <= 0 || !m || !theta) return ADMM_ERR_INVALID;
     if (g->failed) return ADMM_ERR_STATE;
-    forward(g);
-    k_outputs<<<nblk(g->n, 256), 256, 0, g->st>>>(g->B, g->o, g->n, g->r, g->zv);
-    cudaMemcpyAsync(m, g->r, sizeof(float) * g->n, cudaMemcpyDeviceToHost, g->st);
-    cudaMemcpyAsync(theta, g->zv, sizeof(float) * g->n, cudaMemcpyDeviceToHost, g->st);
+    forward(g, false);
+    cudaMemcpyAsync(m, g->om, sizeof(float) * g->n, cudaMemcpyDeviceToHost, g->st);
+    cudaMemcpyAsync(theta, g->oth, sizeof(float) * g->n, cudaMemcpyDeviceToHost, g->st);
     if (cudaStreamSynchronize(g->st) != cudaSuccess || cudaGetLastError() != cudaSuccess) return ADMM_ERR_CUDA;
     return tc_status(g);
 }
@@ -1047,7 +1090,7 @@ int admm_gnn_backward(AdmmGnn* g, const float* gm, const float* gtheta, float* g
     if (!g || g->n <= 0 || !gm || !gtheta) return ADMM_ERR_INVALID;
     if (g->failed) return ADMM_ERR_STATE;
     const int n = g->n;
-    forward(g);
+    forward(g, true);
     cudaMemsetAsync(g->grad, 0, sizeof(float) * g->P, g->st);
     cudaMemcpyAsync(g->r, gm, sizeof(float) * n, cudaMemcpyHostToDevice, g->st);
     cudaMemcpyAsync(g->zv, gtheta, sizeof(float) * n, cudaMemcpyHostToDevice, g->st);
@@ -1077,13 +1120,13 @@ void backward_from_head(AdmmGnn* g) {
         dense_dw(g, g->gz, g->h[l], g->agg[l], n, kNodeIn, f.Wn[l], kNodeIn, f.bn[l], kH, tc, tc);
         k_mean_grad<<<nblk(nh, 256), 256, 0, g->st>>>(g->gnin + nh, g->start, n, g->q, tc);
         const int eb = std::min(nblk(n, 16), kDwBlocks);
-        k_edge_grad<<<eb, 256, 0, g->st>>>(g->q, g->bits[l], g->ef, g->start, g->col, g->rev, n, g->gr, g->gc, g->part, tc);
-        k_reduce_parts<<<nblk(3 * kH, 64), 256, 0, g->st>>>(g->part, eb, kH, kFe, g->grad, f.We[l] + 2 * kH, kEdgeIn, f.be[l]);
-        dense_dw(g, g->gr, g->h[l], g->h[l], n, kH, f.We[l], kEdgeIn, -1, kH, 0, tc);
-        dense_dw(g, g->gc, g->h[l], g->h[l], n, kH, f.We[l] + kH, kEdgeIn, -1, kH, 0, tc);
+        float* gc = g->grc + nh;
+        k_edge_grad<<<eb, 256, 0, g->st>>>(g->q, g->bits[l], g->ef, g->start, g->col, g->rev, n, g->grc, gc, g->part, tc);
+        k_reduce_parts<<<nblk(3 * kH, 32), 1024, 0, g->st>>>(g->part, eb, kH, kFe, g->grad, f.We[l] + 2 * kH, kEdgeIn, f.be[l]);
+        dense_dw(g, g->grc, g->h[l], g->h[l], n, kH, f.We[l], kEdgeIn, -1, kH, 0, tc, 2);
         // gh <- gh + (h half of gnin) + Gr W_r + Gc W_c
         const MatIndex ix = {1, kEdgeIn, kH, 0};
-        k_gemm<2 * kH><<<nblk(n, 64), 256, gemm_smem(2 * kH), g->st>>>(g->gr, g->gc, n, g->theta + f.We[l], ix, nullptr,
+        k_gemm<2 * kH><<<nblk(n, 64), 256, gemm_smem(2 * kH), g->st>>>(g->grc, gc, n, g->theta + f.We[l], ix, nullptr,
                                                                       g->gh2, nullptr, nullptr, 0, g->gh, g->gnin, tc);
         std::swap(g->gh, g->gh2);
     }
