@@ -342,19 +342,14 @@ void enqueue_dcd(AdmmB200* h, bool rebuild = true) {
     const int nq = s.nsv + s.nse;
     if (h->use_grid) {
         const int ne = s.nst + s.nse;
-        cudaMemsetAsync(s.grid.ctr, 0, sizeof(int) * 4, h->cstream);
+        LAUNCH(k_grid_count, blocks(ne, 256), 256, s);
         if (ne > 0) {
-            LAUNCH(k_grid_count, blocks(ne, 256), 256, s);
-            {
-                LaunchTimer lt(h, 0);
-                exclusive_scan(s.grid.cnt, s.grid.start, h->grid_buckets, s.scan_tmp, s.grid.start + h->grid_buckets,
-                               h->cstream, h->pdl);
-                h->launch_counter += 3;
-            }
+            LAUNCH(k_grid_alloc, scan_tiles(h->grid_buckets), kScanThreads, s, h->grid_buckets);
             LAUNCH(k_grid_scatter, blocks(ne, 256), 256, s);
         }
         if (nq > 0) launch_grid_query(h, false, nq);
     } else {
+        LAUNCH(k_contact_clear, h->contact_grid, kContactThreads, s);
         if (rebuild) {
             LAUNCH(k_scene_init, 1, 32, s.bf, s.be);
             enqueue_build(h, s.bf, (const int*)s.st, 4, true);
@@ -366,38 +361,18 @@ void enqueue_dcd(AdmmB200* h, bool rebuild = true) {
         if (s.nsv > 0) LAUNCH(k_dcd_vf<false>, blocks(s.nsv, 128), 128, s);
         if (s.nse > 0) LAUNCH(k_dcd_ee<false>, blocks(s.nse, 128), 128, s);
     }
-    if (nq > 0) {
-        LaunchTimer lt(h, 0);
-        exclusive_scan(s.qcount, s.qoff, nq, s.scan_tmp, s.nc_raw, h->cstream, h->pdl);
-        h->launch_counter += 3;
-    } else {
-        cudaMemsetAsync(s.nc_raw, 0, sizeof(int), h->cstream);
-    }
-    LAUNCH(k_set_count, 1, 1, s);
+    if (nq > 0) LAUNCH(k_scan_tiles, scan_tiles(nq), kScanThreads, (const int*)s.qcount, s.qoff, nq, s.scan_tmp);
+    LAUNCH(k_count_total, 1, kScanThreads, s, nq > 0 ? scan_tiles(nq) : 0);
     if (h->use_grid) {
         if (nq > 0) launch_grid_query(h, true, nq);
     } else {
         if (s.nsv > 0) LAUNCH_P(ADMM_KERNEL_DCD_VF, k_dcd_vf<true>, blocks(s.nsv, 128), 128, s);
         if (s.nse > 0) LAUNCH_P(ADMM_KERNEL_DCD_EE, k_dcd_ee<true>, blocks(s.nse, 128), 128, s);
     }
-    cudaMemsetAsync(s.vcnt, 0, sizeof(int) * s.n, h->cstream);
-    cudaMemsetAsync(s.vfill, 0, sizeof(int) * s.n, h->cstream);
-    LAUNCH(k_contact_count, h->contact_grid, kContactThreads, s);
-    {
-        LaunchTimer lt(h, 0);
-        exclusive_scan(s.vcnt, s.vstart, s.n, s.scan_tmp, s.vstart + s.n, h->cstream, h->pdl);
-        h->launch_counter += 3;
-    }
-    {
-        LaunchTimer lt(h, 0);
-        exclusive_scan(s.vcnt, s.tpos, s.n, s.scan_tmp, s.ntv, h->cstream, h->pdl, true);
-        h->launch_counter += 3;
-    }
-    LAUNCH(k_contact_touched, blocks(s.n, kContactThreads), kContactThreads, s);
-    LAUNCH(k_contact_fill, h->contact_grid, kContactThreads, s);
-    LAUNCH(k_contact_sort_lists, h->warp_grid, kContactThreads, s);
+    if (!h->use_grid) LAUNCH(k_contact_count, h->contact_grid, kContactThreads, s);
+    LAUNCH(k_contact_alloc, h->contact_grid, kContactThreads, s);
     LAUNCH(k_contact_scc, h->contact_grid, kContactThreads, s);
-    LAUNCH(k_contact_incidence, h->contact_grid, kContactThreads, s);
+    LAUNCH(k_contact_sort_lists, h->warp_grid, kContactThreads, s);
 }
 
 void enqueue_local(AdmmB200* h, int mode) {
@@ -1544,7 +1519,7 @@ int setup_grid(AdmmB200* h, const AdmmB200Desc* d) {
     h->grid_buckets = (int)nb;
     g.cap = (int)std::min<int64_t>(4 * ins + 4096, int64_t(1) << 30);
     TRY(dalloc(h, &g.cnt, nb));
-    TRY(dalloc(h, &g.start, nb + 1));
+    TRY(dalloc(h, &g.bkt, nb));
     TRY(dalloc(h, &g.ent_lo, g.cap));
     TRY(dalloc(h, &g.ent_up, g.cap));
     TRY(dalloc(h, &g.ent_key, g.cap));
@@ -1776,9 +1751,8 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     TRY(dalloc(h, &s.du2, s.cap));
     TRY(dalloc(h, &s.p2, n));
     TRY(dalloc(h, &s.vcnt, n));
-    TRY(dalloc(h, &s.vfill, n));
-    TRY(dalloc(h, &s.vstart, n + 1));
-    TRY(dalloc(h, &s.vlist, 4 * (size_t)s.cap));
+    TRY(dalloc(h, &s.vbeg, n));
+    TRY(dalloc(h, &s.crank, 4 * (size_t)s.cap));
     TRY(alloc_bvh(h, s.bf, s.nst));
     TRY(alloc_bvh(h, s.be, s.nse));
     TRY(dalloc(h, &s.qcount, s.nsv + s.nse + 1));
@@ -1807,8 +1781,7 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     }
 
     TRY(setup_grid(h, d));
-    const int scan_n = std::max(std::max(std::max(scan_tiles(hist_n), scan_tiles(n + 1)), scan_tiles(s.nsv + s.nse + 1)),
-                                scan_tiles(h->grid_buckets)) + 4;
+    const int scan_n = std::max(scan_tiles(hist_n), scan_tiles(s.nsv + s.nse + 1)) + 4;
     TRY(dalloc(h, &s.scan_tmp, scan_n));
     TRY(dalloc(h, &s.res, 4));
     TRY(dalloc(h, &s.done, 4));
@@ -1819,10 +1792,10 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     // 8 * 148 of them cost a quarter more per launch than 4 * 148
     h->pass_grid = std::max(1, std::min(blocks(s.cap * 32, kContactThreads), 3 * 148));
     h->warp_grid = std::max(1, std::min(blocks(std::min(n, 4 * s.cap) * 32, kContactThreads), 8 * 148));
-    TRY(dalloc(h, &s.tpos, n));
     TRY(dalloc(h, &s.tv, n));
     TRY(dalloc(h, &s.tvr, n));
     TRY(dalloc(h, &s.ntv, 1));
+    TRY(dalloc(h, &s.nalloc, 1));
 
     h->tet_blocks = s.ntet ? blocks(s.ntet, kLocalThreads) : 0;
     h->tri_blocks = s.ntri ? blocks(s.ntri, kLocalThreads) : 0;

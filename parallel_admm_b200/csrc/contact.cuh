@@ -13,71 +13,90 @@ ADMM_DEV int ccount(const DevScene& s) { return *s.nc; }
 
 ADMM_DEV float comp(float4 v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
 
-// per-vertex contact counts over all four vertices (updateContactCounts,
-// contact_solver.cu:90-101)
-__global__ void __launch_bounds__(kContactThreads) k_contact_count(DevScene s) {
-    ADMM_PDL_PROLOGUE();
-    const int nc = ccount(s);
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int4 q = s.pairs[c];
-        atomicAdd(&s.vcnt[q.x], 1);
-        atomicAdd(&s.vcnt[q.y], 1);
-        atomicAdd(&s.vcnt[q.z], 1);
-        atomicAdd(&s.vcnt[q.w], 1);
+// The incidence of a detection's contacts on the vertices: per-vertex counts over all four
+// vertices (updateContactCounts, contact_solver.cu:90-101), the vertices with contacts (tv, in no
+// particular order) and per contact corner its number among its vertex's contacts (crank), from
+// one atomic per corner; then a segment of ginc per vertex (k_contact_alloc, by an atomic per
+// warp), its entries (k_contact_scc, without atomics) and their order (k_contact_sort_lists).
+// The segments' and the list's places depend on the order of the atomics, nothing computed from
+// them does.  (Counted, scanned twice over all vertices, listed, filled and copied in incidence
+// order, a detection took 13 more launches.)
+ADMM_DEV void contact_touch(const DevScene& s, int c, int4 q) {
+    const int v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int r = atomicAdd(&s.vcnt[v[k]], 1);
+        s.crank[4 * c + k] = r;
+        if (r == 0) s.tv[atomicAdd(s.ntv, 1)] = v[k];
     }
 }
 
-// incidence slots (compute_Scc_kernel's CSR fill, contact_solver.cu:210-223)
-__global__ void __launch_bounds__(kContactThreads) k_contact_fill(DevScene s) {
+// After a write pass that does not do it itself (LBVH).
+__global__ void __launch_bounds__(kContactThreads) k_contact_count(DevScene s) {
     ADMM_PDL_PROLOGUE();
     const int nc = ccount(s);
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-        const int4 q = s.pairs[c];
-        const int v[4] = {q.x, q.y, q.z, q.w};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x)
+        contact_touch(s, c, s.pairs[c]);
+}
+
+// The counts of the last detection's vertices back to zero (thread `tid` of `threads`), before
+// this detection counts.
+ADMM_DEV void contact_clear(const DevScene& s, int tid, int threads) {
+    const int ntv = *s.ntv;
+    for (int t = tid; t < ntv; t += threads) s.vcnt[s.tv[t]] = 0;
+}
+
+__global__ void __launch_bounds__(kContactThreads) k_contact_clear(DevScene s) {
+    ADMM_PDL_PROLOGUE();
+    contact_clear(s, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
+// A segment of the incidence lists for every vertex with contacts: vbeg, and per list entry the
+// vertex with its bounds (tvr), which the gathers load in one round trip.  The grid's counters
+// are done with: back to zero for the next detection.
+__global__ void __launch_bounds__(kContactThreads) k_contact_alloc(DevScene s) {
+    ADMM_PDL_PROLOGUE();
+    if (s.grid.ctr && blockIdx.x == 0 && threadIdx.x < 4) s.grid.ctr[threadIdx.x] = 0;
+    const int lane = threadIdx.x & 31, ntv = *s.ntv;
+    for (int t0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31; t0 < ntv; t0 += gridDim.x * blockDim.x) {
+        const int t = t0 + lane, i = t < ntv ? s.tv[t] : 0, L = t < ntv ? s.vcnt[i] : 0;
+        int inc = L;
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const int pos = atomicAdd(&s.vfill[v[k]], 1);
-            s.vtmp[s.vstart[v[k]] + pos] = 4 * c + k;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        int base = 0;
+        if (lane == 31) base = atomicAdd(s.nalloc, inc);
+        const int b = __shfl_sync(0xffffffffu, base, 31) + inc - L;
+        if (t < ntv) {
+            s.vbeg[i] = b;
+            s.tvr[t] = make_int4(i, b, b + L, 0);
         }
     }
 }
 
-// Sort each vertex's incidence list by (contact, slot) so the gathers below
-// sum in a fixed order (the reference's order depends on atomics, F13).  The
-// fill leaves the lists unsorted in vtmp; one warp per vertex writes each key
-// to vlist at its rank (the keys are distinct), counted against the list held
-// in two registers per lane up to 64 keys, else read back from vtmp.  The lists
-// of static vertices are read by no gather: they are copied unsorted (a static
-// ground under an impact holds thousands of entries, and the quadratic sort of
-// those lists dominated the detection), so that vlist and the incidence entries
-// still cover every position.
+// Sort each dynamic vertex's incidence list by (contact, slot), so that the gathers sum in a
+// fixed order (the reference's order depends on atomics, F13), and write its incidence entries
+// (contact, Gamma_c,i), so that a gather needs no further indirection.  One warp per vertex places
+// each key at its rank (the keys are distinct), counted against the list held in two registers
+// per lane up to 64 keys, else read back from vtmp.  The lists of static vertices are read by no
+// gather and left out (a static ground under an impact holds thousands of entries).
 constexpr int kRankSortRegs = 64;
 
-// The vertices with contacts, ascending: tv[tpos[i]] = i for vcnt[i] > 0
-// (tpos = exclusive scan of vcnt != 0, *ntv = their number), and beside it the
-// vertex with its incidence-list bounds (tvr), which the gather loads in one
-// round trip.
-__global__ void __launch_bounds__(kContactThreads) k_contact_touched(DevScene s) {
-    ADMM_PDL_PROLOGUE();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < s.n && s.vcnt[i] > 0) {
-        const int t = s.tpos[i];
-        s.tv[t] = i;
-        s.tvr[t] = make_int4(i, s.vstart[i], s.vstart[i + 1], 0);
-    }
-}
-
-// One warp per vertex with contacts (grid-stride over the touched list).
 __global__ void __launch_bounds__(kContactThreads) k_contact_sort_lists(DevScene s) {
     ADMM_PDL_PROLOGUE();
     const int lane = threadIdx.x & 31;
     const int ntv = *s.ntv;
+    auto put = [&](int at, int key) {
+        const int c = key >> 2;
+        s.ginc[at] = make_float2(__int_as_float(c), comp(s.gamma[c], key & 3));
+    };
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntv; t += (gridDim.x * blockDim.x) >> 5) {
-        const int i = s.tv[t];
-        const int b = s.vstart[i], e = s.vstart[i + 1], L = e - b;
-        if (i >= s.nd) {
-            for (int m = lane; m < L; m += 32) s.vlist[b + m] = s.vtmp[b + m];
-        } else if (L <= kRankSortRegs) {
+        const int4 v = s.tvr[t];
+        const int b = v.y, L = v.z - v.y;
+        if (v.x >= s.nd) continue;
+        if (L <= kRankSortRegs) {
             const int k0 = lane < L ? s.vtmp[b + lane] : 0x7fffffff;
             const int k1 = lane + 32 < L ? s.vtmp[b + 32 + lane] : 0x7fffffff;
             int r0 = 0, r1 = 0;
@@ -86,21 +105,21 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_sort_lists(DevScene
                 r0 += kj < k0;
                 r1 += kj < k1;
             }
-            if (lane < L) s.vlist[b + r0] = k0;
-            if (lane + 32 < L) s.vlist[b + r1] = k1;
+            if (lane < L) put(b + r0, k0);
+            if (lane + 32 < L) put(b + r1, k1);
         } else {
             for (int m = lane; m < L; m += 32) {
                 const int key = s.vtmp[b + m];
                 int r = 0;
                 for (int j = 0; j < L; j++) r += s.vtmp[b + j] < key;
-                s.vlist[b + r] = key;
+                put(b + r, key);
             }
         }
     }
 }
 
 // S_c, Gamma_c, K_c, r_c = 0 (compute_Scc_kernel, contact_solver.cu:188-227;
-// the fills at 240-243).
+// the fills at 240-243) and the contact's entries in its vertices' lists (its CSR fill, 210-223).
 __global__ void __launch_bounds__(kContactThreads) k_contact_scc(DevScene s) {
     ADMM_PDL_PROLOGUE();
     const int nc = ccount(s);
@@ -132,20 +151,11 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_scc(DevScene s) {
         s.cmu[c] = mu;
         const int v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int k = 0; k < 4; k++) s.cinc[4 * c + k] = make_int4(v[k], s.vstart[v[k]], s.vstart[v[k] + 1], 0);
-    }
-}
-
-// Friction-cone projection of contact c (get_delta_u_kernel, contact_solver.cu:337-379).
-// Incidence entries in list order: (contact, Gamma_c,i) for every position of
-// the sorted lists, so that a gather needs no further indirection.
-__global__ void __launch_bounds__(kContactThreads) k_contact_incidence(DevScene s) {
-    ADMM_PDL_PROLOGUE();
-    const int n4 = 4 * ccount(s);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n4; k += gridDim.x * blockDim.x) {
-        const int slot = s.vlist[k];
-        const int c = slot >> 2;
-        s.ginc[k] = make_float2(__int_as_float(c), comp(s.gamma[c], slot & 3));
+        for (int k = 0; k < 4; k++) {
+            const int b = s.vbeg[v[k]];
+            s.vtmp[b + s.crank[4 * c + k]] = 4 * c + k;
+            s.cinc[4 * c + k] = make_int4(v[k], b, b + s.vcnt[v[k]], 0);
+        }
     }
 }
 

@@ -10,7 +10,7 @@
 //
 // Layout: every surface triangle and edge whose box spans at most kGridMaxSpan
 // cells per axis is inserted into each cell it overlaps, in a hash table of
-// (cell, type) buckets built by count -> scan -> scatter; each entry carries
+// (cell, type) buckets built by count -> place -> scatter; each entry carries
 // the element's box and the key of the cell it was entered for, so that other
 // cells sharing the bucket are rejected by one 8-byte compare and the box test
 // needs no further load.  Larger
@@ -29,6 +29,7 @@
 // atomic arrival order.
 #pragma once
 #include "common.cuh"
+#include "contact.cuh"
 #include "lbvh.cuh"
 #include "scene_dev.cuh"
 
@@ -126,11 +127,13 @@ ADMM_DEV void grid_for_cells(int3 a, int3 b, int type, int hmask, F f) {
 
 // Pass 1: bucket counts; elements that are too large (or beyond the entry
 // capacity) go to the big lists.  ctr[0] = entries reserved, ctr[1..2] = big
-// triangle / edge counts (zeroed before the launch).
+// triangle / edge counts (zero before the launch).  Also clears the last detection's contact
+// counts.
 __global__ void __launch_bounds__(256) k_grid_count(DevScene s) {
     ADMM_PDL_PROLOGUE();
     const GridDev& g = s.grid;
     const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    contact_clear(s, u, gridDim.x * blockDim.x);
     if (u >= s.nst + s.nse) return;
     int type, id;
     float4 lo, up;
@@ -153,7 +156,34 @@ __global__ void __launch_bounds__(256) k_grid_count(DevScene s) {
     }
 }
 
-// Pass 2 (after the scan of the counts into start): entries, one per element
+// The buckets' places among the entries: consecutive within a block's 2048 buckets, the blocks in
+// the order of their atomics (nothing depends on the entries' order: every query sorts its
+// partners).  A bucket's place and size are one load for the queries, and no launch waits for
+// a scan over all buckets.
+__global__ void __launch_bounds__(kScanThreads) k_grid_alloc(DevScene s, int buckets) {
+    ADMM_PDL_PROLOGUE();
+    __shared__ int sh[32];
+    __shared__ int first;
+    const GridDev& g = s.grid;
+    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    int v[kScanItems], t = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        v[k] = base + k < buckets ? g.cnt[base + k] : 0;
+        t += v[k];
+    }
+    int run = block_exclusive_scan(t, sh);
+    if (threadIdx.x == kScanThreads - 1) first = run + t ? atomicAdd(&g.ctr[3], run + t) : 0;
+    __syncthreads();
+    run += first;
+#pragma unroll
+    for (int k = 0; k < kScanItems; k++) {
+        if (base + k < buckets) g.bkt[base + k] = make_int2(run, v[k]);
+        run += v[k];
+    }
+}
+
+// Pass 2: entries, one per element
 // and cell; the counts are consumed back to zero for the next DCD.
 __global__ void __launch_bounds__(256) k_grid_scatter(DevScene s) {
     ADMM_PDL_PROLOGUE();
@@ -167,7 +197,7 @@ __global__ void __launch_bounds__(256) k_grid_scatter(DevScene s) {
     grid_range(lo, up, g.inv_c, a, b);
     lo.w = __int_as_float(id);
     grid_for_cells(a, b, type, g.hmask, [&](int4 c, int bk) {
-        const int pos = g.start[bk] + atomicSub(&g.cnt[bk], 1) - 1;
+        const int pos = g.bkt[bk].x + atomicSub(&g.cnt[bk], 1) - 1;
         // w of up: for each axis, whether this cell is the element's first
         const int first = (c.x == a.x ? 1 : 0) | (c.y == a.y ? 2 : 0) | (c.z == a.z ? 4 : 0);
         g.ent_lo[pos] = lo;
@@ -319,8 +349,9 @@ ADMM_DEV void grid_walk(const DevScene& s, const QueryGroup<G>& grp, bool vf, in
                 if (c0 + sub < nc) {
                     const int3 c = grid_cell_at(a, b, c0 + sub);
                     const int bk = grid_bucket(c.x, c.y, c.z, type, g.hmask);
-                    d = g.start[bk];
-                    cnt = g.start[bk + 1] - d;
+                    const int2 e = g.bkt[bk];
+                    d = e.x;
+                    cnt = e.y;
                     key = grid_cell_key(c.x, c.y, c.z);
                     qfirst = (c.x == a.x ? 1 : 0) | (c.y == a.y ? 2 : 0) | (c.z == a.z ? 4 : 0);
                 }
@@ -519,7 +550,7 @@ ADMM_DEV bool grid_hit_ee(const DevScene& s, int e, int o, int4& ids, NpResult& 
 // The write pass places each recorded partner at qoff + its rank among the
 // query's partners, so the segment comes out sorted by partner; a query with
 // more partners than were recorded walks the grid again, writes in walk order
-// and sorts its segment.
+// and sorts its segment.  The write pass also counts the contacts' vertices.
 template <bool WRITE, int G>
 ADMM_DEV void grid_query(DevScene& s) {
     ADMM_PDL_PROLOGUE();
@@ -556,7 +587,7 @@ ADMM_DEV void grid_query(DevScene& s) {
     }
     const int total = s.qcount[q];
     if (total == 0) return;
-    const int base = s.qoff[q];
+    const int base = query_offset(s, q);
     if (total <= kQueryHitsMax) {
         for (int k = grp.sub; k < total; k += G) {
             const int partner = qh[k];
@@ -566,7 +597,10 @@ ADMM_DEV void grid_query(DevScene& s) {
             NpResult r;
             const bool hit = vf ? grid_hit_vf(s, v, lo, partner, ids, r) : grid_hit_ee(s, e, partner, ids, r);
             const int slot = base + rank;
-            if (hit && slot < s.cap) write_contact(s, slot, ids, r, !vf);
+            if (hit && slot < s.cap) {
+                write_contact(s, slot, ids, r, !vf);
+                contact_touch(s, slot, ids);
+            }
         }
         return;
     }
@@ -584,10 +618,10 @@ ADMM_DEV void grid_query(DevScene& s) {
     };
     grid_walk(s, grp, vf, e, lo, up, gq, emit);
     __syncwarp(grp.mask);
-    if (grp.sub == 0) {
-        const int end = min(base + total, s.cap);
-        if (end - base > 1) grid_sort_segment(s, base, end);
-    }
+    const int end = min(base + total, s.cap);
+    if (grp.sub == 0 && end - base > 1) grid_sort_segment(s, base, end);
+    __syncwarp(grp.mask);
+    for (int c = base + grp.sub; c < end; c += G) contact_touch(s, c, s.pairs[c]);
 }
 
 template <bool WRITE, int G>

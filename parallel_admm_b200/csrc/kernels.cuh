@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(kVertThreads) k_contact_p(DevScene s, int spli
     ADMM_PDL_WAIT_THEN_TRIGGER();
     if ((int)blockIdx.x < split) {
         const int i = blockIdx.x * blockDim.x + threadIdx.x;
-        if (i < s.nd && s.vstart[i] == s.vstart[i + 1]) s.p[i] = contact_p_base<DUALC>(s, i);
+        if (i < s.nd && s.vcnt[i] == 0) s.p[i] = contact_p_base<DUALC>(s, i);
         return;
     }
     const int sub = threadIdx.x % kGatherLanes;

@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(128) k_dcd_vf(DevScene s) {
     const float4 P = s.x[v];
     const float gap = s.thickness;
     int count = 0;
-    const int base = WRITE ? s.qoff[q] : 0;
+    const int base = WRITE ? query_offset(s, q) : 0;
     int stack[kStackDepth];
     int sp = 0;
     const int n = t.n;
@@ -549,7 +549,7 @@ __global__ void __launch_bounds__(128) k_dcd_ee(DevScene s) {
     box_add(lo, up, A1);
     const float gap = s.thickness;
     int count = 0;
-    const int base = WRITE ? s.qoff[s.nsv + e] : 0;
+    const int base = WRITE ? query_offset(s, s.nsv + e) : 0;
     int stack[kStackDepth];
     int sp = 0;
     const int n = t.n;
@@ -594,14 +594,6 @@ __global__ void __launch_bounds__(128) k_dcd_ee(DevScene s) {
         }
     }
     if (!WRITE) s.qcount[s.nsv + e] = count;
-}
-
-// nc = min(total, cap); overflow flag.
-__global__ void k_set_count(DevScene s) {
-    ADMM_PDL_PROLOGUE();
-    const int raw = *s.nc_raw;
-    *s.nc = raw < s.cap ? raw : s.cap;
-    if (raw > s.cap) s.err[0] = 1;
 }
 
 }  // namespace admm

@@ -3,6 +3,7 @@
 // call, unlike the reference's thrust::sort_by_key, lbvh.cu:1473-1474).
 #pragma once
 #include "common.cuh"
+#include "scene_dev.cuh"
 
 namespace admm {
 
@@ -38,9 +39,7 @@ ADMM_DEV int block_exclusive_scan(int v, int* sh_warp) {
     return r;
 }
 
-// Phase 1: per-tile exclusive scan in place (out) and tile totals.  FLAGS
-// scans (in[i] != 0) instead of in[i].
-template <bool FLAGS>
+// Phase 1: per-tile exclusive scan in place (out) and tile totals.
 __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* __restrict__ in, int* __restrict__ out,
                                                             int n, int* __restrict__ tile_sums) {
     ADMM_PDL_PROLOGUE();
@@ -51,7 +50,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* __restri
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
         v[k] = (base + k < n) ? in[base + k] : 0;
-        if (FLAGS) v[k] = v[k] != 0;
         t += v[k];
     }
     const int off = block_exclusive_scan(t, sh);
@@ -86,6 +84,38 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(int* __restrict__ ti
     if (threadIdx.x == 0 && total) *total = carry;
 }
 
+// Phase 2 of the queries' scan: the tile offsets stay in tile_sums (query_offset adds them), the
+// total becomes the contact count, clamped to the capacity, and the counters of the incidence
+// lists start from zero.
+__global__ void __launch_bounds__(kScanThreads) k_count_total(DevScene s, int ntiles) {
+    ADMM_PDL_PROLOGUE();
+    __shared__ int sh[32];
+    __shared__ int carry;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (int base = 0; base < ntiles; base += kScanThreads) {
+        const int i = base + threadIdx.x;
+        const int v = i < ntiles ? s.scan_tmp[i] : 0;
+        const int ex = block_exclusive_scan(v, sh);
+        const int c = carry;
+        if (i < ntiles) s.scan_tmp[i] = ex + c;
+        __syncthreads();
+        if (threadIdx.x == kScanThreads - 1) carry = c + ex + v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const int raw = carry;
+        *s.nc_raw = raw;
+        *s.nc = raw < s.cap ? raw : s.cap;
+        if (raw > s.cap) s.err[0] = 1;
+        *s.ntv = 0;
+        *s.nalloc = 0;
+    }
+}
+
+// First contact slot of query q.
+ADMM_DEV int query_offset(const DevScene& s, int q) { return s.qoff[q] + s.scan_tmp[q / kScanTile]; }
+
 // Phase 3: add tile offsets.
 __global__ void __launch_bounds__(kScanThreads) k_scan_add(int* __restrict__ out, int n,
                                                           const int* __restrict__ tile_sums) {
@@ -99,14 +129,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_add(int* __restrict__ out
 
 inline int scan_tiles(int n) { return (n + kScanTile - 1) / kScanTile; }
 
-// exclusive scan of n ints: out[i] = sum_{j<i} in[j] (flags: of in[j] != 0);
+// exclusive scan of n ints: out[i] = sum_{j<i} in[j];
 // *total = sum (device).  tmp needs scan_tiles(n) ints.  in and out may alias.
-inline void exclusive_scan(const int* in, int* out, int n, int* tmp, int* total, cudaStream_t st, bool pdl = false,
-                           bool flags = false) {
+inline void exclusive_scan(const int* in, int* out, int n, int* tmp, int* total, cudaStream_t st, bool pdl = false) {
     if (n <= 0) return;
     const int nt = scan_tiles(n);
-    if (flags) launch_k(k_scan_tiles<true>, dim3(nt), dim3(kScanThreads), 0, st, pdl, in, out, n, tmp);
-    else launch_k(k_scan_tiles<false>, dim3(nt), dim3(kScanThreads), 0, st, pdl, in, out, n, tmp);
+    launch_k(k_scan_tiles, dim3(nt), dim3(kScanThreads), 0, st, pdl, in, out, n, tmp);
     launch_k(k_scan_sums, dim3(1), dim3(kScanThreads), 0, st, pdl, tmp, nt, total);
     launch_k(k_scan_add, dim3(nt), dim3(kScanThreads), 0, st, pdl, out, n, (const int*)tmp);
 }

@@ -67,11 +67,11 @@ struct GridDev {
     int hmask = 0;                 // buckets - 1 (power of two)
     int cap = 0;                   // entry capacity
     int* cnt = nullptr;            // [buckets] entries per bucket (zero between DCDs)
-    int* start = nullptr;          // [buckets + 1] bucket offsets
+    int2* bkt = nullptr;           // [buckets] first entry and number of entries of a bucket
     float4* ent_lo = nullptr;      // [cap] element box lo, w = element index (int bits)
     float4* ent_up = nullptr;      // [cap] element box up, w = first-cell bits (x 1, y 2, z 4)
     unsigned long long* ent_key = nullptr;  // [cap] key of the cell the entry was made for
-    int* ctr = nullptr;            // [4] entries reserved, big triangles, big edges
+    int* ctr = nullptr;            // [4] entries reserved, big triangles, big edges, entries placed (zero between DCDs)
     int* big_tri = nullptr;        // [n surface triangles]
     int* big_edge = nullptr;       // [n surface edges]
     int* mode = nullptr;           // [triangles + edges] 1 = in the grid, 0 = big list
@@ -137,14 +137,13 @@ struct DevScene {
     float4* du2 = nullptr;  // [cap] second buffer of the fused projection passes
     float4* p2 = nullptr;   // [n] second buffer of p in the fused projection passes
     int* vcnt = nullptr;                  // [n] contacts per vertex
-    int* vfill = nullptr;                 // [n]
-    int* vstart = nullptr;                // [n+1]
-    int* vlist = nullptr;                 // [4*cap] contact*4 + slot, sorted per vertex
-    float2* ginc = nullptr;               // [4*cap] (contact as int bits, Gamma_c,i) in list order
-    int* vtmp = nullptr;                  // [4*cap] incidence lists before sorting
-    int* tpos = nullptr;                  // [n] position of a vertex in the touched list
-    int* tv = nullptr;                    // [n] vertices with contacts, ascending
+    int* vbeg = nullptr;                  // [n] first entry of the vertex's incidence list (vertices with contacts)
+    int* crank = nullptr;                 // [4*cap] number of a contact corner among its vertex's contacts
+    float2* ginc = nullptr;               // [4*cap] (contact as int bits, Gamma_c,i), sorted per dynamic vertex
+    int* vtmp = nullptr;                  // [4*cap] incidence lists (4 * contact + slot) before sorting
+    int* tv = nullptr;                    // [n] vertices with contacts
     int* ntv = nullptr;                   // [1] their number
+    int* nalloc = nullptr;                // [1] incidence entries handed out
     int4* cinc = nullptr;                 // [4*cap] per contact corner: (vertex, list begin, list end, 0)
     int4* tvr = nullptr;                  // [n] per touched vertex, in tv order: (vertex, list begin, list end, 0)
     // collision geometry
@@ -155,8 +154,8 @@ struct DevScene {
     BvhDev bf, be;                        // face tree, edge tree
     GridDev grid;                         // uniform-grid broad phase
     int* qcount = nullptr;                // [nsv + nse] per-query pair counts
-    int* qoff = nullptr;                  // [nsv + nse + 1] exclusive offsets
-    int* scan_tmp = nullptr;              // block sums for scans
+    int* qoff = nullptr;                  // [nsv + nse + 1] exclusive offsets within a scan tile
+    int* scan_tmp = nullptr;              // block sums for scans; after the queries' scan, tile offsets
     // residuals: [0] primal^2, [1] dual^2, [2] scale^2
     double* res = nullptr;
     double* res_part = nullptr;           // [3 x residual blocks] per-block partial sums
