@@ -73,7 +73,8 @@ struct AdmmB200 {
     LearnDev learn;
     int learn_sweeps = 0;
     std::vector<float> learn_omega, learn_beta;
-    int* fail_host = nullptr;       // pinned copy of learn.fail (eager substeps)
+    int* fail_host = nullptr;       // pinned: learn.fail (eager substeps)
+    int* status_host = nullptr;     // pinned copy of the status words (err, nc, nc_raw)
     int64_t learn_substeps = 0;
     int kernels_fallback = 0;       // kernels of the plain solve that replaces a failed learned one
     cudaStream_t if_stream = nullptr;  // capture of the bodies of the fallback IF nodes
@@ -125,7 +126,8 @@ struct AdmmB200 {
     float tune_ms_tiled = 0.f;
     float tune_ms_persist = 0.f, tune_ms_sweeps = 0.f;  // one global step, both modes
     // host-buffer stepping
-    float* stage = nullptr;    // [6n] row-major x then v
+    float* stage = nullptr;    // row-major host rows on their way to or from the device
+    size_t stage_floats = 0;
     // profiling: eager launches with one event pair per launch, tagged by phase
     bool profiling = false;
     int phase = 0;
@@ -234,6 +236,8 @@ int alloc_bvh(AdmmB200* h, BvhDev& t, int n) {
     TRY(dalloc(h, &t.node4, n > 1 ? 4 * (size_t)(n - 1) : 4));
     return ADMM_OK;
 }
+
+constexpr int kStatusWords = 8;  // err[4], nc, nc_raw
 
 // ------------------------------ enqueue helpers -----------------------------
 constexpr int kMaxProfEvents = 1 << 14;
@@ -1726,9 +1730,9 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
         s.st = a; s.se = b; s.sv = c;
     }
     s.cap = d->enable_contact ? d->max_contacts : 1;
-    TRY(dalloc(h, &s.nc, 1));
-    TRY(dalloc(h, &s.nc_raw, 1));
-    TRY(dalloc(h, &s.err, 4));
+    TRY(dalloc(h, &s.err, kStatusWords));  // the words that every step reports, in one copy
+    s.nc = s.err + 4;
+    s.nc_raw = s.err + 5;
     TRY(dalloc(h, &s.pairs, s.cap));
     TRY(dalloc(h, &s.bary, s.cap));
     TRY(dalloc(h, &s.nrm, s.cap));
@@ -1865,6 +1869,7 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
         TRY(dalloc(h, &L.fail, 1));
         TRY(dalloc(h, &L.warm, 1));
         CK(cudaHostAlloc((void**)&h->fail_host, sizeof(int), cudaHostAllocDefault));
+        CK(cudaHostAlloc((void**)&h->status_host, sizeof(int) * kStatusWords, cudaHostAllocDefault));
         h->learn_sweeps = std::max(1, h->jac_iter);
         h->learn_omega.assign(h->learn_sweeps, 1.f);
         h->learn_beta.assign(h->learn_sweeps, 0.f);
@@ -1919,6 +1924,90 @@ __global__ void k_pack_state(DevScene s, float* __restrict__ stage, const int* _
     stage[3 * s.n + 3 * c] = v.x; stage[3 * s.n + 3 * c + 1] = v.y; stage[3 * s.n + 3 * c + 2] = v.z;
 }
 
+// Rows [first, first + n) of a float4 buffer to row-major n x 3 floats, or back (w = 0); perm[i] =
+// the caller's row of internal row i (whole per-vertex buffers only; null: identity).
+__global__ void k_pack_rows(const float4* __restrict__ src, int first, int n, float* __restrict__ out,
+                            const int* __restrict__ perm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 v = src[first + i];
+    const size_t c = 3 * (size_t)(perm ? perm[i] : i);
+    out[c] = v.x;
+    out[c + 1] = v.y;
+    out[c + 2] = v.z;
+}
+
+__global__ void k_unpack_rows(const float* __restrict__ in, int first, int n, float4* __restrict__ dst,
+                              const int* __restrict__ perm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t c = 3 * (size_t)(perm ? perm[i] : i);
+    dst[first + i] = make_float4(in[c], in[c + 1], in[c + 2], 0.f);
+}
+
+// y = z - Ue, the right-hand side's operand
+__global__ void k_elastic_y(DevScene s) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= s.m) return;
+    const float4 z = s.z[i], u = s.ue[i];
+    s.y[i] = make_float4(z.x - u.x, z.y - u.y, z.z - u.z, 0.f);
+}
+
+// Contacts [first, first + n): pair, bary, normal and gap, point as one 64-byte record each.
+__global__ void k_pack_contacts(DevScene s, int first, int n, float4* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int4 q = s.pairs[first + i];
+    out[4 * (size_t)i] = make_float4(__int_as_float(q.x), __int_as_float(q.y), __int_as_float(q.z), __int_as_float(q.w));
+    out[4 * (size_t)i + 1] = s.bary[first + i];
+    out[4 * (size_t)i + 2] = s.nrm[first + i];
+    out[4 * (size_t)i + 3] = s.point[first + i];
+}
+
+// At least `floats` floats of staging (not in use: the callers wait for the stream).
+int grow_stage(AdmmB200* h, size_t floats) {
+    if (h->stage_floats >= floats) return ADMM_OK;
+    CK(cudaStreamSynchronize(h->stream));
+    cudaFree(h->stage);
+    h->stage = nullptr;
+    h->stage_floats = 0;
+    CK(cudaMalloc((void**)&h->stage, floats * sizeof(float)));
+    h->stage_floats = floats;
+    return ADMM_OK;
+}
+
+// Rows of at most so many floats pass through the staging at a time (per-vertex buffers whole:
+// their rows may be permuted).
+constexpr size_t kStageFloats = (size_t)3 << 22;
+
+// A float4 buffer of `rows` rows to (read) or from (write) the caller's row-major rows, converted on
+// the device: a fourth less over the bus than the float4 rows, and no pass over them on the host.
+int read_rows(AdmmB200* h, const float4* src, int rows, bool per_vertex, float* out) {
+    const int step = per_vertex ? rows : (int)std::min<size_t>(rows, kStageFloats / 3);
+    if (rows <= 0) return ADMM_OK;
+    TRY(grow_stage(h, 3 * (size_t)step));
+    for (int r = 0; r < rows; r += step) {
+        const int n = std::min(step, rows - r);
+        k_pack_rows<<<blocks(n, 256), 256, 0, h->stream>>>(src, r, n, h->stage, per_vertex ? h->d_perm : nullptr);
+        CK(cudaMemcpyAsync(out + 3 * (size_t)r, h->stage, sizeof(float) * 3 * (size_t)n, cudaMemcpyDeviceToHost, h->stream));
+    }
+    CK(cudaStreamSynchronize(h->stream));
+    return ADMM_OK;
+}
+
+int write_rows(AdmmB200* h, float4* dst, int rows, bool per_vertex, const float* in) {
+    const int step = per_vertex ? rows : (int)std::min<size_t>(rows, kStageFloats / 3);
+    if (rows <= 0) return ADMM_OK;
+    TRY(grow_stage(h, 3 * (size_t)step));
+    for (int r = 0; r < rows; r += step) {
+        const int n = std::min(step, rows - r);
+        CK(cudaMemcpyAsync(h->stage, in + 3 * (size_t)r, sizeof(float) * 3 * (size_t)n, cudaMemcpyHostToDevice, h->stream));
+        k_unpack_rows<<<blocks(n, 256), 256, 0, h->stream>>>(h->stage, r, n, dst, per_vertex ? h->d_perm : nullptr);
+    }
+    CK(cudaGetLastError());
+    return ADMM_OK;
+}
+
 int accumulate_timers(AdmmB200* h) {
     if (h->profiling) {
         for (int k = 0; k + 1 < h->prof_used; k += 2) {
@@ -1950,9 +2039,12 @@ int accumulate_timers(AdmmB200* h) {
     return ADMM_OK;
 }
 
-int read_err_flags(AdmmB200* h, int* status) {
-    int e[4] = {0, 0, 0, 0};
-    CK(cudaMemcpy(e, h->s.err, sizeof(e), cudaMemcpyDeviceToHost));
+// Waits for the stream; the status of what ran on it (cleared on the device) and, in
+// h->status_host, the contact counts (4: stored, 5: found).
+int read_status(AdmmB200* h, int* status) {
+    int* e = h->status_host;
+    CK(cudaMemcpyAsync(e, h->s.err, sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
     if (e[0] || e[1] || e[2] || e[3]) CK(cudaMemset(h->s.err, 0, sizeof(int) * 4));
     // after a timed-out wait the blocks' sweep counters disagree: start them again from 0
     if (e[3] && h->pp.epoch) CK(cudaMemset(h->pp.epoch, 0, sizeof(unsigned) * h->pp.blocks));
@@ -2180,6 +2272,8 @@ void admm_b200_destroy(AdmmB200* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
     if (h->fail_host) cudaFreeHost(h->fail_host);
+    if (h->status_host) cudaFreeHost(h->status_host);
+    cudaFree(h->stage);
     for (void* p : h->allocs)
         if (p) cudaFree(p);
     for (auto e : h->prof_ev) cudaEventDestroy(e);
@@ -2232,15 +2326,13 @@ int admm_b200_step(AdmmB200* h, int n_steps, AdmmStepStats* stats) {
     if (!h) return ADMM_ERR_INVALID;
     const auto t0 = std::chrono::steady_clock::now();
     TRY(admm_b200_step_async(h, n_steps));
-    CK(cudaStreamSynchronize(h->stream));
+    int status = ADMM_OK;
+    TRY(read_status(h, &status));
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
     h->last_ms = n_steps > 0 ? ms / n_steps : 0.f;
     if (!h->profiling) TRY(accumulate_timers(h));
-    int status = ADMM_OK;
-    TRY(read_err_flags(h, &status));
-    int nc = 0;
-    CK(cudaMemcpy(&nc, h->s.nc, sizeof(int), cudaMemcpyDeviceToHost));
+    const int nc = h->status_host[4];
     h->peak = std::max(h->peak, nc);
     h->last_iters = h->admm_max_iter;
     if (h->residual_tol > 0.f) CK(cudaMemcpy(&h->last_iters, h->s.done, sizeof(int), cudaMemcpyDeviceToHost));
@@ -2265,36 +2357,22 @@ int admm_b200_set_state(AdmmB200* h, const float* x, const float* v, int n) {
     if (!h || !x) return ADMM_ERR_INVALID;
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
-    std::vector<float4> hx(n), hv(n, make_float4(0.f, 0.f, 0.f, 0.f));
-    for (int i = 0; i < n; i++) {
-        const int c = caller_of(h, i);
-        hx[i] = pack(x + 3 * c);
-        if (v) hv[i] = pack(v + 3 * c);
-    }
+    DevScene& d = h->s;
+    TRY(write_rows(h, d.x0, n, true, x));
+    CK(cudaMemcpyAsync(d.x, d.x0, sizeof(float4) * n, cudaMemcpyDeviceToDevice, h->stream));
+    if (v) TRY(write_rows(h, d.v, n, true, v));
+    else CK(cudaMemsetAsync(d.v, 0, sizeof(float4) * n, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    return upload_state(h, hx, hv);
+    return ADMM_OK;
 }
 
 int admm_b200_get_state(AdmmB200* h, float* x, float* v, int n) {
     if (!h) return ADMM_ERR_INVALID;
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
-    std::vector<float4> tmp(n);
-    CK(cudaStreamSynchronize(h->stream));
-    if (x) {
-        CK(cudaMemcpy(tmp.data(), h->s.x0, sizeof(float4) * n, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < n; i++) {
-            const int c = caller_of(h, i);
-            x[3 * c] = tmp[i].x; x[3 * c + 1] = tmp[i].y; x[3 * c + 2] = tmp[i].z;
-        }
-    }
-    if (v) {
-        CK(cudaMemcpy(tmp.data(), h->s.v, sizeof(float4) * n, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < n; i++) {
-            const int c = caller_of(h, i);
-            v[3 * c] = tmp[i].x; v[3 * c + 1] = tmp[i].y; v[3 * c + 2] = tmp[i].z;
-        }
-    }
+    if (x) TRY(read_rows(h, h->s.x0, n, true, x));
+    if (v) TRY(read_rows(h, h->s.v, n, true, v));
+    if (!x && !v) CK(cudaStreamSynchronize(h->stream));
     return ADMM_OK;
 }
 
@@ -2401,15 +2479,7 @@ int admm_b200_read_buffer(AdmmB200* h, int which, float* out, int n) {
     float4* p = buffer_ptr(h, which, &rows);
     if (!p || n != rows) return fail(h, ADMM_ERR_INVALID, "buffer id or row count");
     CK(cudaSetDevice(h->device));
-    CK(cudaStreamSynchronize(h->stream));
-    std::vector<float4> tmp(rows);
-    CK(cudaMemcpy(tmp.data(), p, sizeof(float4) * rows, cudaMemcpyDeviceToHost));
-    const bool pv = per_vertex_buffer(which);
-    for (int i = 0; i < rows; i++) {
-        const int c = pv ? caller_of(h, i) : i;
-        out[3 * c] = tmp[i].x; out[3 * c + 1] = tmp[i].y; out[3 * c + 2] = tmp[i].z;
-    }
-    return ADMM_OK;
+    return read_rows(h, p, rows, per_vertex_buffer(which), out);
 }
 
 int admm_b200_write_buffer(AdmmB200* h, int which, const float* in, int n) {
@@ -2418,19 +2488,10 @@ int admm_b200_write_buffer(AdmmB200* h, int which, const float* in, int n) {
     float4* p = buffer_ptr(h, which, &rows);
     if (!p || n != rows) return fail(h, ADMM_ERR_INVALID, "buffer id or row count");
     CK(cudaSetDevice(h->device));
+    TRY(write_rows(h, p, rows, per_vertex_buffer(which), in));
+    if (which == ADMM_BUF_Z || which == ADMM_BUF_UE) k_elastic_y<<<blocks(h->s.m, 256), 256, 0, h->stream>>>(h->s);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
-    std::vector<float4> tmp(rows);
-    const bool pv = per_vertex_buffer(which);
-    for (int i = 0; i < rows; i++) tmp[i] = pack(in + 3 * (pv ? caller_of(h, i) : i));
-    CK(cudaMemcpy(p, tmp.data(), sizeof(float4) * rows, cudaMemcpyHostToDevice));
-    if (which == ADMM_BUF_Z || which == ADMM_BUF_UE) {
-        // keep y = z - Ue consistent for the right-hand side
-        std::vector<float4> z(h->s.m), ue(h->s.m);
-        CK(cudaMemcpy(z.data(), h->s.z, sizeof(float4) * h->s.m, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(ue.data(), h->s.ue, sizeof(float4) * h->s.m, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < h->s.m; i++) z[i] = make_float4(z[i].x - ue[i].x, z[i].y - ue[i].y, z[i].z - ue[i].z, 0.f);
-        CK(cudaMemcpy(h->s.y, z.data(), sizeof(float4) * h->s.m, cudaMemcpyHostToDevice));
-    }
     return ADMM_OK;
 }
 
@@ -2476,15 +2537,11 @@ int admm_b200_detect(AdmmB200* h, int* count) {
     CK(cudaSetDevice(h->device));
     enqueue_dcd(h);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(h->stream));
-    int raw = 0, nc = 0;
-    CK(cudaMemcpy(&raw, h->s.nc_raw, sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(&nc, h->s.nc, sizeof(int), cudaMemcpyDeviceToHost));
-    h->peak = std::max(h->peak, nc);
-    h->detected = true;
-    if (count) *count = raw;
     int status = ADMM_OK;
-    TRY(read_err_flags(h, &status));
+    TRY(read_status(h, &status));
+    h->peak = std::max(h->peak, h->status_host[4]);
+    h->detected = true;
+    if (count) *count = h->status_host[5];
     return status;
 }
 
@@ -2492,10 +2549,7 @@ int admm_b200_detect_host(AdmmB200* h, const float* x, int n, int* count) {
     if (!h || !x) return ADMM_ERR_INVALID;
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
-    std::vector<float4> hx(n);
-    for (int i = 0; i < n; i++) hx[i] = pack(x + 3 * caller_of(h, i));
-    CK(cudaStreamSynchronize(h->stream));
-    CK(cudaMemcpy(h->s.x, hx.data(), sizeof(float4) * n, cudaMemcpyHostToDevice));
+    TRY(write_rows(h, h->s.x, n, true, x));
     return admm_b200_detect(h, count);
 }
 
@@ -2514,29 +2568,34 @@ int admm_b200_contacts(AdmmB200* h, int32_t* pairs, float* bary4, float* normal3
                        int cap, int* count) {
     if (!h) return ADMM_ERR_INVALID;
     CK(cudaSetDevice(h->device));
+    CK(cudaMemcpyAsync(h->status_host + 4, h->s.nc, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    int nc = 0;
-    CK(cudaMemcpy(&nc, h->s.nc, sizeof(int), cudaMemcpyDeviceToHost));
+    const int nc = h->status_host[4];
     if (count) *count = nc;
     const int k = std::min(nc, std::max(cap, 0));
     if (k == 0) return ADMM_OK;
-    if (pairs) {
-        CK(cudaMemcpy(pairs, h->s.pairs, sizeof(int4) * k, cudaMemcpyDeviceToHost));
-        if (!h->perm.empty())
-            for (int i = 0; i < 4 * k; i++) pairs[i] = h->perm[pairs[i]];
-    }
-    std::vector<float4> tmp(k);
-    if (bary4) CK(cudaMemcpy(bary4, h->s.bary, sizeof(float4) * k, cudaMemcpyDeviceToHost));
-    if (normal3 || gap) {
-        CK(cudaMemcpy(tmp.data(), h->s.nrm, sizeof(float4) * k, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < k; i++) {
-            if (normal3) { normal3[3 * i] = tmp[i].x; normal3[3 * i + 1] = tmp[i].y; normal3[3 * i + 2] = tmp[i].z; }
-            if (gap) gap[i] = tmp[i].w;
+    if (!pairs && !bary4 && !normal3 && !point3 && !gap) return ADMM_OK;
+    const int step = std::min(k, 1 << 16);
+    TRY(grow_stage(h, 16 * (size_t)step));
+    std::vector<float> rec(16 * (size_t)step);
+    for (int f = 0; f < k; f += step) {
+        const int m = std::min(step, k - f);
+        k_pack_contacts<<<blocks(m, 256), 256, 0, h->stream>>>(h->s, f, m, (float4*)h->stage);
+        CK(cudaMemcpyAsync(rec.data(), h->stage, sizeof(float) * 16 * (size_t)m, cudaMemcpyDeviceToHost, h->stream));
+        CK(cudaStreamSynchronize(h->stream));
+        for (int i = 0; i < m; i++) {
+            const float* r = rec.data() + 16 * (size_t)i;
+            const size_t c = (size_t)f + i;
+            if (pairs) {
+                std::memcpy(pairs + 4 * c, r, 16);
+                if (!h->perm.empty())
+                    for (int t = 0; t < 4; t++) pairs[4 * c + t] = h->perm[pairs[4 * c + t]];
+            }
+            if (bary4) std::memcpy(bary4 + 4 * c, r + 4, 16);
+            if (normal3) std::memcpy(normal3 + 3 * c, r + 8, 12);
+            if (gap) gap[c] = r[11];
+            if (point3) std::memcpy(point3 + 3 * c, r + 12, 12);
         }
-    }
-    if (point3) {
-        CK(cudaMemcpy(tmp.data(), h->s.point, sizeof(float4) * k, cudaMemcpyDeviceToHost));
-        for (int i = 0; i < k; i++) { point3[3 * i] = tmp[i].x; point3[3 * i + 1] = tmp[i].y; point3[3 * i + 2] = tmp[i].z; }
     }
     return ADMM_OK;
 }
@@ -2603,7 +2662,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     if (!h || !x_in) return ADMM_ERR_INVALID;
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
-    if (!h->stage) TRY(dalloc(h, &h->stage, (size_t)6 * n));
+    TRY(grow_stage(h, (size_t)6 * n));
     TRY(build_step_graph(h));
     const size_t bytes = sizeof(float) * 3 * (size_t)n;
     CK(cudaMemcpyAsync(h->stage, x_in, bytes, cudaMemcpyHostToDevice, h->stream));
@@ -2613,10 +2672,9 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     k_pack_state<<<blocks(n, 256), 256, 0, h->stream>>>(h->s, h->stage, h->d_perm);
     if (x_out) CK(cudaMemcpyAsync(x_out, h->stage, bytes, cudaMemcpyDeviceToHost, h->stream));
     if (v_out) CK(cudaMemcpyAsync(v_out, h->stage + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     h->frame += 1;
     int status = ADMM_OK;
-    TRY(read_err_flags(h, &status));
+    TRY(read_status(h, &status));
     return status;
 }
 
