@@ -22,6 +22,7 @@
 #include "admm_b200.h"
 #include "animate.cuh"
 #include "contact.cuh"
+#include "contact_one.cuh"
 #include "grid.cuh"
 #include "kernels.cuh"
 #include "lbvh.cuh"
@@ -54,6 +55,14 @@ struct AdmmB200 {
     // graph
     cudaGraphExec_t step_exec = nullptr;
     int kernels_per_step = 0;
+    // The contact passes run in one block (contact_one.cuh) or with a launch each; the graph of the
+    // other choice is kept while it lasts (pick_contact_passes).
+    bool contact_one = false, contact_small = false;
+    int last_contacts = 0;          // of the last status read
+    struct OtherGraph {
+        cudaGraphExec_t exec = nullptr;
+        int kernels_per_step = 0, kernels_body = 0, kernels_fallback = 0;
+    } other;
     int launch_counter = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     float last_ms = 0.f;
@@ -239,6 +248,14 @@ int alloc_bvh(AdmmB200* h, BvhDev& t, int n) {
 
 constexpr int kStatusWords = 8;  // err[4], nc, nc_raw
 
+// The captured substep graphs are out of date.
+void drop_graphs(AdmmB200* h) {
+    if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
+    if (h->other.exec) cudaGraphExecDestroy(h->other.exec);
+    h->step_exec = nullptr;
+    h->other = AdmmB200::OtherGraph{};
+}
+
 // ------------------------------ enqueue helpers -----------------------------
 constexpr int kMaxProfEvents = 1 << 14;
 constexpr int kMaxProbes = 64;
@@ -404,6 +421,12 @@ int enqueue_contact(AdmmB200* h, bool dual) {
     if (G <= 0) return ADMM_OK;
     if (s.cpu_backend) {
         LAUNCH_P(ADMM_KERNEL_CONTACT_DU, k_contact_gs_serial, 1, 32, s, G);
+        return ADMM_OK;
+    }
+    if (h->contact_one) {
+        // loads detection data before its dependency wait, legal because k_contact_p waits before
+        // it triggers: keep k_contact_p directly before it
+        LAUNCH_SMEM(ADMM_KERNEL_CONTACT_DU, k_contact_one, 1, kOneContacts, sizeof(ContactOneSmem), s, G);
         return ADMM_OK;
     }
     // pass 1 projects from s.p into s.du; pass g = 2..G rebuilds p of pass g-1
@@ -1413,6 +1436,26 @@ int build_step_graph(AdmmB200* h) {
     return build_step_graph_once(h);
 }
 
+// How the contact passes of the next substeps run: in one block while the last known detection had
+// few contacts, else with a launch each; the same bits either way, and a substep whose count the
+// guess missed is still right (contact_one_global).  Only for scenes of up to kSmallSurface surface
+// vertices: on larger ones the local step, which runs beside the contact step, takes as long as
+// the launches.  Measured per ADMM iteration: 5 contacts 24.6 us with launches.  Two thresholds,
+// so that a count near them does not switch graphs back and forth; probed and profiled substeps
+// keep what they were captured with.
+constexpr int kSmallSurface = 8192, kOneAgain = 512;
+
+void pick_contact_passes(AdmmB200* h) {
+    if (!h->contact_small || h->probe_kernel != 0) return;
+    const bool one = h->last_contacts <= (h->contact_one ? kOneContacts : kOneAgain);
+    if (one == h->contact_one) return;
+    h->contact_one = one;
+    std::swap(h->step_exec, h->other.exec);
+    std::swap(h->kernels_per_step, h->other.kernels_per_step);
+    std::swap(h->kernels_body, h->other.kernels_body);
+    std::swap(h->kernels_fallback, h->other.kernels_fallback);
+}
+
 bool learned_active(const AdmmB200* h) { return h->global_solver == 3; }
 
 // One substep from its graph (a learned substep judges and replaces its failed
@@ -1809,6 +1852,9 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     TRY(dalloc(h, &s.res_part, 3 * (size_t)(h->tet_blocks + h->tri_blocks + h->bend_blocks + h->pin_blocks +
                                             blocks(s.nd, kLocalThreads))));
 
+    h->contact_small = h->contact_one = s.contact && !s.cpu_backend && s.nsv <= kSmallSurface;
+    if (h->contact_one)
+        CK(cudaFuncSetAttribute(k_contact_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ContactOneSmem)));
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->if_stream, cudaStreamNonBlocking));
@@ -2045,6 +2091,7 @@ int read_status(AdmmB200* h, int* status) {
     int* e = h->status_host;
     CK(cudaMemcpyAsync(e, h->s.err, sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    h->last_contacts = e[5];
     if (e[0] || e[1] || e[2] || e[3]) CK(cudaMemset(h->s.err, 0, sizeof(int) * 4));
     // after a timed-out wait the blocks' sweep counters disagree: start them again from 0
     if (e[3] && h->pp.epoch) CK(cudaMemset(h->pp.epoch, 0, sizeof(unsigned) * h->pp.blocks));
@@ -2076,10 +2123,7 @@ int anim_publish(AdmmB200* h) {
     a.n_verts = first;
     if (a.n_tracks)
         CK(cudaMemcpy(a.tracks, h->tracks.data(), sizeof(TrackDev) * h->tracks.size(), cudaMemcpyHostToDevice));
-    if (h->step_exec) {
-        cudaGraphExecDestroy(h->step_exec);
-        h->step_exec = nullptr;
-    }
+    drop_graphs(h);
     return ADMM_OK;
 }
 
@@ -2270,7 +2314,7 @@ void admm_b200_destroy(AdmmB200* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
+    drop_graphs(h);
     if (h->fail_host) cudaFreeHost(h->fail_host);
     if (h->status_host) cudaFreeHost(h->status_host);
     cudaFree(h->stage);
@@ -2295,6 +2339,7 @@ int admm_b200_step_async(AdmmB200* h, int n_steps) {
     if (!h) return ADMM_ERR_INVALID;
     if (n_steps < 0) return fail(h, ADMM_ERR_INVALID, "n_steps");
     CK(cudaSetDevice(h->device));
+    pick_contact_passes(h);
     if (h->profiling) {
         // eager, one substep at a time so that every event pair can be read back
         CK(cudaEventRecord(h->ev0, h->stream));
@@ -2558,6 +2603,7 @@ int admm_b200_contact_step(AdmmB200* h) {
     if (!h->s.contact || !h->detected) return fail(h, ADMM_ERR_STATE, "contact_step needs a detection first");
     CK(cudaSetDevice(h->device));
     h->cstream = h->stream;
+    pick_contact_passes(h);
     TRY(enqueue_contact(h, false));
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
@@ -2663,6 +2709,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
     TRY(grow_stage(h, (size_t)6 * n));
+    pick_contact_passes(h);
     TRY(build_step_graph(h));
     const size_t bytes = sizeof(float) * 3 * (size_t)n;
     CK(cudaMemcpyAsync(h->stage, x_in, bytes, cudaMemcpyHostToDevice, h->stream));
@@ -2694,10 +2741,7 @@ int admm_b200_set_probe(AdmmB200* h, int kernel_class) {
         return ADMM_ERR_INVALID;
     CK(cudaSetDevice(h->device));
     CK(cudaStreamSynchronize(h->stream));
-    if (h->step_exec) {
-        cudaGraphExecDestroy(h->step_exec);
-        h->step_exec = nullptr;
-    }
+    drop_graphs(h);
     h->probe_kernel = kernel_class;
     h->probe_ms = 0.0;
     h->probe_n = 0;
@@ -2748,10 +2792,7 @@ int admm_b200_set_preconditioner(AdmmB200* h, const float* blocks9, int nd) {
         for (int k = 0; k < 9; k++) bl[9 * (size_t)i + k] = blocks9[9 * (size_t)caller_of(h, i) + k];
     CK(cudaMemcpy(h->pcg_blocks, bl.data(), sizeof(float) * 9 * (size_t)nd, cudaMemcpyHostToDevice));
     // the step graph holds the preconditioner pointer: capture it again
-    if (h->step_exec) {
-        cudaGraphExecDestroy(h->step_exec);
-        h->step_exec = nullptr;
-    }
+    drop_graphs(h);
     return ADMM_OK;
 }
 
@@ -2778,10 +2819,7 @@ int admm_b200_set_learned(AdmmB200* h, int sweeps, const float* omega, const flo
     h->learn_beta.assign(beta, beta + sweeps);
     h->learn_beta[0] = 0.f;  // the first sweep has no previous iterate
     // the coefficients are kernel arguments of the step graph: capture it again
-    if (h->step_exec) {
-        cudaGraphExecDestroy(h->step_exec);
-        h->step_exec = nullptr;
-    }
+    drop_graphs(h);
     return ADMM_OK;
 }
 

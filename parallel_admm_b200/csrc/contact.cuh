@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_clear(DevScene s) {
     contact_clear(s, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// A segment of the incidence lists for every vertex with contacts: vbeg, and per list entry the
+// A segment of the incidence lists for every vertex with contacts: vbeg (with its place in tv), and per list entry the
 // vertex with its bounds (tvr), which the gathers load in one round trip.  The grid's counters
 // are done with: back to zero for the next detection.
 __global__ void __launch_bounds__(kContactThreads) k_contact_alloc(DevScene s) {
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_alloc(DevScene s) {
         if (lane == 31) base = atomicAdd(s.nalloc, inc);
         const int b = __shfl_sync(0xffffffffu, base, 31) + inc - L;
         if (t < ntv) {
-            s.vbeg[i] = b;
+            s.vbeg[i] = make_int2(b, t);
             s.tvr[t] = make_int4(i, b, b + L, 0);
         }
     }
@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_scc(DevScene s) {
         const int v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const int b = s.vbeg[v[k]];
-            s.vtmp[b + s.crank[4 * c + k]] = 4 * c + k;
-            s.cinc[4 * c + k] = make_int4(v[k], b, b + s.vcnt[v[k]], 0);
+            const int2 b = s.vbeg[v[k]];
+            s.vtmp[b.x + s.crank[4 * c + k]] = 4 * c + k;
+            s.cinc[4 * c + k] = make_int4(v[k], b.x, b.x + s.vcnt[v[k]], b.y);
         }
     }
 }

@@ -137,14 +137,14 @@ struct DevScene {
     float4* du2 = nullptr;  // [cap] second buffer of the fused projection passes
     float4* p2 = nullptr;   // [n] second buffer of p in the fused projection passes
     int* vcnt = nullptr;                  // [n] contacts per vertex
-    int* vbeg = nullptr;                  // [n] first entry of the vertex's incidence list (vertices with contacts)
+    int2* vbeg = nullptr;                 // [n] first entry of the vertex's incidence list, its place in tv (vertices with contacts)
     int* crank = nullptr;                 // [4*cap] number of a contact corner among its vertex's contacts
     float2* ginc = nullptr;               // [4*cap] (contact as int bits, Gamma_c,i), sorted per dynamic vertex
     int* vtmp = nullptr;                  // [4*cap] incidence lists (4 * contact + slot) before sorting
     int* tv = nullptr;                    // [n] vertices with contacts
     int* ntv = nullptr;                   // [1] their number
     int* nalloc = nullptr;                // [1] incidence entries handed out
-    int4* cinc = nullptr;                 // [4*cap] per contact corner: (vertex, list begin, list end, 0)
+    int4* cinc = nullptr;                 // [4*cap] per contact corner: (vertex, list begin, list end, place in tv)
     int4* tvr = nullptr;                  // [n] per touched vertex, in tv order: (vertex, list begin, list end, 0)
     // collision geometry
     int nst = 0, nse = 0, nsv = 0;
