@@ -5,15 +5,15 @@
 // counterpart; the network and loss are specified in the header of the CPU
 // restatement that the tests check these kernels against.
 //
-// Layout: every activation is a row-major FP32 matrix with a row per vertex; nothing of a
-// message's width is kept per edge but one bit per channel.  An edge layer
-// W [h_i, h_j, f_ij] + b of the message from j to i is W_r h_i + b (U), W_c h_j (V) and
-// W_f f_ij: U and V are products per vertex (14 edges per vertex on a tet lattice, so a
-// fourteenth of the work of a product per edge), and one pass over the edges adds the three,
-// applies the ReLU and averages.  Its gradient needs per vertex the sums of the message
-// gradients over its row (Gr) and over the reversed edges (Gc); the products with W and with
-// h follow per vertex.  (With an E x 130 input, an E x 64 output and an E x 130 gradient per
-// layer, forward took 1.18 ms on the 20^3 cube's graph, 9261 vertices and 103 k edges.)
+// Layout: every activation is a row-major FP32 matrix with a row per vertex; per edge only a
+// layer's messages pass through one E x 64 buffer, and one bit per channel is kept.  An edge layer
+// W [h_i, h_j, f_ij] + b of the message from j to i gathers its operand straight into shared
+// memory (k_edge_fwd_tc, BF16 weights).  With FP32 weights it is W_r h_i + b (U), W_c h_j (V) and
+// W_f f_ij: U and V are products per vertex (a fourteenth of the work on a tet lattice), and one
+// pass over the edges adds the three, applies the ReLU and averages; the tensor cores keep the
+// product per edge, whose sums the next layer's rounding to TF32 would otherwise meet in another
+// order.  The gradient needs per vertex the sums of the message gradients over its row (Gr) and
+// over the reversed edges (Gc); the products with W and with h follow per vertex.
 // Dense layers are Z = X W^T + b with W row-major [out][in]; with bf16 set, the forward and
 // input-gradient passes use the weights rounded to BF16 and the activations rounded to TF32
 // (FP32 accumulation), the sums Gr and Gc stay FP32; the master weights and Adam moments are
@@ -120,12 +120,10 @@ __device__ __forceinline__ void read_rows(uint32_t td, int row0, F f) {
 // The same layer on the tensor cores (tcgen05, kind::tf32, FP32 accumulation in
 // tensor memory) for 64 outputs: one CTA per 128 rows.  The
 // rows of X (K = 64 or 128: one or two [R][64] matrices side by side; K = 8: [R][Kin] padded with
-// zeros) and the weights (element (n, k) at W[n * ldw + blockIdx.y * 64 + k], rounded to BF16
-// first) are rounded to TF32 and staged in shared memory in the canonical K-major layout;
+// zeros) and the weights (element (n, k) at W[n * ldw + k], rounded to BF16 first) are rounded to TF32 and staged in shared memory in the canonical K-major layout;
 // thread 0 issues K / 8 MMAs of 128 x 64 x 8 into 64 TMEM columns and commits them to an
 // mbarrier; the warps then read the accumulator and apply bias and activation.
-// blockIdx.y > 0: another 64 input columns of the same weights into the next [R][64] output,
-// without bias (the two halves of an edge layer).  Bound by the latency of staging: with K and the
+// Bound by the latency of staging: with K and the
 // loads' trip counts known to the compiler, 64 -> 19 us for 28 k rows and K = 64 (cold caches).
 // The wait for the MMAs is bounded: a wait that gives up sets err[0] and the
 // CTA releases its TMEM and leaves without writing.
@@ -155,7 +153,7 @@ __global__ void __launch_bounds__(kTcThreads) k_dense_fwd_tc(const float* __rest
 #pragma unroll 16
     for (int u = 0; u < kTcN * K / kTcThreads; u++) {
         const int i = threadIdx.x + u * kTcThreads, n = i / K, k = i % K;
-        const float v = k < Kin ? wval(W, n * ldw + blockIdx.y * kH + k, 1) : 0.f;
+        const float v = k < Kin ? wval(W, n * ldw + k, 1) : 0.f;
         *(float*)(Bs + umma::core_offset(n, k >> 2, C) + (k & 3) * 4) = v;  // BF16 is exact in TF32
     }
     umma::fence_operands();
@@ -177,11 +175,10 @@ __global__ void __launch_bounds__(kTcThreads) k_dense_fwd_tc(const float* __rest
     ok = __syncthreads_and(ok) != 0;              // uniform: the TMEM loads below are warp-wide
     umma::fence_after();
     if (ok) {
-        const bool bias = b && blockIdx.y == 0;
         read_rows<kTcN>(td, row0, [&](int row, int c, float4 v) {
             if (row >= R) return;
-            if (bias) v = make_float4(v.x + b[c], v.y + b[c + 1], v.z + b[c + 2], v.w + b[c + 3]);
-            *(float4*)(Z + ((size_t)blockIdx.y * R + row) * kTcN + c) = v;
+            v = make_float4(v.x + b[c], v.y + b[c + 1], v.z + b[c + 2], v.w + b[c + 3]);
+            *(float4*)(Z + (size_t)row * kTcN + c) = v;
             if (!act) return;
             float4 q = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
             if (act == 2) {
@@ -199,6 +196,122 @@ __global__ void __launch_bounds__(kTcThreads) k_dense_fwd_tc(const float* __rest
         umma::fence_after();
         umma::tmem_dealloc(td, kTcN);
     }
+}
+
+// An edge layer's messages Z[E x 64] = [h_row, h_col, f] W^T + b on the tensor cores, the operand
+// gathered as it is staged: 128 edges per tile, K = 130 padded to 136, 17 MMAs of 128 x 64 x 8.  A
+// CTA keeps the weights in shared memory and takes tiles in steps of the grid (two CTAs per SM:
+// one stages while the other's tile is multiplied and written).  Bound by the gathers (512 B per
+// edge, from L2) and the messages' store.  The MMA wait is bounded as in k_dense_fwd_tc.
+constexpr int kEdgeK = (kEdgeIn + 7) / 8 * 8;
+
+__global__ void __launch_bounds__(kTcThreads) k_edge_fwd_tc(const float* __restrict__ h, const float* __restrict__ ef,
+                                                            const int* __restrict__ rows, const int* __restrict__ col,
+                                                            int E, const float* __restrict__ W,
+                                                            const float* __restrict__ b, float* __restrict__ Z,
+                                                            int* __restrict__ err) {
+    extern __shared__ __align__(128) unsigned char tc_smem[];
+    __shared__ uint64_t mbar;
+    __shared__ uint32_t tmem_base;
+    constexpr int C = kEdgeK / 4;
+    unsigned char* As = tc_smem;
+    unsigned char* Bs = tc_smem + (size_t)kTcRows * kEdgeK * 4;
+#pragma unroll 17
+    for (int u = 0; u < kTcN * kEdgeK / kTcThreads; u++) {
+        const int i = threadIdx.x + u * kTcThreads, n = i / kEdgeK, k = i % kEdgeK;
+        const float v = k < kEdgeIn ? wval(W, n * kEdgeIn + k, 1) : 0.f;
+        *(float*)(Bs + umma::core_offset(n, k >> 2, C) + (k & 3) * 4) = v;  // BF16 is exact in TF32
+    }
+    if (threadIdx.x == 0) umma::mbar_init(&mbar, 1);
+    if (threadIdx.x < 32) umma::tmem_alloc(&tmem_base, kTcN);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t td = tmem_base;
+    bool ok = true;
+    uint32_t phase = 0;
+    for (int e0 = blockIdx.x * kTcRows; e0 < E && ok; e0 += gridDim.x * kTcRows) {
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int* at = half ? col : rows;
+#pragma unroll
+            for (int u = 0; u < kTcRows * 16 / kTcThreads; u++) {
+                const int i = threadIdx.x + u * kTcThreads;
+                const int r = (i & 7) | ((i >> 5) & 15) << 3, c = ((i >> 3) & 3) | (i >> 9) << 2;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (e0 + r < E) v = *(const float4*)(h + (size_t)at[e0 + r] * kH + 4 * c);
+                *(float4*)(As + umma::core_offset(r, 16 * half + c, C)) =
+                    make_float4(umma::tf32_round(v.x), umma::tf32_round(v.y), umma::tf32_round(v.z), umma::tf32_round(v.w));
+            }
+        }
+        {
+            const int r = threadIdx.x & 127, c = threadIdx.x >> 7;  // chunk 32: the edge's two features, chunk 33: padding
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c == 0 && e0 + r < E) {
+                const float2 f = ((const float2*)ef)[e0 + r];
+                v = make_float4(umma::tf32_round(f.x), umma::tf32_round(f.y), 0.f, 0.f);
+            }
+            *(float4*)(As + umma::core_offset(r, 32 + c, C)) = v;
+        }
+        umma::fence_operands();
+        umma::fence_before();
+        __syncthreads();
+        umma::fence_after();
+        if (threadIdx.x == 0) {
+            const uint32_t idesc = umma::idesc_tf32(kTcRows, kTcN);
+            const uint32_t a0 = umma::smem_u32(As), b0 = umma::smem_u32(Bs);
+            for (int k = 0; k < kEdgeK / 8; k++)
+                umma::mma_tf32(td, umma::smem_desc(a0 + 256u * k, C), umma::smem_desc(b0 + 256u * k, C), idesc, k > 0);
+            umma::commit(&mbar);
+        }
+        ok = umma::mbar_wait(&mbar, phase, 1 << 22);
+        if (!ok) umma::mbar_wait(&mbar, phase, 1 << 22);  // the MMAs in flight, once more with a bound
+        ok = __syncthreads_and(ok) != 0;                  // uniform
+        phase ^= 1u;
+        umma::fence_after();
+        if (ok)
+            read_rows<kTcN>(td, e0, [&](int row, int c, float4 v) {
+                if (row < E)
+                    *(float4*)(Z + (size_t)row * kTcN + c) = make_float4(v.x + b[c], v.y + b[c + 1], v.z + b[c + 2], v.w + b[c + 3]);
+            });
+        else if (threadIdx.x == 0)
+            atomicExch(err, 1);
+        umma::fence_before();
+        __syncthreads();  // the accumulator has been read, the operands may be overwritten
+        umma::fence_after();
+    }
+    umma::fence_before();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        umma::fence_after();
+        umma::tmem_dealloc(td, kTcN);
+    }
+}
+
+// agg_i = mean over the edges of row i of relu(Z_e), and the bits as in k_edge_agg.
+template <bool BITS>
+__global__ void __launch_bounds__(256) k_node_agg(const float* __restrict__ Z, const int* __restrict__ start, int n,
+                                                  float* __restrict__ agg, uint2* __restrict__ bits) {
+    const int lane = threadIdx.x & 15, i = (blockIdx.x * blockDim.x + threadIdx.x) / 16;
+    if (i >= n) return;
+    const unsigned gm = 0xffffu << (threadIdx.x & 16);
+    const int shift = threadIdx.x & 16, b = start[i], e1 = start[i + 1];
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int e = b; e < e1; e++) {
+        const float4 v = ((const float4*)Z)[(size_t)e * 16 + lane];
+        const float z[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int t = 0; t < 4; t++) a[t] += fmaxf(z[t], 0.f);
+        if (BITS) {
+            unsigned m[4];
+#pragma unroll
+            for (int t = 0; t < 4; t++) m[t] = (__ballot_sync(gm, z[t] > 0.f) >> shift) & 0xffffu;
+            if (lane == 0) bits[e] = make_uint2(m[0] | m[1] << 16, m[2] | m[3] << 16);
+        }
+    }
+    const float d = (float)max(e1 - b, 1);
+    ((float4*)agg)[(size_t)i * 16 + lane] = make_float4(a[0] / d, a[1] / d, a[2] / d, a[3] / d);
 }
 
 // The input gradients on the tensor cores (bf16 set), the same tcgen05 path as
@@ -490,7 +603,7 @@ template <bool BITS>
 __global__ void __launch_bounds__(256) k_edge_agg(const float* __restrict__ UV, const float* __restrict__ We,
                                                   const float* __restrict__ ef, const int* __restrict__ start,
                                                   const int* __restrict__ col, int n, float* __restrict__ agg,
-                                                  uint2* __restrict__ bits, int bf16) {
+                                                  uint2* __restrict__ bits) {
     const int lane = threadIdx.x & 15, i = (blockIdx.x * blockDim.x + threadIdx.x) / 16;
     if (i >= n) return;
     const unsigned gm = 0xffffu << (threadIdx.x & 16);
@@ -500,16 +613,15 @@ __global__ void __launch_bounds__(256) k_edge_agg(const float* __restrict__ UV, 
     float w0[4], w1[4];
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-        w0[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH, bf16);
-        w1[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH + 1, bf16);
+        w0[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH, 0);
+        w1[t] = wval(We, (4 * lane + t) * kEdgeIn + 2 * kH + 1, 0);
     }
     float a[4] = {0.f, 0.f, 0.f, 0.f};
     const int b = start[i], e1 = start[i + 1];
 #pragma unroll 4
     for (int e = b; e < e1; e++) {
         const float4 v = V[(size_t)col[e] * 16];
-        float2 f = ((const float2*)ef)[e];
-        if (bf16) f = make_float2(umma::tf32_round(f.x), umma::tf32_round(f.y));
+        const float2 f = ((const float2*)ef)[e];
         const float z[4] = {fmaf(f.y, w1[0], fmaf(f.x, w0[0], u.x + v.x)), fmaf(f.y, w1[1], fmaf(f.x, w0[1], u.y + v.y)),
                             fmaf(f.y, w1[2], fmaf(f.x, w0[2], u.z + v.z)), fmaf(f.y, w1[3], fmaf(f.x, w0[3], u.w + v.w))};
 #pragma unroll
@@ -759,11 +871,12 @@ inline int nblk(size_t n, int t) { return (int)((n + t - 1) / t); }
 struct AdmmGnn {
     int n = 0, E = 0, P = 0, bf16 = 1, steps = 0;
     std::vector<void*> allocs, gallocs;  // parameters and optimiser state; per-graph buffers
-    int *start = nullptr, *col = nullptr, *rev = nullptr;
+    int *start = nullptr, *col = nullptr, *rows = nullptr, *rev = nullptr;
     float *val = nullptr, *adiag = nullptr, *x = nullptr, *ef = nullptr;
     float *theta = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
     float *z0 = nullptr, *h[4] = {nullptr, nullptr, nullptr, nullptr};
-    float *uv = nullptr, *agg[3] = {nullptr, nullptr, nullptr}, *zn[3] = {nullptr, nullptr, nullptr};
+    float *zm = nullptr, *uv = nullptr;  // messages of a layer (BF16 weights), U then V (FP32)
+    float *agg[3] = {nullptr, nullptr, nullptr}, *zn[3] = {nullptr, nullptr, nullptr};
     uint2* bits[3] = {nullptr, nullptr, nullptr};  // per edge: which channels of its message are positive
     float *o = nullptr, *B = nullptr;
     float *gh = nullptr, *gh2 = nullptr, *gz = nullptr, *gnin = nullptr, *go = nullptr, *gB = nullptr;
@@ -824,24 +937,24 @@ constexpr size_t dx_smem(int NP, int K) {
     return need > least ? need : least;
 }
 
-// A layer of 64 outputs on [R][64] inputs X (and X1 beside it for K = 128): `halves` products with
-// consecutive 64 input columns of the weights (k_dense_fwd_tc), on the tensor cores with BF16
-// weights, else on the FP32 pipes.
-void dense64(AdmmGnn* g, const float* X, const float* X1, int R, int K, int halves, int wo, int ldw, int bo, float* Z,
-             float* Y, const float* res, int act) {
-    const float *W = g->theta + wo, *b = g->theta + bo;
+// U (with the bias) and V of layer l with FP32 weights: the two halves of the edge layer's weights.
+void edge_halves(AdmmGnn* g, const Off& f, int l) {
+    const MatIndex ix = {kEdgeIn, 1, 0, kH};
+    k_gemm<kH><<<dim3(nblk(g->n, 64), 2), 256, gemm_smem(kH), g->st>>>(
+        g->h[l], g->h[l], g->n, g->theta + f.We[l], ix, g->theta + f.be[l], g->uv, nullptr, nullptr, 0, nullptr, nullptr, 0);
+}
+
+// The node layer l: h[l + 1] = h[l] + relu(W [h[l], agg] + b), on the tensor cores with BF16 weights.
+void node_layer(AdmmGnn* g, const Off& f, int l) {
+    const float *W = g->theta + f.Wn[l], *b = g->theta + f.bn[l];
     if (g->bf16) {
-        const dim3 grid(nblk(R, kTcRows), halves);
-        if (K == kH)
-            k_dense_fwd_tc<kH><<<grid, kTcThreads, fwd_smem(kH), g->st>>>(X, X1, R, K, W, ldw, b, Z, Y, res, act, g->derr);
-        else
-            k_dense_fwd_tc<2 * kH><<<grid, kTcThreads, fwd_smem(2 * kH), g->st>>>(X, X1, R, K, W, ldw, b, Z, Y, res, act, g->derr);
+        k_dense_fwd_tc<kNodeIn><<<nblk(g->n, kTcRows), kTcThreads, fwd_smem(kNodeIn), g->st>>>(
+            g->h[l], g->agg[l], g->n, kNodeIn, W, kNodeIn, b, g->zn[l], g->h[l + 1], g->h[l], 2, g->derr);
         return;
     }
-    const MatIndex ix = {ldw, 1, kH, kH};
-    const dim3 grid(nblk(R, 64), halves);
-    if (K == kH) k_gemm<kH><<<grid, 256, gemm_smem(kH), g->st>>>(X, X1, R, W, ix, b, Z, Y, res, act, nullptr, nullptr, 0);
-    else k_gemm<2 * kH><<<grid, 256, gemm_smem(2 * kH), g->st>>>(X, X1, R, W, ix, b, Z, Y, res, act, nullptr, nullptr, 0);
+    const MatIndex ix = {kNodeIn, 1, kH, 0};
+    k_gemm<kNodeIn><<<nblk(g->n, 64), 256, gemm_smem(kNodeIn), g->st>>>(g->h[l], g->agg[l], g->n, W, ix, b, g->zn[l],
+                                                                       g->h[l + 1], g->h[l], 2, nullptr, nullptr, 0);
 }
 
 // dX = dZ W (K = 64 or 128 columns, in [R][64] matrices one after the other): on the tensor cores
@@ -884,10 +997,18 @@ void forward(AdmmGnn* g, bool bits) {
         k_dense_fwd<<<nblk(n, 4), 256, sizeof(float) * (kH * kFin + 4 * kFin), g->st>>>(
             g->x, n, kFin, g->theta + f.W0, g->theta + f.b0, kH, g->z0, g->h[0], nullptr, 1, 0);
     for (int l = 0; l < 3; l++) {
-        dense64(g, g->h[l], g->h[l], n, kH, 2, f.We[l], kEdgeIn, f.be[l], g->uv, nullptr, nullptr, 0);
-        (bits ? k_edge_agg<true> : k_edge_agg<false>)<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(
-            g->uv, g->theta + f.We[l], g->ef, g->start, g->col, n, g->agg[l], g->bits[l], g->bf16);
-        dense64(g, g->h[l], g->agg[l], n, kNodeIn, 1, f.Wn[l], kNodeIn, f.bn[l], g->zn[l], g->h[l + 1], g->h[l], 2);
+        if (g->bf16) {
+            if (g->E > 0)
+                k_edge_fwd_tc<<<std::min(nblk(g->E, kTcRows), 2 * 148), kTcThreads, fwd_smem(kEdgeK), g->st>>>(
+                    g->h[l], g->ef, g->rows, g->col, g->E, g->theta + f.We[l], g->theta + f.be[l], g->zm, g->derr);
+            (bits ? k_node_agg<true> : k_node_agg<false>)<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(
+                g->zm, g->start, n, g->agg[l], g->bits[l]);
+        } else {
+            edge_halves(g, f, l);
+            (bits ? k_edge_agg<true> : k_edge_agg<false>)<<<nblk((size_t)n * 16, 256), 256, 0, g->st>>>(
+                g->uv, g->theta + f.We[l], g->ef, g->start, g->col, n, g->agg[l], g->bits[l]);
+        }
+        node_layer(g, f, l);
     }
     k_head<<<nblk(n, 64), 256, 0, g->st>>>(g->h[3], g->theta + f.Wo, g->theta + f.bo, g->adiag, n, g->o, g->B, g->om,
                                            g->oth, g->bf16);
@@ -929,8 +1050,8 @@ int admm_gnn_create(int bf16, AdmmGnn** out) {
         admm_gnn_destroy(g);
         return ADMM_ERR_CUDA;
     }
-    cudaFuncSetAttribute(k_dense_fwd_tc<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(kH));
     cudaFuncSetAttribute(k_dense_fwd_tc<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(2 * kH));
+    cudaFuncSetAttribute(k_edge_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem(kEdgeK));
     cudaFuncSetAttribute(k_dense_dx_tc<kH, 2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dx_smem(kH, 2 * kH));
     cudaFuncSetAttribute(k_gemm<kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(kH));
     cudaFuncSetAttribute(k_gemm<2 * kH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gemm_smem(2 * kH));
@@ -951,7 +1072,9 @@ int admm_gnn_set_graph(AdmmGnn* g, int n, int n_edges, const int32_t* start, con
     g->gallocs.clear();
     g->n = n;
     g->E = n_edges;
-    std::vector<int> rev(n_edges, 0);
+    std::vector<int> rows(n_edges), rev(n_edges, 0);
+    for (int i = 0; i < n; i++)
+        for (int e = start[i]; e < start[i + 1]; e++) rows[e] = i;
     for (int i = 0; i < n; i++)  // reverse edge: (j -> i) in row j, binary search (columns sorted)
         for (int e = start[i]; e < start[i + 1]; e++) {
             const int j = col[e];
@@ -972,11 +1095,11 @@ int admm_gnn_set_graph(AdmmGnn* g, int n, int n_edges, const int32_t* start, con
     auto ga = [&](auto** p, size_t cnt) -> int { return galloc(g, p, cnt, true); };
     const size_t H = kH, N = n, Ee = n_edges;
     int rc = ADMM_OK;
-    if ((rc = up(&g->start, start, N + 1)) || (rc = up(&g->col, col, Ee)) ||
+    if ((rc = up(&g->start, start, N + 1)) || (rc = up(&g->col, col, Ee)) || (rc = up(&g->rows, rows.data(), Ee)) ||
         (rc = up(&g->rev, rev.data(), Ee)) || (rc = up(&g->val, val, Ee)) || (rc = up(&g->adiag, adiag, N)) ||
         (rc = up(&g->x, node_feat, N * kFin)) || (rc = up(&g->ef, edge_feat, Ee * kFe)) || (rc = ga(&g->z0, N * H)) ||
         (rc = ga(&g->o, N * kOut)) || (rc = ga(&g->B, N * 9)) || (rc = ga(&g->gh, N * H)) || (rc = ga(&g->gh2, N * H)) ||
-        (rc = ga(&g->gz, N * H)) || (rc = ga(&g->gnin, N * kNodeIn)) || (rc = ga(&g->uv, 2 * N * H)) ||
+        (rc = ga(&g->gz, N * H)) || (rc = ga(&g->gnin, N * kNodeIn)) || (rc = g->bf16 ? ga(&g->zm, Ee * H) : ga(&g->uv, 2 * N * H)) ||
         (rc = ga(&g->q, N * H)) || (rc = ga(&g->grc, 2 * N * H)) || (rc = ga(&g->om, N)) || (rc = ga(&g->oth, N)) ||
         (rc = ga(&g->go, N * kOut)) || (rc = ga(&g->gB, N * 9)) ||
         (rc = ga(&g->part, (size_t)std::min(kDwBlocks, nblk(N, 64)) * 2 * (kH * kNodeIn + kH))) ||
