@@ -125,7 +125,7 @@ struct AdmmB200 {
     bool persist = false;           // chosen mode: persistent global step
     bool tiled = false;             // chosen mode: two sweeps per launch over row tiles
     TileSet ts;
-    int tile_smem = 0;
+    int tile_smem = 0, tile_threads = 0;
     // the global step resident in shared memory (resident.cuh), where the scene fits
     ResidentDev res;
     bool resident = false;
@@ -463,10 +463,10 @@ void launch_jacobi2(AdmmB200* h, const float4* src, float4* dst) {
     DevScene& s = h->s;
     const size_t sm = (size_t)h->tile_smem;
     switch (s.A.lanes) {
-        case 1: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<1>, h->ts.ntiles, kTileThreads, sm, s, h->ts, src, dst); break;
-        case 2: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<2>, h->ts.ntiles, kTileThreads, sm, s, h->ts, src, dst); break;
-        case 4: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<4>, h->ts.ntiles, kTileThreads, sm, s, h->ts, src, dst); break;
-        default: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<8>, h->ts.ntiles, kTileThreads, sm, s, h->ts, src, dst); break;
+        case 1: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<1>, h->ts.ntiles, h->tile_threads, sm, s, h->ts, src, dst); break;
+        case 2: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<2>, h->ts.ntiles, h->tile_threads, sm, s, h->ts, src, dst); break;
+        case 4: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<4>, h->ts.ntiles, h->tile_threads, sm, s, h->ts, src, dst); break;
+        default: LAUNCH_SMEM(ADMM_KERNEL_JACOBI, k_jacobi2<8>, h->ts.ntiles, h->tile_threads, sm, s, h->ts, src, dst); break;
     }
 }
 
@@ -942,17 +942,26 @@ int build_tiles_dev(AdmmB200* h, const HostCsr& A) {
         pos[3 * i + 1] = h->x_init[i].y;
         pos[3 * i + 2] = h->x_init[i].z;
     }
-    const HostTiles t = build_tiles(A, s.nd, pos.data(), 3, kTileOwn, s.A.lanes);
+    // one tile per SM while that is no more than kTileOwnMax rows each, whole slices
+    int sms = 148;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    const int S = 32 / s.A.lanes, own = std::min(kTileOwnMax, std::max(kTileOwn, (blocks(s.nd, sms) + S - 1) / S * S));
+    const HostTiles t = build_tiles(A, s.nd, pos.data(), 3, own, s.A.lanes);
     TileSet& d = h->ts;
     d.ntiles = t.ntiles;
     int* a;
-    TRY(dupload(h, &a, t.row0.data(), t.row0.size())); d.row0 = a;
-    TRY(dupload(h, &a, t.nlocal.data(), t.nlocal.size())); d.nlocal = a;
-    TRY(dupload(h, &a, t.nown.data(), t.nown.size())); d.nown = a;
-    TRY(dupload(h, &a, t.s1_0.data(), t.s1_0.size())); d.s1_0 = a;
-    TRY(dupload(h, &a, t.s1_n.data(), t.s1_n.size())); d.s1_n = a;
-    TRY(dupload(h, &a, t.s2_0.data(), t.s2_0.size())); d.s2_0 = a;
-    TRY(dupload(h, &a, t.s2_n.data(), t.s2_n.size())); d.s2_n = a;
+    std::vector<int4> head(2 * (size_t)t.ntiles);
+    int slices = 1;
+    for (int k = 0; k < t.ntiles; k++) {
+        head[2 * k] = make_int4(t.row0[k], t.nlocal[k], t.nown[k], 0);
+        head[2 * k + 1] = make_int4(t.s1_0[k], t.s1_n[k], t.s2_0[k], t.s2_n[k]);
+        slices = std::max(slices, t.s1_n[k]);
+    }
+    int4* dh;
+    TRY(dupload(h, &dh, head.data(), head.size())); d.head = dh;
+    const int most = s.A.lanes == 1 ? tile_threads<1>() : s.A.lanes == 2 ? tile_threads<2>()
+                   : s.A.lanes == 4 ? tile_threads<4>() : tile_threads<8>();
+    h->tile_threads = std::min(most, 32 * slices);
     TRY(dupload(h, &a, t.trow.data(), t.trow.size())); d.trow = a;
     TRY(upload_host_ell(h, t.e1, d.e1));
     TRY(upload_host_ell(h, t.e2, d.e2));
@@ -1924,25 +1933,19 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     h->hostAdiag = as.a_diag;
     h->persist = h->tiled = false;
     if (!h->resident && h->jac_iter >= 2 && (d->global_solver == 0 || d->global_solver == 3)) {
-        if (d->jacobi_mode == 0 || d->jacobi_mode == 2) TRY(build_persist_plan(h, as.A));
-        if (d->jacobi_mode == 0 || d->jacobi_mode == 3) TRY(build_tiles_dev(h, as.A));
+        if (d->jacobi_mode == 2) TRY(build_persist_plan(h, as.A));  // slower than launches wherever it was timed
+        // two sweeps per launch pay while a launch is bound by latency: up to a tile per SM
+        const bool try_tiles = d->jacobi_mode == 0 && s.nd <= 148 * kTileOwnMax;
+        if (try_tiles || d->jacobi_mode == 3) TRY(build_tiles_dev(h, as.A));
         if (d->jacobi_mode == 2 && h->persist_ok) {
             h->persist = true;
         } else if (d->jacobi_mode == 3) {
             h->tiled = true;
         } else if (d->jacobi_mode == 0) {
             TRY(time_global(h, 1, &h->tune_ms_sweeps));
-            TRY(time_global(h, 3, &h->tune_ms_tiled));
-            if (h->persist_ok) TRY(time_global(h, 2, &h->tune_ms_persist));
-            float best = h->tune_ms_sweeps;
-            if (h->tune_ms_tiled < best) {
-                best = h->tune_ms_tiled;
-                h->tiled = true;
-            }
-            if (h->persist_ok && h->tune_ms_persist < best) {
-                h->tiled = false;
-                h->persist = true;
-            }
+            h->tune_ms_tiled = 1e30f;
+            if (try_tiles) TRY(time_global(h, 3, &h->tune_ms_tiled));
+            h->tiled = h->tune_ms_tiled < h->tune_ms_sweeps;
         }
     }
     TRY(upload_state(h, h->x_init, h->v_init));

@@ -458,23 +458,100 @@ __global__ void __launch_bounds__(kVertThreads, 16) k_jacobi(DevScene s, const f
 // the same order and lane layout as k_jacobi, so two launches of k_jacobi and
 // one of k_jacobi2 give identical bits; the halo rows are computed twice (by
 // their own tile and by their neighbours'), the price of half the launches.
+// A warp does one slice of rows in both phases where the tile has no more
+// slices than the block has warps; everything constant of it (row ids, the
+// diagonal, both phases' matrix entries) is loaded before the dependency wait,
+// so after it there is one round trip to L2 (b and the gathers of src) and one
+// through shared memory.  (With all loads after the wait, a chain of five round
+// trips, two sweeps took 7.1 us on the 20^3 cube against 5.0 for two launches.)
 // ---------------------------------------------------------------------------
-constexpr int kTileThreads = 1024;
-constexpr int kTileOwn = 64;
+constexpr int kTileOwn = 64, kTileOwnMax = 256;  // own rows per tile
+
+// The lane's entries of one slice: the first PF steps in registers, as EllRowPf.
+template <int T>
+struct TileRow {
+    static constexpr int PF = T == 1 ? 18 : T == 2 ? 10 : T == 4 ? 6 : 4;
+    int b, e;
+    int cc[PF];
+    float vv[PF];
+
+    ADMM_DEV void load(const SlicedEll& M, int w, int lane) {
+        b = __ldg(&M.ptr[w]);
+        e = __ldg(&M.ptr[w + 1]);
+#pragma unroll
+        for (int j = 0; j < PF; j++) {
+            const int k = b + lane + 32 * j;
+            cc[j] = k < e ? __ldg(&M.col[k]) : 0;
+            vv[j] = k < e ? __ldg(&M.val[k]) : 0.f;
+        }
+    }
+
+    ADMM_DEV float4 sum(const SlicedEll& M, const float4* __restrict__ v, int lane) const {
+        float ax = 0.f, ay = 0.f, az = 0.f;
+#pragma unroll
+        for (int j = 0; j < PF; j++)
+            if (b + lane + 32 * j < e) {
+                const float4 q = v[cc[j]];
+                ax = fmaf(vv[j], q.x, ax);
+                ay = fmaf(vv[j], q.y, ay);
+                az = fmaf(vv[j], q.z, az);
+            }
+#pragma unroll 2
+        for (int k = b + lane + 32 * PF; k < e; k += 32) {
+            const float4 q = v[__ldg(&M.col[k])];
+            const float a = __ldg(&M.val[k]);
+            ax = fmaf(a, q.x, ax);
+            ay = fmaf(a, q.y, ay);
+            az = fmaf(a, q.z, az);
+        }
+#pragma unroll
+        for (int o = 32 / T; o < 32; o <<= 1) {
+            ax += __shfl_xor_sync(0xffffffffu, ax, o);
+            ay += __shfl_xor_sync(0xffffffffu, ay, o);
+            az += __shfl_xor_sync(0xffffffffu, az, o);
+        }
+        return f4(ax, ay, az);
+    }
+};
+
+// Most threads of a block: 32 warps of T lanes per row where a lane's entries are few.
+template <int T>
+constexpr int tile_threads() {
+    return T == 1 ? 512 : T == 2 ? 768 : 1024;
+}
 
 template <int T>
-__global__ void __launch_bounds__(kTileThreads) k_jacobi2(DevScene s, TileSet ts, const float4* __restrict__ src,
-                                                          float4* __restrict__ dst) {
-    ADMM_PDL_PROLOGUE();
+__global__ void __launch_bounds__(tile_threads<T>(), 1) k_jacobi2(DevScene s, TileSet ts, const float4* __restrict__ src,
+                                                                  float4* __restrict__ dst) {
+    ADMM_PDL_TRIGGER();
     extern __shared__ float4 ysh[];
     constexpr int S = 32 / T;
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int r0 = ts.row0[t], n1 = ts.nlocal[t], no = ts.nown[t];
-    const int a1 = ts.s1_0[t], b1 = a1 + ts.s1_n[t];
-    for (int w = a1 + warp; w < b1; w += nw) {
+    const int4 h0 = ts.head[2 * t], h1 = ts.head[2 * t + 1];  // row0, local rows, own rows, -; slices and their counts
+    const int r0 = h0.x, n1 = h0.y, no = h0.z, a1 = h1.x, m1 = h1.y, a2 = h1.z, m2 = h1.w;
+    TileRow<T> p1, p2;
+    const int li0 = warp * S + lane % S;
+    int g0 = -1;
+    float d0 = 1.f;
+    p1.b = p1.e = p2.b = p2.e = 0;
+    if (warp < m1) {
+        if (li0 < n1) {
+            g0 = __ldg(&ts.trow[r0 + li0]);
+            d0 = __ldg(&s.a_diag[g0]);
+        }
+        p1.load(ts.e1, a1 + warp, lane);
+        if (warp < m2) p2.load(ts.e2, a2 + warp, lane);
+    }
+    ADMM_PDL_WAIT();
+    const float4 b0 = g0 >= 0 ? s.b[g0] : f4(0.f, 0.f, 0.f);
+    if (warp < m1) {
+        const float4 acc = p1.sum(ts.e1, src, lane);
+        if (lane < S && g0 >= 0) ysh[li0] = f4((b0.x - acc.x) / d0, (b0.y - acc.y) / d0, (b0.z - acc.z) / d0);
+    }
+    for (int w = warp + nw; w < m1; w += nw) {
         int lr;
-        const float4 acc = ell_row_sum<T>(ts.e1, src, w, lane, lr);
+        const float4 acc = ell_row_sum<T>(ts.e1, src, a1 + w, lane, lr);
         const int li = lr - a1 * S;
         if (lane < S && li < n1) {
             const int g = ts.trow[r0 + li];
@@ -484,10 +561,13 @@ __global__ void __launch_bounds__(kTileThreads) k_jacobi2(DevScene s, TileSet ts
         }
     }
     __syncthreads();
-    const int a2 = ts.s2_0[t], b2 = a2 + ts.s2_n[t];
-    for (int w = a2 + warp; w < b2; w += nw) {
+    if (warp < m2) {
+        const float4 acc = p2.sum(ts.e2, ysh, lane);
+        if (lane < S && li0 < no) dst[g0] = f4((b0.x - acc.x) / d0, (b0.y - acc.y) / d0, (b0.z - acc.z) / d0);
+    }
+    for (int w = warp + nw; w < m2; w += nw) {
         int lr;
-        const float4 acc = ell_row_sum<T>(ts.e2, ysh, w, lane, lr);
+        const float4 acc = ell_row_sum<T>(ts.e2, ysh, a2 + w, lane, lr);
         const int li = lr - a2 * S;
         if (lane < S && li < no) jacobi_row(s, ts.trow[r0 + li], acc, dst);
     }

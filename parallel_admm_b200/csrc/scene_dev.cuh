@@ -45,8 +45,8 @@ struct BvhDev {
 // Row tiles of the two-sweep Jacobi kernel (see build_tiles in setup.hpp).
 struct TileSet {
     int ntiles = 0;
-    const int *row0 = nullptr, *nlocal = nullptr, *nown = nullptr;
-    const int *s1_0 = nullptr, *s1_n = nullptr, *s2_0 = nullptr, *s2_n = nullptr;
+    const int4* head = nullptr;  // [2 ntiles] (first local row, local rows, own rows, 0), (first slice and slices of
+                                 // phase 1, of phase 2)
     const int* trow = nullptr;   // local row -> global row (-1 = padding)
     SlicedEll e1, e2;            // phase 1 (global columns), phase 2 (tile-local columns)
 };

@@ -43,6 +43,27 @@ def test_sweeps_bitwise(name, lanes):
         assert np.array_equal(a.read(B.BUF_X), b.read(B.BUF_X)), sweeps
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("name", ["cloth5", "cloth46", "cube3", "cube11", "bodies"])
+def test_two_sweeps_per_launch_bitwise(name, lanes):
+    """jacobi_mode 3 (a tile of rows per block; tiles of fewer rows than a slice, and with more
+    slices than the block has warps, among them)."""
+    sc = SCENES[name]()
+    hs = [B.Handle(sc, ell_lanes=lanes, jacobi_mode=m) for m in (1, 3)]
+    rng = np.random.default_rng(5)
+    x = sc.verts + rng.normal(scale=1e-3, size=sc.verts.shape).astype(np.float32)
+    for h in hs:
+        h.set_state(x)
+        h.pre_integration()
+        h.local_step()
+        h.global_step()
+    assert hs[1].global_mode()["mode"] == "tiled"
+    for sweeps in (0, 2, 3, 4, 5):
+        for h in hs:
+            h.jacobi(sweeps)
+        assert np.array_equal(hs[0].read(B.BUF_X), hs[1].read(B.BUF_X)), sweeps
+
+
 @pytest.mark.parametrize("name", ["cloth33", "cube11", "bodies"])
 def test_substeps_bitwise(name):
     a, b = _pair(name, 4)
