@@ -105,7 +105,7 @@ struct AdmmB200 {
     int enqueue_rc = ADMM_OK;       // first error while enqueueing or capturing a substep
     float grid_cell_size = 0.f;
     int grid_buckets = 0;
-    int query_lanes = 32;           // lanes per grid DCD query (8, 16, 32)
+    int query_lanes = 16;           // lanes per grid DCD query (8, 16, 32)
     bool pdl = true;                // programmatic dependent launch between the kernels of a substep
     cudaStream_t cstream = nullptr; // stream the enqueue helpers launch on (capture target)
     cudaStream_t side = nullptr;    // second branch of an ADMM iteration (local step)
@@ -341,17 +341,23 @@ void enqueue_build(AdmmB200* h, BvhDev& t, const int* elems, int stride, bool tr
     LAUNCH(k_refit, blocks(n, 256), 256, t);
 }
 
-// Grid queries with h->query_lanes lanes per query (count or write pass).
+// Grid queries: the count pass with h->query_lanes lanes per query, or the write pass.
 void launch_grid_query(AdmmB200* h, bool write, int nq) {
     DevScene& s = h->s;
+    const bool cpu = s.cpu_contact != 0;
+    if (write) {
+        if (cpu) LAUNCH_P(ADMM_KERNEL_DCD_VF, k_grid_write_pairs<true>, blocks(nq, kQueryThreads), kQueryThreads, s);
+        else LAUNCH_P(ADMM_KERNEL_DCD_VF, k_grid_write_pairs<false>, blocks(nq, kQueryThreads), kQueryThreads, s);
+        return;
+    }
     const int g = blocks((int)std::min<int64_t>((int64_t)nq * h->query_lanes, INT32_MAX), kQueryThreads);
-    switch (h->query_lanes * 2 + (write ? 1 : 0)) {
-        case 16: LAUNCH(k_grid_count8, g, kQueryThreads, s); break;
-        case 17: LAUNCH_P(ADMM_KERNEL_DCD_VF, (k_grid_query<true, 8>), g, kQueryThreads, s); break;
-        case 32: LAUNCH((k_grid_query<false, 16>), g, kQueryThreads, s); break;
-        case 33: LAUNCH_P(ADMM_KERNEL_DCD_VF, (k_grid_query<true, 16>), g, kQueryThreads, s); break;
-        case 64: LAUNCH((k_grid_query<false, 32>), g, kQueryThreads, s); break;
-        default: LAUNCH_P(ADMM_KERNEL_DCD_VF, (k_grid_query<true, 32>), g, kQueryThreads, s); break;
+    switch (h->query_lanes * 2 + (cpu ? 1 : 0)) {
+        case 16: LAUNCH((k_grid_count_pairs<8, false>), g, kQueryThreads, s); break;
+        case 17: LAUNCH((k_grid_count_pairs<8, true>), g, kQueryThreads, s); break;
+        case 32: LAUNCH((k_grid_count_pairs<16, false>), g, kQueryThreads, s); break;
+        case 33: LAUNCH((k_grid_count_pairs<16, true>), g, kQueryThreads, s); break;
+        case 64: LAUNCH((k_grid_count_pairs<32, false>), g, kQueryThreads, s); break;
+        default: LAUNCH((k_grid_count_pairs<32, true>), g, kQueryThreads, s); break;
     }
 }
 
@@ -1573,7 +1579,7 @@ int setup_grid(AdmmB200* h, const AdmmB200Desc* d) {
     if (nb > (int64_t(1) << 28)) return fail(h, ADMM_ERR_INVALID, "collision grid too large");
     g.hmask = (int)nb - 1;
     h->grid_buckets = (int)nb;
-    g.cap = (int)std::min<int64_t>(4 * ins + 4096, int64_t(1) << 30);
+    g.cap = (int)std::min<int64_t>(4 * ins + 4096, (int64_t(1) << 29) - 1);
     TRY(dalloc(h, &g.cnt, nb));
     TRY(dalloc(h, &g.bkt, nb));
     TRY(dalloc(h, &g.ent_lo, g.cap));
@@ -1585,17 +1591,16 @@ int setup_grid(AdmmB200* h, const AdmmB200Desc* d) {
     TRY(dalloc(h, &g.mode, std::max(ne, 1)));
     TRY(dalloc(h, &g.qkey, std::max(s.cap, 1)));
     TRY(dalloc(h, &g.qhits, (size_t)std::max(s.nsv + s.nse, 1) * kQueryHitsMax));
-    // lanes per query: 32 while 32 lanes per query fill at most four waves of
-    // the device, else 16 or 8 (a detection of millions of queries is bound by
-    // throughput, not by the latency of one query's loads)
+    // Lanes per query: 16 while that fits the device's threads at once (the latency of one query's
+    // chain of loads counts), else 8 (the instructions of a turn count).  Detection per substep with
+    // 32 / 16 / 8 lanes: 9.6 k queries 0.331 / 0.307 / 0.333 ms, 18 k 0.462 / 0.412 / 0.411,
+    // 43 k 0.667 / 0.543 / 0.507, 147 k 1.95 / 1.43 / 1.25.
     if (d->query_lanes != 0) {
         h->query_lanes = d->query_lanes;
     } else {
         int sms = 148;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-        const int64_t four_waves = 4ll * sms * 2048;
-        const int64_t nq = s.nsv + s.nse;
-        h->query_lanes = nq * 32 <= four_waves ? 32 : nq * 16 <= four_waves ? 16 : 8;
+        h->query_lanes = (int64_t)(s.nsv + s.nse) * 16 <= (int64_t)sms * 2048 ? 16 : 8;
     }
     return ADMM_OK;
 }

@@ -231,16 +231,9 @@ ADMM_DEV void grid_sort_segment(const DevScene& s, int b, int e) {
 }
 
 // ---------------------------------------------------------------------------
-// Queries: G consecutive lanes of a warp serve one query (G = 8, 16 or 32).
-// The entries of all cells of the query's range are numbered consecutively (an
-// inclusive scan of the bucket sizes over the group, G cells at a time) and
-// lane k of the group takes entries k, k + G, ..., so every lane has the same
-// share whatever the cell sizes; an entry's cell key, box and first-cell bits
-// are loaded together.  Candidates that pass the cell-key, once-per-pair and
-// box tests are queued in shared memory and handed to the narrow phase G at a
-// time, so that it runs on full groups.  G = 32 suits a few thousand queries
-// (latency bound: more lanes per query shorten each query's chain of loads);
-// G = 8 suits millions (throughput bound: less scan and queue work per entry).
+// Queries: k_grid_count_pairs (L lanes per query) counts and records each query's partners,
+// k_grid_write_pairs writes the contacts.  grid_walk is the walk of one query by a whole warp, for
+// the few queries whose range or partners outgrow those kernels.
 // ---------------------------------------------------------------------------
 constexpr int kQueryThreads = 128;  // block size of the query kernels
 constexpr int kQueryHitsMax = 32;   // partners the count pass records per query
@@ -271,71 +264,55 @@ ADMM_DEV float4 edge_box_lo(const DevScene& s, int o, float4& up) {
     return lo;
 }
 
-// The lanes of one query: sub = lane within the group, mask = the group's lanes.
-template <int G>
-struct QueryGroup {
-    int sub;
-    unsigned mask;
-    ADMM_DEV QueryGroup() {
-        const int lane = threadIdx.x & 31;
-        sub = lane % G;
-        mask = G == 32 ? ~0u : (((1u << G) - 1u) << (lane - sub));
-    }
-    // bits of the group's lanes with pred set, lane `sub` of the group at bit `sub`
-    ADMM_DEV unsigned ballot(bool pred) const {
-        const unsigned m = __ballot_sync(mask, pred);
-        return G == 32 ? m : (m >> ((threadIdx.x & 31) - sub)) & ((1u << G) - 1u);
-    }
-    ADMM_DEV unsigned below() const { return (1u << sub) - 1u; }
-};
-
-// Candidate partners of one group waiting for the narrow phase (2G slots in
-// shared memory; the fill n is the same in every lane of the group).
+// Candidate partners waiting for the narrow phase (64 slots in shared memory; the fill n is the
+// same in every lane).
 struct GridQueue {
     int* buf;
     int n;
 };
 
-// Queues the partner of every lane with ok set (called by the whole group);
-// once G or more wait, hands the first G to narrow(partner, true).
-template <int G, class F>
-ADMM_DEV void grid_queue_push(const QueryGroup<G>& grp, GridQueue& q, bool ok, int partner, F& narrow) {
-    const unsigned m = grp.ballot(ok);
-    if (ok) q.buf[q.n + __popc(m & grp.below())] = partner;
+// Queues the partner of every lane with ok set (called by the whole warp);
+// once 32 or more wait, hands the first 32 to narrow(partner, true).
+template <class F>
+ADMM_DEV void grid_queue_push(GridQueue& q, bool ok, int partner, F& narrow) {
+    const int lane = threadIdx.x & 31;
+    const unsigned m = __ballot_sync(~0u, ok);
+    if (ok) q.buf[q.n + __popc(m & ((1u << lane) - 1u))] = partner;
     q.n += __popc(m);
-    if (q.n >= G) {
-        __syncwarp(grp.mask);
-        const int p = q.buf[grp.sub];
-        if (grp.sub < q.n - G) q.buf[grp.sub] = q.buf[G + grp.sub];
-        __syncwarp(grp.mask);
-        q.n -= G;
+    if (q.n >= 32) {
+        __syncwarp();
+        const int p = q.buf[lane];
+        if (lane < q.n - 32) q.buf[lane] = q.buf[32 + lane];
+        __syncwarp();
+        q.n -= 32;
         narrow(p, true);
     }
 }
 
-template <int G, class F>
-ADMM_DEV void grid_queue_drain(const QueryGroup<G>& grp, GridQueue& q, F& narrow) {
+template <class F>
+ADMM_DEV void grid_queue_drain(GridQueue& q, F& narrow) {
     if (q.n == 0) return;
-    __syncwarp(grp.mask);
-    const bool valid = grp.sub < q.n;
-    const int p = valid ? q.buf[grp.sub] : 0;
-    __syncwarp(grp.mask);
+    __syncwarp();
+    const int lane = threadIdx.x & 31;
+    const bool valid = lane < q.n;
+    const int p = valid ? q.buf[lane] : 0;
+    __syncwarp();
     q.n = 0;
     narrow(p, valid);
 }
 
-// The group's walk of one query.  Vertex query (vf): position P = lo = up
+// A warp's walk of one query.  Vertex query (vf): position P = lo = up
 // against the triangles.  Edge query: edge e with box [lo, up] against grid
 // edges with a larger index (grid edge e), every big edge (grid edge e) or big
 // edges with a larger index (big edge e).  Grid part: the cells of the query's
 // range, or every grid element of the type when the range is too large.
-template <int G, class F>
-ADMM_DEV void grid_walk(const DevScene& s, const QueryGroup<G>& grp, bool vf, int e, float4 lo, float4 up,
-                        GridQueue& q, F& narrow) {
+template <bool CPU, class F>
+ADMM_DEV void grid_walk(const DevScene& s, bool vf, int e, float4 lo, float4 up, GridQueue& q, F& narrow) {
     const GridDev& g = s.grid;
     const float gap = s.thickness;
-    const int sub = grp.sub;
-    const unsigned gm = grp.mask;
+    constexpr int G = 32;
+    const int sub = threadIdx.x & 31;
+    const unsigned gm = ~0u;
     const int type = vf ? 0 : 1;
     const bool small = vf || g.mode[s.nst + e] != 0;
     if (small) {
@@ -385,9 +362,9 @@ ADMM_DEV void grid_walk(const DevScene& s, const QueryGroup<G>& grp, bool vf, in
                         // same cell (not another of the bucket); larger edge index; once per pair:
                         // this cell is the first of the query's or of the element's range on every axis
                         ok = ek == kj && (vf || partner > e) && ((fj | __float_as_int(eup.w)) & 7) == 7 &&
-                             (s.cpu_contact || box_overlap(lo, up, elo, eup, gap));
+                             (CPU || box_overlap(lo, up, elo, eup, gap));
                     }
-                    grid_queue_push(grp, q, ok, partner, narrow);
+                    grid_queue_push(q, ok, partner, narrow);
                 }
             }
         } else {
@@ -398,9 +375,9 @@ ADMM_DEV void grid_walk(const DevScene& s, const QueryGroup<G>& grp, bool vf, in
                 if (t < n && g.mode[vf ? t : s.nst + t]) {
                     float4 eup;
                     const float4 elo = vf ? tri_box_lo(s, t, eup) : edge_box_lo(s, t, eup);
-                    ok = s.cpu_contact || box_overlap(lo, up, elo, eup, gap);
+                    ok = CPU || box_overlap(lo, up, elo, eup, gap);
                 }
-                grid_queue_push(grp, q, ok, t, narrow);
+                grid_queue_push(q, ok, t, narrow);
             }
         }
     }
@@ -414,16 +391,18 @@ ADMM_DEV void grid_walk(const DevScene& s, const QueryGroup<G>& grp, bool vf, in
             if (vf || (o != e && (small || o > e))) {
                 float4 oup;
                 const float4 olo = vf ? tri_box_lo(s, o, oup) : edge_box_lo(s, o, oup);
-                ok = s.cpu_contact || box_overlap(lo, up, olo, oup, gap);  // the overlap rule is symmetric
+                ok = CPU || box_overlap(lo, up, olo, oup, gap);  // the overlap rule is symmetric
             }
         }
-        grid_queue_push(grp, q, ok, o, narrow);
+        grid_queue_push(q, ok, o, narrow);
     }
-    grid_queue_drain(grp, q, narrow);
+    grid_queue_drain(q, narrow);
 }
 
 // ---------------------------------------------------------------------------
-// Cheap distance filters in front of the exact narrow phase.  Closest points by
+// Cheap distance filters in front of the exact narrow phase of the CPU backend's predicates (its
+// closest points over all regions are long; the GPU backend's predicate rejects by region within
+// fewer operations than the filter takes).  Closest points by
 // the Voronoi-region construction (point-triangle) and the clamped-parameter
 // construction (segment-segment), in ordinary FP32 arithmetic.  A pair is
 // dropped only when this distance exceeds 1.1 x thickness plus 1e-5 of the
@@ -506,37 +485,37 @@ ADMM_DEV bool surely_apart(float d2, float thickness, float4 a, float4 b, float4
     return d2 > lim * lim;  // false for NaN
 }
 
-// Narrow phase of vertex v against triangle f (region 0, 0 <= d < thickness).
 // Narrow phase of vertex v against triangle f: the GPU backend's (region 0,
 // 0 <= d < thickness) or, with cpu_contact, the CPU backend's (no pair of two
 // static elements, any closest point, d <= thickness).
+template <bool CPU>
 ADMM_DEV bool grid_hit_vf(const DevScene& s, int v, float4 P, int f, int4& ids, NpResult& r) {
     const int4 tri = s.st[f];
     if (v == tri.x || v == tri.y || v == tri.z) return false;
-    if (s.cpu_contact && v >= s.nd && tri.x >= s.nd) return false;
+    if (CPU && v >= s.nd && tri.x >= s.nd) return false;
     ids = make_int4(v, tri.x, tri.y, tri.z);
     const float4 a = s.x[tri.x], b = s.x[tri.y], c = s.x[tri.z];
-    if (surely_apart(fast_pt_dist2(P, a, b, c), s.thickness, P, a, b, c)) return false;
-    if (s.cpu_contact) {
+    if (CPU) {
+        if (surely_apart(fast_pt_dist2(P, a, b, c), s.thickness, P, a, b, c)) return false;
         closest_pt_all(P, a, b, c, r);
         return r.dist <= s.thickness;
     }
     return narrow_pt(P, a, b, c, r) && r.dist < s.thickness && r.dist >= 0.f;
 }
 
-// Narrow phase of edges e and o (no shared vertex), lower index first.
 // Narrow phase of edges e and o (no shared vertex), lower index first: the GPU
 // backend's (region 0) or, with cpu_contact, the CPU backend's (no pair of two
 // static edges, d < thickness unless both closest points are end points).
+template <bool CPU>
 ADMM_DEV bool grid_hit_ee(const DevScene& s, int e, int o, int4& ids, NpResult& r) {
     const int2 ed = s.se[e], od = s.se[o];
     if (ed.x == od.x || ed.x == od.y || ed.y == od.x || ed.y == od.y) return false;
     const int2 lo = o > e ? ed : od, hi = o > e ? od : ed;
-    if (s.cpu_contact && lo.x >= s.nd && hi.x >= s.nd) return false;
+    if (CPU && lo.x >= s.nd && hi.x >= s.nd) return false;
     ids = make_int4(lo.x, lo.y, hi.x, hi.y);
     const float4 p0 = s.x[lo.x], p1 = s.x[lo.y], q0 = s.x[hi.x], q1 = s.x[hi.y];
-    if (surely_apart(fast_ee_dist2(p0, p1, q0, q1), s.thickness, p0, p1, q0, q1)) return false;
-    if (s.cpu_contact) {
+    if (CPU) {
+        if (surely_apart(fast_ee_dist2(p0, p1, q0, q1), s.thickness, p0, p1, q0, q1)) return false;
         closest_ee_all(p0, p1, q0, q1, r);
         const bool corner = (r.bary[0] == 0.f || r.bary[0] == 1.f) && (r.bary[1] == 0.f || r.bary[1] == 1.f);
         return r.dist < s.thickness && !corner;
@@ -544,98 +523,276 @@ ADMM_DEV bool grid_hit_ee(const DevScene& s, int e, int o, int4& ids, NpResult& 
     return narrow_ee(p0, p1, q0, q1, r) && r.dist < s.thickness && r.dist >= 0.f;
 }
 
-// Count (WRITE = false) or write (WRITE = true) the pairs of every query, G
-// lanes per query: surface vertices first, then edges.  The count pass stores
-// the query's pair count in qcount and up to kQueryHitsMax partners in qhits.
-// The write pass places each recorded partner at qoff + its rank among the
-// query's partners, so the segment comes out sorted by partner; a query with
-// more partners than were recorded walks the grid again, writes in walk order
-// and sorts its segment.  The write pass also counts the contacts' vertices.
-template <bool WRITE, int G>
-ADMM_DEV void grid_query(DevScene& s) {
-    ADMM_PDL_PROLOGUE();
-    __shared__ int qbuf[kQueryThreads * 2];
-    const QueryGroup<G> grp;
-    const int q = (blockIdx.x * kQueryThreads + threadIdx.x) / G;
-    if (q >= s.nsv + s.nse) return;  // whole groups leave together
-    const bool vf = q < s.nsv;
-    const int e = q - s.nsv;
-    int v = 0;
-    float4 lo, up;
-    if (vf) {
-        v = s.sv[q];
-        lo = up = s.x[v];
-    } else {
-        lo = edge_box_lo(s, e, up);
+// Is (query q, partner) a pair?  Surface vertices first, then edges.
+template <bool CPU>
+ADMM_DEV bool grid_pair(const DevScene& s, int q, int partner, int4& ids, NpResult& r) {
+    if (q < s.nsv) {
+        const int v = s.sv[q];
+        return grid_hit_vf<CPU>(s, v, s.x[v], partner, ids, r);
     }
-    GridQueue gq{qbuf + 2 * (threadIdx.x - grp.sub), 0};
-    int* qh = s.grid.qhits + (size_t)q * kQueryHitsMax;
-    int nhit = 0;  // the same in every lane of the group
-    if (!WRITE) {
+    return grid_hit_ee<CPU>(s, q - s.nsv, partner, ids, r);
+}
+
+// Box of query q.
+ADMM_DEV void grid_query_box(const DevScene& s, int q, float4& lo, float4& up) {
+    if (q < s.nsv) lo = up = s.x[s.sv[q]];
+    else lo = edge_box_lo(s, q - s.nsv, up);
+}
+
+// Count pass: the pair count of every query (qcount) and up to kQueryHitsMax of its partners
+// (qhits, in no order).
+//
+// L lanes serve a query, 32 / L queries a warp, and the warp stays together.  The non-empty cells
+// of every query's range are listed in shared memory (kQueryCells at a time); each lane then takes
+// every L-th entry of its query's cells, one per turn of the loop, and goes on to the next cell by
+// itself, so a turn costs the loads of an entry's box and a few compares: no scan over the cells
+// and no search for an entry's cell.  The cell key is read only for entries that pass the box test.
+// Candidates of all the warp's queries go to one queue, from which the narrow phase takes 32 at a
+// time.  A query whose range has more than kQueryWarpCells cells is walked by the whole warp.
+// Bound by instruction issue and the entries' load latency: a typical edge query looks at 50 to 110
+// entries, of which ten pass the box test.  64 registers (8 blocks per SM): with 88 the detections
+// of a substep of the 147 k queries of 24 bodies took 1.51 ms, with 64 1.25, with 48 1.37; before
+// (a scan over the cells, a search for each entry's cell, a queue per query and the distance filter in
+// front of both predicates) 1.78.  140 k queries of the two 128 x 128 sheets: 1.33 -> 1.09 ms.
+constexpr int kQueryCells = 32;
+constexpr int kQueryWarpCells = 256;
+
+template <int L, bool CPU>
+__global__ void __launch_bounds__(kQueryThreads, 8) k_grid_count_pairs(DevScene s) {
+    ADMM_PDL_PROLOGUE();
+    constexpr int NQ = 32 / L, W = kQueryThreads / 32;
+    constexpr unsigned all = ~0u;
+    __shared__ int4 cell_list[W][NQ][kQueryCells];
+    __shared__ int2 queue_buf[W][64];
+    __shared__ int hit_count[W][NQ];
+    const GridDev& g = s.grid;
+    const int nq = s.nsv + s.nse;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qi = lane / L, sub = lane % L;
+    const int q0 = (blockIdx.x * W + warp) * NQ;
+    if (q0 >= nq) return;
+    int4* cells = cell_list[warp][qi];
+    int2* queue = queue_buf[warp];
+    int* hits = hit_count[warp];
+    const int q = q0 + qi;
+    const bool live = q < nq;
+    const bool vf = q < s.nsv;
+    const int type = vf ? 0 : 1;
+    const int e = vf ? -1 : q - s.nsv;  // edge queries take partners of a larger index
+    const bool small = live && (vf || g.mode[s.nst + e] != 0);
+    const float gap = s.thickness;
+    float4 lo = f4(0.f, 0.f, 0.f), up = lo;
+    int3 a = make_int3(0, 0, 0), b = a;
+    int nc = 0, nb = live ? g.ctr[1 + type] : 0;
+    bool wide = false;
+    if (live) grid_query_box(s, q, lo, up);
+    if (small) {
+        grid_query_range(lo, up, gap, g.inv_c, a, b);
+        wide = !grid_range_small(a, b) || grid_cells(a, b) > kQueryWarpCells;
+        nc = wide ? 0 : grid_cells(a, b);
+    }
+    if (wide) nb = 0;
+    if (lane < NQ) hits[lane] = 0;
+    const int dx = b.x - a.x + 1, dy = b.y - a.y + 1;
+    const int mx = 65535 / dx + 1, my = 65535 / dy + 1;  // n / d = n * m >> 16 for n < 256
+    int c0 = 0;          // cells of the range listed so far
+    int li = 0, ln = 0;  // the lane's place in the list, the list's length
+    int ent = 0, rem = 0, first = 0;  // the lane's next entry, entries from there to the cell's end
+    float4 elo = lo, eup = lo;        // that entry's box, loaded a turn ahead
+    auto fetch = [&]() {
+        while (rem <= 0 && li < ln) {
+            const int2 c = *reinterpret_cast<const int2*>(cells + li++);
+            ent = c.x + sub;
+            rem = (c.y & 0x1fffffff) - sub;
+            first = (int)((unsigned)c.y >> 29);
+        }
+        if (rem > 0) {
+            elo = g.ent_lo[ent];
+            eup = g.ent_up[ent];
+        }
+    };
+    int j = sub;  // place in the big list
+    int n = 0;    // queued candidates (the same in every lane)
+    auto push = [&](bool ok, int from, int what) {
+        const unsigned m = __ballot_sync(all, ok);
+        if (ok) queue[n + __popc(m & ((1u << lane) - 1u))] = make_int2(from, what);
+        n += __popc(m);
+    };
+    bool big = false;
+    for (;;) {
+        bool more;
+        if (!big) {
+            while ((more = __any_sync(all, rem > 0)) && n < 32) {
+                // larger edge index; once per pair: this cell is the first of the query's or of the
+                // element's range on every axis
+                const bool ok = rem > 0 && __float_as_int(elo.w) > e && ((first | __float_as_int(eup.w)) & 7) == 7 &&
+                                (CPU || box_overlap(lo, up, elo, eup, gap));
+                const int from = qi | (li << 8), what = ent;
+                ent += L;
+                rem -= L;
+                fetch();
+                push(ok, from, what);
+            }
+        } else {
+            while ((more = __any_sync(all, j < nb)) && n < 32) {
+                bool ok = false;
+                int partner = 0;
+                if (j < nb) {
+                    partner = vf ? g.big_tri[j] : g.big_edge[j];
+                    if (vf || (partner != e && (small || partner > e))) {
+                        float4 oup;
+                        const float4 olo = vf ? tri_box_lo(s, partner, oup) : edge_box_lo(s, partner, oup);
+                        ok = CPU || box_overlap(lo, up, olo, oup, gap);  // the rule is symmetric
+                    }
+                    j += L;
+                }
+                push(ok, qi, partner);
+            }
+        }
+        if (n >= 32 || (!more && n > 0)) {
+            __syncwarp();
+            bool valid = lane < n;
+            const int2 it = valid ? queue[lane] : make_int2(0, 0);
+            const int2 nx = lane + 32 < n ? queue[lane + 32] : make_int2(0, 0);
+            __syncwarp();
+            if (lane + 32 < n) queue[lane] = nx;
+            n = max(n - 32, 0);
+            const int iq = it.x & 255, pos = it.x >> 8;
+            int partner = it.y;
+            if (pos > 0) {  // an entry: of the cell itself, not of another in its bucket?
+                const int4 c = cell_list[warp][iq][pos - 1];
+                partner = __float_as_int(g.ent_lo[it.y].w);
+                valid = valid && g.ent_key[it.y] == ((unsigned long long)(unsigned)c.z | ((unsigned long long)(unsigned)c.w << 32));
+            }
+            int4 ids;
+            NpResult r;
+            if (valid && grid_pair<CPU>(s, q0 + iq, partner, ids, r)) {
+                const int h = atomicAdd(&hits[iq], 1);
+                if (h < kQueryHitsMax) g.qhits[(size_t)(q0 + iq) * kQueryHitsMax + h] = partner;
+            }
+            __syncwarp();
+        } else if (!more) {
+            if (big) break;
+            if (__any_sync(all, c0 < nc)) {
+                int len = 0;
+                for (int t = 0; t < kQueryCells && __any_sync(all, c0 + t < nc); t += L) {
+                    const int ci = c0 + t + sub;
+                    int4 c = make_int4(0, 0, 0, 0);
+                    if (ci < nc) {
+                        const int row = ci * mx >> 16, layer = row * my >> 16;
+                        const int3 p = make_int3(a.x + ci - row * dx, a.y + row - layer * dy, a.z + layer);
+                        const int2 r = g.bkt[grid_bucket(p.x, p.y, p.z, type, g.hmask)];
+                        const unsigned long long kk = grid_cell_key(p.x, p.y, p.z);
+                        const unsigned f = (p.x == a.x ? 1 : 0) | (p.y == a.y ? 2 : 0) | (p.z == a.z ? 4 : 0);
+                        c = make_int4(r.x, r.y, (int)(unsigned)kk, (int)(unsigned)(kk >> 32));
+                        if (r.y > 0) c.y |= (int)(f << 29);
+                    }
+                    const unsigned mm = (__ballot_sync(all, c.y != 0) >> (lane - sub)) & (L == 32 ? all : (1u << L) - 1u);
+                    if (c.y != 0) cells[len + __popc(mm & ((1u << sub) - 1u))] = c;
+                    len += __popc(mm);
+                }
+                __syncwarp();
+                c0 += kQueryCells;
+                li = 0;
+                ln = len;
+                fetch();
+            } else {
+                big = true;
+            }
+        }
+    }
+    for (unsigned wm = __ballot_sync(all, wide && sub == 0); wm; wm &= wm - 1) {
+        const int wq = q0 + (__ffs(wm) - 1) / L;
+        float4 wlo, wup;
+        grid_query_box(s, wq, wlo, wup);
+        GridQueue gq{reinterpret_cast<int*>(queue), 0};
+        int nhit = 0;
         auto narrow = [&](int partner, bool valid) {
             int4 ids;
             NpResult r;
-            const bool hit = valid && (vf ? grid_hit_vf(s, v, lo, partner, ids, r) : grid_hit_ee(s, e, partner, ids, r));
-            const unsigned m = grp.ballot(hit);
-            const int k = nhit + __popc(m & grp.below());
-            if (hit && k < kQueryHitsMax) qh[k] = partner;
+            const bool hit = valid && grid_pair<CPU>(s, wq, partner, ids, r);
+            const unsigned m = __ballot_sync(all, hit);
+            const int h = nhit + __popc(m & ((1u << lane) - 1u));
+            if (hit && h < kQueryHitsMax) g.qhits[(size_t)wq * kQueryHitsMax + h] = partner;
             nhit += __popc(m);
         };
-        grid_walk(s, grp, vf, e, lo, up, gq, narrow);
-        if (grp.sub == 0) s.qcount[q] = nhit;
-        return;
+        grid_walk<CPU>(s, wq < s.nsv, wq - s.nsv, wlo, wup, gq, narrow);
+        if (lane == 0) hits[wq - q0] = nhit;
     }
-    const int total = s.qcount[q];
-    if (total == 0) return;
-    const int base = query_offset(s, q);
-    if (total <= kQueryHitsMax) {
-        for (int k = grp.sub; k < total; k += G) {
-            const int partner = qh[k];
+    __syncwarp();
+    if (lane < NQ && q0 + lane < nq) s.qcount[q0 + lane] = hits[lane];
+}
+
+// Write pass: places each recorded partner at the query's offset + its rank among the query's
+// partners, so the segment comes out sorted by partner, and counts the contacts' vertices.  A lane
+// holds a query, and the pairs of the warp's 32 queries are dealt out over its lanes.  A query
+// with more partners than were recorded walks the grid again with the whole warp, writes in walk
+// order and sorts its segment.
+template <bool CPU>
+__global__ void __launch_bounds__(kQueryThreads) k_grid_write_pairs(DevScene s) {
+    ADMM_PDL_PROLOGUE();
+    constexpr unsigned all = ~0u;
+    __shared__ int qbuf[kQueryThreads / 32][64];
+    const int nq = s.nsv + s.nse;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q0 = blockIdx.x * kQueryThreads + warp * 32;
+    if (q0 >= nq) return;
+    const int total = q0 + lane < nq ? s.qcount[q0 + lane] : 0;
+    if (!__any_sync(all, total > 0)) return;
+    const int base = total > 0 ? query_offset(s, q0 + lane) : 0;
+    int incl = total <= kQueryHitsMax ? total : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(all, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int sum = __shfl_sync(all, incl, 31);
+    for (int i0 = 0; i0 < sum; i0 += 32) {
+        const int i = i0 + lane;
+        int j = 0;  // the query of pair i: the first lane whose inclusive count exceeds i
+#pragma unroll
+        for (int st = 16; st >= 1; st >>= 1)
+            if (__shfl_sync(all, incl, j + st - 1) <= i) j += st;
+        const int tj = __shfl_sync(all, total, j), bj = __shfl_sync(all, base, j), ij = __shfl_sync(all, incl, j);
+        if (i < sum) {
+            const int q = q0 + j;
+            const int* qh = s.grid.qhits + (size_t)q * kQueryHitsMax;
+            const int partner = qh[i - (ij - tj)];
             int rank = 0;
-            for (int j = 0; j < total; j++) rank += qh[j] < partner ? 1 : 0;
+            for (int k = 0; k < tj; k++) rank += qh[k] < partner ? 1 : 0;
             int4 ids;
             NpResult r;
-            const bool hit = vf ? grid_hit_vf(s, v, lo, partner, ids, r) : grid_hit_ee(s, e, partner, ids, r);
-            const int slot = base + rank;
-            if (hit && slot < s.cap) {
-                write_contact(s, slot, ids, r, !vf);
+            const int slot = bj + rank;
+            if (grid_pair<CPU>(s, q, partner, ids, r) && slot < s.cap) {
+                write_contact(s, slot, ids, r, q >= s.nsv);
                 contact_touch(s, slot, ids);
             }
         }
-        return;
     }
-    auto emit = [&](int partner, bool valid) {
-        int4 ids;
-        NpResult r;
-        const bool hit = valid && (vf ? grid_hit_vf(s, v, lo, partner, ids, r) : grid_hit_ee(s, e, partner, ids, r));
-        const unsigned m = grp.ballot(hit);
-        const int slot = base + nhit + __popc(m & grp.below());
-        if (hit && slot < s.cap) {
-            write_contact(s, slot, ids, r, !vf);
-            s.grid.qkey[slot] = partner;
-        }
-        nhit += __popc(m);
-    };
-    grid_walk(s, grp, vf, e, lo, up, gq, emit);
-    __syncwarp(grp.mask);
-    const int end = min(base + total, s.cap);
-    if (grp.sub == 0 && end - base > 1) grid_sort_segment(s, base, end);
-    __syncwarp(grp.mask);
-    for (int c = base + grp.sub; c < end; c += G) contact_touch(s, c, s.pairs[c]);
-}
-
-template <bool WRITE, int G>
-__global__ void __launch_bounds__(kQueryThreads) k_grid_query(DevScene s) {
-    grid_query<WRITE, G>(s);
-}
-
-// The count pass of a throughput-bound detection (G = 8), capped at 48
-// registers (10 blocks per SM): more resident warps hide its load latency
-// better than the few spilled registers cost (4.2 M queries of the 4 x 512^2
-// sheets: 46.6 against 52.6 ms of DCD per substep).  The other passes keep the
-// compiler's register choice.
-__global__ void __launch_bounds__(kQueryThreads, 10) k_grid_count8(DevScene s) {
-    grid_query<false, 8>(s);
+    for (unsigned wm = __ballot_sync(all, total > kQueryHitsMax); wm; wm &= wm - 1) {
+        const int l = __ffs(wm) - 1, q = q0 + l;
+        const int wbase = __shfl_sync(all, base, l), end = min(wbase + __shfl_sync(all, total, l), s.cap);
+        float4 lo, up;
+        grid_query_box(s, q, lo, up);
+        GridQueue gq{qbuf[warp], 0};
+        int nhit = 0;
+        auto emit = [&](int partner, bool valid) {
+            int4 ids;
+            NpResult r;
+            const bool hit = valid && grid_pair<CPU>(s, q, partner, ids, r);
+            const unsigned m = __ballot_sync(all, hit);
+            const int slot = wbase + nhit + __popc(m & ((1u << lane) - 1u));
+            if (hit && slot < s.cap) {
+                write_contact(s, slot, ids, r, q >= s.nsv);
+                s.grid.qkey[slot] = partner;
+            }
+            nhit += __popc(m);
+        };
+        grid_walk<CPU>(s, q < s.nsv, q - s.nsv, lo, up, gq, emit);
+        __syncwarp();
+        if (lane == 0 && end - wbase > 1) grid_sort_segment(s, wbase, end);
+        __syncwarp();
+        for (int c = wbase + lane; c < end; c += 32) contact_touch(s, c, s.pairs[c]);
+    }
 }
 
 }  // namespace admm

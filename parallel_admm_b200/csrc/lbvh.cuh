@@ -440,10 +440,8 @@ ADMM_DEV void closest_ee_all(float4 P0, float4 P1, float4 Q0, float4 Q1, NpResul
 }
 
 ADMM_DEV bool box_overlap(float4 llo, float4 lup, float4 rlo, float4 rup, float gap) {
-    if ((rlo.x - lup.x) >= gap || (llo.x - rup.x) >= gap) return false;
-    if ((rlo.y - lup.y) >= gap || (llo.y - rup.y) >= gap) return false;
-    if ((rlo.z - lup.z) >= gap || (llo.z - rup.z) >= gap) return false;
-    return true;
+    return !(((rlo.x - lup.x) >= gap) | ((llo.x - rup.x) >= gap) | ((rlo.y - lup.y) >= gap) |
+             ((llo.y - rup.y) >= gap) | ((rlo.z - lup.z) >= gap) | ((llo.z - rup.z) >= gap));
 }
 
 // convert_DCD_info_kernel (contact_solver.cu:118-154) for one accepted pair.
