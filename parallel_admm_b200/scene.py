@@ -59,7 +59,7 @@ class SolverParams:
     w_scale: float = 200.0
     bvh_refit: bool = True
     ell_lanes: int = 0
-    jacobi_mode: int = 0  # 0 autotuned, 1 one kernel per sweep, 2 persistent global step
+    jacobi_mode: int = 0  # 0 chosen by size or timed, 1 one kernel per sweep, 2 persistent, 3 two sweeps per launch
     broad_phase: int = 0  # 0 default (grid), 1 LBVH, 2 uniform grid
     global_solver: int = 0  # 0 Jacobi (reference), 1 PCG with diag(A), 2 PCG with learned blocks
     pcg_iter: int = 0  # 0 = jacobi_iter // 2
