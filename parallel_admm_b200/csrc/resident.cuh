@@ -156,7 +156,9 @@ ADMM_DEV float4 resident_row(const ResidentView& w, const float4* __restrict__ x
 }
 
 // The matrix entries of a thread's row, kept in registers over the sweeps: up to NP pair steps
-// (rows of 20 entries), the rest stays in shared memory.
+// (rows of 20 entries), the rest stays in shared memory.  The steps past the row's end are 0 times
+// the row's own value, like the plan's padding: a CTA holds rows of several bodies, and 0 times
+// another body's value is NaN once that body has diverged.
 constexpr int kResidentRows = 2;  // rows per thread in registers
 
 template <int Q, int TP>
@@ -169,11 +171,13 @@ struct ResidentRow {
     int b, n;
 
     ADMM_DEV void load(const ResidentView& w, int sl) {
+        const int r = sl * (32 / TP) + (threadIdx.x & 31) / TP;
+        const uint32_t self = r < w.own ? (uint32_t)r | (uint32_t)r << 16 : 0u;
         b = n = 0;
 #pragma unroll
         for (int u = 0; u < NP; u++) {
             v[u] = make_float2(0.f, 0.f);
-            c[u] = 0u;
+            c[u] = self;
         }
         if (sl >= w.slices) return;
         b = w.sptr[sl];
@@ -192,7 +196,7 @@ struct ResidentRow {
         for (int q = 0; q < Q; q++) ax[q] = ay[q] = az[q] = 0.f;
 #pragma unroll
         for (int u0 = 0; u0 < NP; u0 += CH) {
-            if (u0 < n) {  // the same in the whole warp; the steps past n add nothing
+            if (u0 < n) {  // the same in the whole warp
                 float4 p[2 * CH];
 #pragma unroll
                 for (int u = 0; u < CH; u++)

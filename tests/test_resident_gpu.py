@@ -108,3 +108,30 @@ def test_pcg(name, solver):
         h.global_step()
     x, y = a.read(B.BUF_X), b.read(B.BUF_X)
     assert np.abs(x - y).max() <= 1e-5 * max(1.0, np.abs(x).max())
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+def test_non_finite_body_stays_alone(lanes):
+    """A CTA of the resident kernels holds rows of several bodies: one that has diverged, wherever
+    its rows lie in the plan, leaves the others' sweeps as they were."""
+    from scipy.sparse import coo_matrix
+    from scipy.sparse.csgraph import connected_components
+    sc = S.batch_bodies(n_bodies=12, seed=3, vmax=3000)
+    e = sc.tet_inds[:, [0, 0, 0]].ravel(), sc.tet_inds[:, 1:].ravel()
+    body = connected_components(coo_matrix((np.ones(len(e[0])), e), (sc.n_dyn, sc.n_dyn)), directed=False)[1]
+    hs = [B.Handle(sc, ell_lanes=lanes, jacobi_mode=m) for m in (1, 0)]
+    assert hs[1].global_mode()["mode"] == "resident"
+    for h in hs:
+        h.pre_integration()
+        h.local_step()
+        h.global_step()
+    x0 = hs[0].read(B.BUF_X)
+    for k, value in zip(range(body.max() + 1), (np.inf, -np.inf, np.nan) * 4):
+        x = x0.copy()
+        x[:sc.n_dyn][body == k] = value
+        out = []
+        for h in hs:
+            h.write(B.BUF_X, x)
+            h.jacobi(3)
+            out.append(h.read(B.BUF_X)[:sc.n_dyn][body != k])
+        assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1]), k
