@@ -704,10 +704,9 @@ void enqueue_learned_replacement(AdmmB200* h) {
 // The decision on a learned solve and the plain solve that replaces a failed one.  In a
 // graph the replacement is the body of an IF node after k_ldecide, which sets its
 // condition (inside the residual-tolerance WHILE body the IF node is nested in it);
-// eagerly, the host reads the decision (one stream synchronisation per solve).
-void enqueue_learned_decide(AdmmB200* h, bool first) {
-    LearnDev L = h->learn;
-    if (h->resident) L.blocks = h->res.groups * h->res.cluster;  // its partials, one per CTA
+// eagerly, the host reads the decision (one stream synchronisation per solve).  L: h->learn with
+// the number of partials that the solve left.
+void enqueue_learned_decide(AdmmB200* h, const LearnDev& L, bool first) {
     const int fi = first ? 1 : 0;
     cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
     cudaGraph_t g = nullptr;
@@ -787,16 +786,18 @@ void enqueue_learned(AdmmB200* h, bool save_prev, bool first) {
     }
 #undef RHSL_CASE
     set_phase(h, ADMM_PHASE_JACOBI);
-    if (h->resident) {
+    // more sweeps than the kernel's coefficients (plain Jacobi sweeps before admm_b200_set_learned:
+    // jacobi_iter of them): a launch per sweep
+    if (h->resident && K <= kLearnMaxSweeps) {
         LearnCoef cf = {};
         for (int k = 0; k < K; k++) {
             cf.omega[k] = h->learn_omega[k];
             cf.beta[k] = h->learn_beta[k];
         }
         LearnDev lr = L;
-        lr.blocks = h->res.groups * h->res.cluster;
+        lr.blocks = h->res.groups * h->res.cluster;  // a partial per CTA
         launch_resident(h, resident_learned_fn(h->res), h->res_smem, s, h->res, lr, (const float4*)buf[s0], cf, K, ex);
-        enqueue_learned_decide(h, first);
+        enqueue_learned_decide(h, lr, first);
         return;
     }
 #define LS_CASE(T)                                                                                         \
@@ -819,7 +820,7 @@ void enqueue_learned(AdmmB200* h, bool save_prev, bool first) {
     }
 #undef LS_CASE
     launch_ljudge(h);
-    enqueue_learned_decide(h, first);
+    enqueue_learned_decide(h, L, first);
 }
 
 // Copies of one global step's inputs for admm_b200_record_global (eager only):

@@ -135,3 +135,15 @@ def test_non_finite_body_stays_alone(lanes):
             h.jacobi(3)
             out.append(h.read(B.BUF_X)[:sc.n_dyn][body != k])
         assert np.isfinite(out[0]).all() and np.array_equal(out[0], out[1]), k
+
+
+@pytest.mark.parametrize("sweeps", [31, 32, 33, 40])
+def test_learned_step_before_its_model(sweeps):
+    """Without a model the learned step runs jacobi_iter plain sweeps, more than a model may have."""
+    a, b = _pair("cloth33", 2, global_solver=3, jacobi_iter=sweeps)
+    for _ in range(2):
+        for h in (a, b):
+            h.step(1, allow=(B.ERR_CONTACT_OVERFLOW,))
+        for p, q in zip(a.get_state(), b.get_state()):
+            assert np.array_equal(p, q)
+    assert a.learned_stats() == b.learned_stats()
