@@ -75,14 +75,16 @@ void* current_context() {
 // row-major n x 3 vectors.  Bound by the chain of dependent loads of a row, not by bytes: four
 // lanes share a row, its first kPre entries per lane are loaded before the dependency wait (the
 // sweeps after a call's first one launch while the sweep before them drains; the first one
-// starts after everything before it, so the matrix and b are complete by then).  28 k rows of 11
+// starts after everything before it, so the matrix and b are complete by then).  src and dst are
+// not __restrict__: the sweep before still writes src when this one starts, so src must not be
+// read through the read-only path, nor before the wait.  28 k rows of 11
 // entries, 20 sweeps: 157 us with a thread per row.
 constexpr int kRowLanes = 4, kPre = 4;
 
 __global__ void __launch_bounds__(128) k_jacobi_csr(int n, const int32_t* __restrict__ start,
                                                     const int32_t* __restrict__ cols, const float* __restrict__ vals,
                                                     const float* __restrict__ diag, const float* __restrict__ b,
-                                                    const float* __restrict__ src, float* __restrict__ dst) {
+                                                    const float* src, float* dst) {
     ADMM_PDL_TRIGGER();
     const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / kRowLanes, sub = t % kRowLanes;
     const bool own = i < n;

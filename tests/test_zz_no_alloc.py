@@ -138,3 +138,36 @@ def test_noalloc_jacobi_matches_handle_path_twice():
     rc = B.lib().admm_b200_jacobi_noalloc(262145, _ptr(t_start), _ptr(t_cols), _ptr(t_vals), _ptr(t_diag),
                                          _ptr(t_b), _ptr(t_x), _ptr(t_out), 1, None)
     assert rc == B.ERR_INVALID
+
+
+@pytest.mark.parametrize("n", [3, 4097, 200_000])
+def test_noalloc_overlapped_sweeps(n):
+    """Sweeps of one call start while the sweep before them runs, calls of one sweep each do not:
+    the same bits, over and over."""
+    import torch
+    torch.cuda.set_device(0)
+    side = 6  # a band of 12 entries that sum to 0.95 of the diagonal: the iterates neither vanish nor grow
+    rows = np.arange(n)[:, None]
+    col = rows + np.concatenate([np.arange(-side, 0), np.arange(1, side + 1)])[None, :]
+    keep = (col >= 0) & (col < n)
+    vals = (np.where((rows + col) % 3 == 0, -1.0, 1.0) * 0.95 / (2 * side)).astype(np.float32)[keep]
+    start = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    rng = np.random.default_rng(n)
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).to("cuda:0")
+           for a in (start, col[keep].astype(np.int32), vals, np.ones(n, np.float32),
+                     rng.normal(size=(n, 3)).astype(np.float32), rng.normal(size=(n, 3)).astype(np.float32))]
+    x = [dev[5], torch.empty_like(dev[5]), torch.empty_like(dev[5])]
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def sweeps(src, dst, k):
+        assert B.lib().admm_b200_jacobi_noalloc(n, *(_ptr(t) for t in dev[:5]), _ptr(src), _ptr(dst), k, st) == B.OK
+
+    k = 40
+    sweeps(x[0], x[1], 1)
+    for i in range(1, k):
+        sweeps(x[1 + (i + 1) % 2], x[1 + i % 2], 1)
+    ref = x[1 + (k - 1) % 2].clone()
+    for _ in range(25):
+        out = torch.full_like(ref, float("nan"))
+        sweeps(x[0], out, k)
+        assert torch.equal(out, ref)
