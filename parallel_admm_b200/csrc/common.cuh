@@ -14,7 +14,9 @@
 // instructions are no-ops for a kernel launched without the PDL attribute.
 // The two halves, for kernels that first load data which no kernel of a substep
 // writes (matrices, constraint records) and only then wait: those loads overlap
-// the tail of the preceding kernels.
+// the tail of the preceding kernels.  What an earlier kernel of the stream writes must not reach
+// such a kernel as a __restrict__ parameter: it still changes while the kernel is resident, and the
+// compiler may move restrict loads before the wait or through the read-only path.
 #define ADMM_PDL_TRIGGER() asm volatile("griddepcontrol.launch_dependents;" ::: "memory")
 #define ADMM_PDL_WAIT() asm volatile("griddepcontrol.wait;" ::: "memory")
 

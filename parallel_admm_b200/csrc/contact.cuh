@@ -262,8 +262,7 @@ __global__ void __launch_bounds__(kContactThreads) k_contact_du(DevScene s) {
 // The pass before it waits before it triggers: the touched list, the list
 // bounds and the first two incidence entries of each lane (detection data) are
 // loaded before the wait.
-__global__ void __launch_bounds__(kContactThreads) k_contact_gather(DevScene s, const float4* __restrict__ p_src,
-                                                                   const float4* __restrict__ du) {
+__global__ void __launch_bounds__(kContactThreads) k_contact_gather(DevScene s, const float4* p_src, const float4* du) {
     ADMM_PDL_TRIGGER();
     const int sub = threadIdx.x % kGatherLanes;
     const unsigned gmask = 0xffu << (threadIdx.x & 31 & ~(kGatherLanes - 1));
@@ -413,10 +412,8 @@ ADMM_DEV void pass_contact(const DevScene& s, int c, const PassRec& P, int lane,
 // The kernel before it (k_contact_du or the previous pass) waits before it
 // triggers, so the detection data of the warp's first contact (PassRec) is
 // loaded before the wait; after it only du_old, p_old and r_c.
-__global__ void __launch_bounds__(kContactThreads) k_contact_pass(DevScene s, const float4* __restrict__ p_old,
-                                                                    float4* __restrict__ p_new,
-                                                                 const float4* __restrict__ du_old,
-                                                                 float4* __restrict__ du_new) {
+__global__ void __launch_bounds__(kContactThreads) k_contact_pass(DevScene s, const float4* p_old, float4* p_new,
+                                                                  const float4* du_old, float4* du_new) {
     const int lane = threadIdx.x & 31, grp = lane >> 3, sub = lane & 7;
     const unsigned gmask = 0xffu << (lane & ~7);
     const int nc = __ldcg(s.nc);

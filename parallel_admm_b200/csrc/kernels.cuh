@@ -432,8 +432,7 @@ ADMM_DEV void jacobi_row(const DevScene& s, int i, float4 acc, float4* __restric
 // waits on its gathers, and the extra resident warps hide more of that latency than the
 // 8 bytes of spill cost (batch: 52.9 -> 49.5 us per sweep in the step graph).
 template <int T>
-__global__ void __launch_bounds__(kVertThreads, 16) k_jacobi(DevScene s, const float4* __restrict__ src,
-                                                             float4* __restrict__ dst) {
+__global__ void __launch_bounds__(kVertThreads, 16) k_jacobi(DevScene s, const float4* src, float4* dst) {
     ADMM_PDL_TRIGGER();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -521,8 +520,8 @@ constexpr int tile_threads() {
 }
 
 template <int T>
-__global__ void __launch_bounds__(tile_threads<T>(), 1) k_jacobi2(DevScene s, TileSet ts, const float4* __restrict__ src,
-                                                                  float4* __restrict__ dst) {
+__global__ void __launch_bounds__(tile_threads<T>(), 1) k_jacobi2(DevScene s, TileSet ts, const float4* src,
+                                                                       float4* dst) {
     ADMM_PDL_TRIGGER();
     extern __shared__ float4 ysh[];
     constexpr int S = 32 / T;
@@ -825,7 +824,7 @@ __global__ void __launch_bounds__(kVertThreads) k_damp_binit(DevScene s) {
     s.mxt[i] = m;
 }
 
-__global__ void k_copy_dyn(DevScene s, const float4* __restrict__ src, float4* __restrict__ dst) {
+__global__ void k_copy_dyn(DevScene s, const float4* src, float4* dst) {
     ADMM_PDL_PROLOGUE();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < s.nd) dst[i] = src[i];

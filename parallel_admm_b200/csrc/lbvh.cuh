@@ -29,7 +29,7 @@ ADMM_DEV void box_add(float4& lo, float4& up, float4 p) {
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) k_elem_boxes(const float4* __restrict__ x, const int* __restrict__ elems,
+__global__ void __launch_bounds__(256) k_elem_boxes(const float4* x, const int* __restrict__ elems,
                                                    int elem_stride, int n, BvhDev t) {
     ADMM_PDL_PROLOGUE();
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -168,7 +168,7 @@ ADMM_DEV void store_in_parent(const BvhDev& t, int c, float4 lo, float4 up) {
 // Refit of an existing tree: recompute the sorted leaves' boxes from the
 // current positions and clear the arrival counters (k_refit follows).
 template <int NV>
-__global__ void __launch_bounds__(256) k_leaf_refresh(const float4* __restrict__ x, const int* __restrict__ elems,
+__global__ void __launch_bounds__(256) k_leaf_refresh(const float4* x, const int* __restrict__ elems,
                                                      int elem_stride, BvhDev t) {
     ADMM_PDL_PROLOGUE();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;

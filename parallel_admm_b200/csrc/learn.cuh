@@ -59,7 +59,7 @@ struct LearnDev {
 // is switched on for the substep.
 template <int T, bool SAVE_PREV>
 __global__ void __launch_bounds__(kVertThreads) k_rhs_learn(DevScene s, LearnDev L, int extrap,
-                                                            float4* __restrict__ x0buf) {
+                                                            float4* x0buf) {
     ADMM_PDL_TRIGGER();
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -95,8 +95,8 @@ __global__ void __launch_bounds__(kVertThreads) k_rhs_learn(DevScene s, LearnDev
 // The sweep and the judge's pass are capped at 40 registers (12 blocks per SM) for the same
 // reason as k_jacobi (batch: 65.4 -> 56.0 us per learned sweep in the step graph).
 template <int T, bool FIRST>
-__global__ void __launch_bounds__(kVertThreads, 12) k_lsweep(DevScene s, LearnDev L, const float4* __restrict__ src,
-                                                         const float4* __restrict__ prev, float4* __restrict__ dst,
+__global__ void __launch_bounds__(kVertThreads, 12) k_lsweep(DevScene s, LearnDev L, const float4* src,
+                                                         const float4* prev, float4* dst,
                                                          float omega, float beta, int extrap) {
     ADMM_PDL_TRIGGER();
     __shared__ double sh[kVertThreads / 32];

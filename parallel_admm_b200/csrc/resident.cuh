@@ -298,7 +298,7 @@ struct LearnCoef {
 
 template <int Q, int TP, bool CLUSTER>
 __global__ void __launch_bounds__(kResidentThreads, 1)
-    k_resident_learned(DevScene s, ResidentDev p, LearnDev L, const float4* __restrict__ x0, LearnCoef coef, int sweeps,
+    k_resident_learned(DevScene s, ResidentDev p, LearnDev L, const float4* x0, LearnCoef coef, int sweeps,
                        int extrap) {
     extern __shared__ __align__(128) unsigned char rsm[];
     __shared__ double sh[32];

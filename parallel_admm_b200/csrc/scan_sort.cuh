@@ -40,8 +40,7 @@ ADMM_DEV int block_exclusive_scan(int v, int* sh_warp) {
 }
 
 // Phase 1: per-tile exclusive scan in place (out) and tile totals.
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* __restrict__ in, int* __restrict__ out,
-                                                            int n, int* __restrict__ tile_sums) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* in, int* out, int n, int* tile_sums) {
     ADMM_PDL_PROLOGUE();
     __shared__ int sh[32];
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
@@ -64,8 +63,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(const int* __restri
 
 // Phase 2: one block scans the tile totals (any count, in chunks with carry);
 // total written to *total (may be NULL) and tile_sums becomes exclusive.
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int* __restrict__ tile_sums, int ntiles,
-                                                           int* __restrict__ total) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(int* tile_sums, int ntiles, int* total) {
     ADMM_PDL_PROLOGUE();
     __shared__ int sh[32];
     __shared__ int carry;
@@ -117,8 +115,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_total(DevScene s, int nt
 ADMM_DEV int query_offset(const DevScene& s, int q) { return s.qoff[q] + s.scan_tmp[q / kScanTile]; }
 
 // Phase 3: add tile offsets.
-__global__ void __launch_bounds__(kScanThreads) k_scan_add(int* __restrict__ out, int n,
-                                                          const int* __restrict__ tile_sums) {
+__global__ void __launch_bounds__(kScanThreads) k_scan_add(int* out, int n, const int* tile_sums) {
     ADMM_PDL_PROLOGUE();
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
     const int add = tile_sums[blockIdx.x];
@@ -148,8 +145,8 @@ constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortTile = 2048;
 
-__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const unsigned long long* __restrict__ keys, int n,
-                                                            int shift, int* __restrict__ hist, int ntiles) {
+__global__ void __launch_bounds__(kSortThreads) k_radix_hist(const unsigned long long* keys, int n, int shift, int* hist,
+                                                            int ntiles) {
     ADMM_PDL_PROLOGUE();
     __shared__ int h[256];
     h[threadIdx.x] = 0;
@@ -163,11 +160,9 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist(const unsigned long
     hist[threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const unsigned long long* __restrict__ kin,
-                                                               const int* __restrict__ vin,
-                                                               unsigned long long* __restrict__ kout,
-                                                               int* __restrict__ vout, int n, int shift,
-                                                               const int* __restrict__ offs, int ntiles) {
+__global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const unsigned long long* kin, const int* vin,
+                                                               unsigned long long* kout, int* vout, int n, int shift,
+                                                               const int* offs, int ntiles) {
     ADMM_PDL_PROLOGUE();
     __shared__ int run[256];
     __shared__ int wcnt[kSortWarps][256];
