@@ -58,7 +58,15 @@ struct AdmmB200 {
     // The contact passes run in one block (contact_one.cuh) or with a launch each; the graph of the
     // other choice is kept while it lasts (pick_contact_passes).
     bool contact_one = false, contact_small = false;
-    int last_contacts = 0;          // of the last status read
+    int calm = 0;                   // looks at the contact counts since the last one with many
+    bool calm_now = true;           // the last one had few
+    // Contact counts of substeps that no status read follows, on their way to the host: sent after
+    // every kPeaks-th substep.
+    static constexpr int kCountRing = 16;
+    cudaEvent_t count_ev[kCountRing] = {};
+    int* count_host = nullptr;      // pinned [kCountRing * kPeaks]
+    int64_t count_sent = 0, count_seen = 0;
+    int unsent = 0;                 // substeps since the last one sent or read
     struct OtherGraph {
         cudaGraphExec_t exec = nullptr;
         int kernels_per_step = 0, kernels_body = 0, kernels_fallback = 0;
@@ -83,7 +91,7 @@ struct AdmmB200 {
     int learn_sweeps = 0;
     std::vector<float> learn_omega, learn_beta;
     int* fail_host = nullptr;       // pinned: learn.fail (eager substeps)
-    int* status_host = nullptr;     // pinned copy of the status words (err, nc, nc_raw)
+    int* status_host = nullptr;     // pinned copy of the status words (kStatusWords)
     int64_t learn_substeps = 0;
     int kernels_fallback = 0;       // kernels of the plain solve that replaces a failed learned one
     cudaStream_t if_stream = nullptr;  // capture of the bodies of the fallback IF nodes
@@ -246,7 +254,8 @@ int alloc_bvh(AdmmB200* h, BvhDev& t, int n) {
     return ADMM_OK;
 }
 
-constexpr int kStatusWords = 8;  // err[4], nc, nc_raw
+constexpr int kPeaks = 4;                       // substeps of nc_peaks
+constexpr int kStatusWords = kPeakWord + kPeaks;  // err[4], nc, nc_raw, -, -, nc_peaks
 
 // The captured substep graphs are out of date.
 void drop_graphs(AdmmB200* h) {
@@ -1452,18 +1461,61 @@ int build_step_graph(AdmmB200* h) {
     return build_step_graph_once(h);
 }
 
-// How the contact passes of the next substeps run: in one block while the last known detection had
-// few contacts, else with a launch each; the same bits either way, and a substep whose count the
-// guess missed is still right (contact_one_global).  Only for scenes of up to kSmallSurface surface
-// vertices: on larger ones the local step, which runs beside the contact step, takes as long as
-// the launches.  Measured per ADMM iteration: 5 contacts 24.6 us with launches.  Two thresholds,
-// so that a count near them does not switch graphs back and forth; probed and profiled substeps
+// How the contact passes of the next substep run: in one block after kCalm looks at the last kPeaks
+// substeps found few contacts in every detection (a cloth on the ground may go from none to thousands
+// and back from one detection of a substep to the next), else with a launch each; the same bits
+// either way, and a substep that the guess missed is still right, but slower (contact_one_global;
+// the first substep in which a cloth of 64^2 / 88^2 vertices lands on the ground: 1.9 / 3.7 ms, the
+// next ones with launches 1.4 / 1.9 ms).  So a launch each, too, where the counts of the last
+// kCountRing * kPeaks substeps have not arrived (a long step_async).  Only for scenes of up to
+// kSmallSurface surface vertices: on larger ones the local step, which runs beside the contact step,
+// takes as long as the launches.  Measured per ADMM iteration: 5 contacts 24.6 us with launches.
+// Two thresholds, so that a count near them does not switch graphs back and forth; probed substeps
 // keep what they were captured with.
-constexpr int kSmallSurface = 8192, kOneAgain = 512;
+constexpr int kSmallSurface = 8192, kOneAgain = 512, kCalm = 4;
+
+// peaks: the largest counts of the last kPeaks substeps.
+void note_counts(AdmmB200* h, const int* peaks) {
+    const int contacts = *std::max_element(peaks, peaks + kPeaks);
+    h->calm_now = contacts <= kOneContacts;
+    h->calm = contacts <= kOneAgain ? h->calm + 1 : 0;
+}
+
+// The counts that have arrived; waits until at most `behind` of those sent have not (< 0: no wait).
+int take_counts(AdmmB200* h, int behind) {
+    for (; h->count_seen < h->count_sent; h->count_seen++) {
+        const int slot = (int)(h->count_seen % AdmmB200::kCountRing);
+        if (behind >= 0 && h->count_sent - h->count_seen > behind) {
+            CK(cudaEventSynchronize(h->count_ev[slot]));
+        } else {
+            const cudaError_t e = cudaEventQuery(h->count_ev[slot]);
+            if (e == cudaErrorNotReady) {
+                cudaGetLastError();
+                break;
+            }
+            CK(e);
+        }
+        note_counts(h, h->count_host + slot * kPeaks);
+    }
+    return ADMM_OK;
+}
+
+// Sends the contact counts of the substeps launched, when it is their turn.
+int send_counts(AdmmB200* h) {
+    if (!h->contact_small || ++h->unsent < kPeaks) return ADMM_OK;
+    h->unsent = 0;
+    if (h->count_sent - h->count_seen == AdmmB200::kCountRing) h->count_seen++;  // its slot is written again
+    const int slot = (int)(h->count_sent % AdmmB200::kCountRing);
+    CK(cudaMemcpyAsync(h->count_host + slot * kPeaks, nc_peaks(h->s), sizeof(int) * kPeaks, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaEventRecord(h->count_ev[slot], h->stream));
+    h->count_sent++;
+    return ADMM_OK;
+}
 
 void pick_contact_passes(AdmmB200* h) {
     if (!h->contact_small || h->probe_kernel != 0) return;
-    const bool one = h->last_contacts <= (h->contact_one ? kOneContacts : kOneAgain);
+    const bool known = h->count_sent - h->count_seen < AdmmB200::kCountRing;
+    const bool one = known && (h->contact_one ? h->calm_now : h->calm >= kCalm);
     if (one == h->contact_one) return;
     h->contact_one = one;
     std::swap(h->step_exec, h->other.exec);
@@ -1868,8 +1920,11 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
                                             blocks(s.nd, kLocalThreads))));
 
     h->contact_small = h->contact_one = s.contact && !s.cpu_backend && s.nsv <= kSmallSurface;
-    if (h->contact_one)
+    if (h->contact_small) {
         CK(cudaFuncSetAttribute(k_contact_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ContactOneSmem)));
+        for (auto& e : h->count_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaHostAlloc((void**)&h->count_host, sizeof(int) * AdmmB200::kCountRing * kPeaks, cudaHostAllocDefault));
+    }
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->if_stream, cudaStreamNonBlocking));
@@ -2094,13 +2149,50 @@ int accumulate_timers(AdmmB200* h) {
     return ADMM_OK;
 }
 
+// n_steps substeps.  wait: the caller waits for them, so this may wait on the way for all but the
+// last 2 kPeaks, for their contact counts.
+int run_substeps(AdmmB200* h, int n_steps, bool wait) {
+    if (n_steps < 0) return fail(h, ADMM_ERR_INVALID, "n_steps");
+    CK(cudaSetDevice(h->device));
+    TRY(take_counts(h, -1));
+    pick_contact_passes(h);
+    if (h->profiling) {
+        // eager, one substep at a time so that every event pair can be read back
+        CK(cudaEventRecord(h->ev0, h->stream));
+        for (int k = 0; k < n_steps; k++) {
+            h->prof_used = 0;
+            TRY(run_substep_eager(h));
+            CK(cudaStreamSynchronize(h->stream));
+            TRY(accumulate_timers(h));
+        }
+        CK(cudaEventRecord(h->ev1, h->stream));
+        h->frame += n_steps;
+        return ADMM_OK;
+    }
+    TRY(build_step_graph(h));
+    CK(cudaEventRecord(h->ev0, h->stream));
+    for (int k = 0; k < n_steps; k++) {
+        if (k > 0) {
+            TRY(take_counts(h, wait ? 1 : -1));
+            pick_contact_passes(h);
+            TRY(build_step_graph(h));
+        }
+        TRY(launch_substep(h));
+        if (!wait || k + 1 < n_steps) TRY(send_counts(h));  // else a status read follows
+    }
+    CK(cudaEventRecord(h->ev1, h->stream));
+    h->frame += n_steps;
+    return ADMM_OK;
+}
+
 // Waits for the stream; the status of what ran on it (cleared on the device) and, in
-// h->status_host, the contact counts (4: stored, 5: found).
+// h->status_host, the contact counts (4: stored, 5: found, from kPeakWord: most found in each of the last kPeaks substeps).
 int read_status(AdmmB200* h, int* status) {
     int* e = h->status_host;
     CK(cudaMemcpyAsync(e, h->s.err, sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    h->last_contacts = e[5];
+    TRY(take_counts(h, 0));
+    h->unsent = 0;
     if (e[0] || e[1] || e[2] || e[3]) CK(cudaMemset(h->s.err, 0, sizeof(int) * 4));
     // after a timed-out wait the blocks' sweep counters disagree: start them again from 0
     if (e[3] && h->pp.epoch) CK(cudaMemset(h->pp.epoch, 0, sizeof(unsigned) * h->pp.blocks));
@@ -2326,6 +2418,9 @@ void admm_b200_destroy(AdmmB200* h) {
     drop_graphs(h);
     if (h->fail_host) cudaFreeHost(h->fail_host);
     if (h->status_host) cudaFreeHost(h->status_host);
+    if (h->count_host) cudaFreeHost(h->count_host);
+    for (auto e : h->count_ev)
+        if (e) cudaEventDestroy(e);
     cudaFree(h->stage);
     for (void* p : h->allocs)
         if (p) cudaFree(p);
@@ -2346,28 +2441,7 @@ void admm_b200_destroy(AdmmB200* h) {
 
 int admm_b200_step_async(AdmmB200* h, int n_steps) {
     if (!h) return ADMM_ERR_INVALID;
-    if (n_steps < 0) return fail(h, ADMM_ERR_INVALID, "n_steps");
-    CK(cudaSetDevice(h->device));
-    pick_contact_passes(h);
-    if (h->profiling) {
-        // eager, one substep at a time so that every event pair can be read back
-        CK(cudaEventRecord(h->ev0, h->stream));
-        for (int k = 0; k < n_steps; k++) {
-            h->prof_used = 0;
-            TRY(run_substep_eager(h));
-            CK(cudaStreamSynchronize(h->stream));
-            TRY(accumulate_timers(h));
-        }
-        CK(cudaEventRecord(h->ev1, h->stream));
-        h->frame += n_steps;
-        return ADMM_OK;
-    }
-    TRY(build_step_graph(h));
-    CK(cudaEventRecord(h->ev0, h->stream));
-    for (int k = 0; k < n_steps; k++) TRY(launch_substep(h));
-    CK(cudaEventRecord(h->ev1, h->stream));
-    h->frame += n_steps;
-    return ADMM_OK;
+    return run_substeps(h, n_steps, false);
 }
 
 int admm_b200_sync(AdmmB200* h) {
@@ -2379,9 +2453,10 @@ int admm_b200_sync(AdmmB200* h) {
 int admm_b200_step(AdmmB200* h, int n_steps, AdmmStepStats* stats) {
     if (!h) return ADMM_ERR_INVALID;
     const auto t0 = std::chrono::steady_clock::now();
-    TRY(admm_b200_step_async(h, n_steps));
+    TRY(run_substeps(h, n_steps, true));
     int status = ADMM_OK;
     TRY(read_status(h, &status));
+    if (n_steps > 0) note_counts(h, h->status_host + kPeakWord);
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
     h->last_ms = n_steps > 0 ? ms / n_steps : 0.f;
@@ -2612,8 +2687,11 @@ int admm_b200_contact_step(AdmmB200* h) {
     if (!h->s.contact || !h->detected) return fail(h, ADMM_ERR_STATE, "contact_step needs a detection first");
     CK(cudaSetDevice(h->device));
     h->cstream = h->stream;
-    pick_contact_passes(h);
-    TRY(enqueue_contact(h, false));
+    const bool graph_one = h->contact_one;
+    h->contact_one = h->contact_small && h->status_host[5] <= kOneContacts;
+    const int rc = enqueue_contact(h, false);
+    h->contact_one = graph_one;
+    TRY(rc);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
     return ADMM_OK;
@@ -2718,6 +2796,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
     TRY(grow_stage(h, (size_t)6 * n));
+    TRY(take_counts(h, -1));
     pick_contact_passes(h);
     TRY(build_step_graph(h));
     const size_t bytes = sizeof(float) * 3 * (size_t)n;
@@ -2731,6 +2810,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     h->frame += 1;
     int status = ADMM_OK;
     TRY(read_status(h, &status));
+    note_counts(h, h->status_host + kPeakWord);
     return status;
 }
 

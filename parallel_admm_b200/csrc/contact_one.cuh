@@ -39,11 +39,28 @@ ADMM_DEV float4 contact_lane_sum(int b, int e, int sub, unsigned gmask, Entry en
     return f4(ax, ay, az);
 }
 
+// The same for a list of 1 to kOneShort entries by one thread: the partial sums of lanes 0..3,
+// combined as by the xor shuffles.
+template <class Entry, class Du>
+ADMM_DEV float4 contact_short_sum(int b, int len, Entry entry, Du du) {
+    float4 a[kOneShort];
+#pragma unroll
+    for (int l = 0; l < kOneShort; l++) {
+        const float2 gi = entry(l < len ? b + l : b);
+        const float4 d = du(__float_as_int(gi.x));
+        a[l] = l < len ? f4(fmaf(d.x, gi.y, 0.f), fmaf(d.y, gi.y, 0.f), fmaf(d.z, gi.y, 0.f)) : f4(0.f, 0.f, 0.f);
+    }
+    return add3(add3(a[0], a[2]), add3(a[1], a[3]));
+}
+
 // More contacts than fit (the host then switches to a launch per pass, see pick_contact_passes):
-// the same passes in global memory.
+// the same passes in global memory, a thread per vertex with a short list, the long lists of a
+// warp's vertices four at a time.
 ADMM_DEV void contact_one_global(const DevScene& s, int nc, int passes) {
-    const int sub = threadIdx.x % kGatherLanes, ntv = *s.ntv;
-    const unsigned gmask = 0xffu << (threadIdx.x & 31 & ~(kGatherLanes - 1));
+    const int lane = threadIdx.x & 31, sub = lane % kGatherLanes, grp = lane / kGatherLanes, ntv = *s.ntv;
+    const unsigned gmask = 0xffu << (lane & ~(kGatherLanes - 1));
+    auto entry = [&](int k) { return s.ginc[k]; };
+    auto du = [&](int c) { return s.du[c]; };
     for (int pass = 1; pass <= passes; pass++) {
         for (int c = threadIdx.x; c < nc; c += blockDim.x) {
             const ContactRec R = contact_rec(s, c);
@@ -55,12 +72,21 @@ ADMM_DEV void contact_one_global(const DevScene& s, int nc, int passes) {
             s.rc[c] = f4(r.x + d.x, r.y + d.y, r.z + d.z);
         }
         __syncthreads();
-        for (int t = threadIdx.x / kGatherLanes; t < ntv; t += blockDim.x / kGatherLanes) {
-            const int4 v = s.tvr[t];
-            if (v.x >= s.nd) continue;  // the same in the whole group
-            const float4 a = contact_lane_sum(v.y, v.z, sub, gmask, [&](int k) { return s.ginc[k]; },
-                                              [&](int k) { return s.du[k]; });
-            if (sub == 0) s.p[v.x] = add3(s.p[v.x], a);
+        for (int t0 = threadIdx.x - lane; t0 < ntv; t0 += blockDim.x) {
+            const int4 v = t0 + lane < ntv ? s.tvr[t0 + lane] : make_int4(0, 0, 0, 0);
+            const int len = v.x < s.nd ? v.z - v.y : 0;
+            if (len > 0 && len <= kOneShort) s.p[v.x] = add3(s.p[v.x], contact_short_sum(v.y, len, entry, du));
+            for (unsigned m = __ballot_sync(~0u, len > kOneShort); m;) {
+                unsigned r = m;
+                for (int k = 0; k < grp; k++) r &= r - 1;  // this group's vertex: bit number grp
+                const int from = r ? __ffs(r) - 1 : 0;
+                const int x = __shfl_sync(~0u, v.x, from), b = __shfl_sync(~0u, v.y, from), n = __shfl_sync(~0u, len, from);
+                if (r) {
+                    const float4 a = contact_lane_sum(b, b + n, sub, gmask, entry, du);
+                    if (sub == 0) s.p[x] = add3(s.p[x], a);
+                }
+                for (int k = 0; k < 32 / kGatherLanes; k++) m &= m - 1;
+            }
         }
         __syncthreads();
     }
@@ -128,14 +154,7 @@ __global__ void __launch_bounds__(kOneContacts, 1) k_contact_one(DevScene s, int
         };
         for (int k = tid; k < nshort; k += kOneContacts) {
             const int t = m.shorts[k], b = m.list[t] & 0xffffu, len = m.list[t] >> 16;
-            float4 a[kOneShort];  // the partial sums of lanes 0..3, combined as by xor shuffles
-#pragma unroll
-            for (int l = 0; l < kOneShort; l++) {
-                const float2 gi = m.ent[l < len ? b + l : b];
-                const float4 d = m.du[__float_as_int(gi.x)];
-                a[l] = l < len ? f4(fmaf(d.x, gi.y, 0.f), fmaf(d.y, gi.y, 0.f), fmaf(d.z, gi.y, 0.f)) : f4(0.f, 0.f, 0.f);
-            }
-            finish(t, add3(add3(a[0], a[2]), add3(a[1], a[3])));
+            finish(t, contact_short_sum(b, len, [&](int e) { return m.ent[e]; }, [&](int c) { return m.du[c]; }));
         }
         for (int k = tid / kGatherLanes; k < nlong; k += kOneContacts / kGatherLanes) {
             const int t = m.longs[k], b = m.list[t] & 0xffffu;

@@ -162,4 +162,9 @@ struct DevScene {
     int* done = nullptr;
 };
 
+// Largest unclamped contact count of the detections of each of the last four substeps, the latest
+// first: behind err among the status words.
+constexpr int kPeakWord = 8;
+__host__ __device__ inline int4* nc_peaks(const DevScene& s) { return reinterpret_cast<int4*>(s.err + kPeakWord); }
+
 }  // namespace admm

@@ -70,3 +70,39 @@ def test_contact_passes_follow_the_count():
         n, x = run(h, (many, few)[k])
         assert n == fresh[k][0] and np.array_equal(x, fresh[k][1])
     h.close()
+
+
+def test_contact_passes_follow_the_count_within_a_call():
+    """Twelve sheets that fall onto each other: contacts grow out of the one block in a call of many
+    substeps.  The launches take over in the call itself, and whichever way the substeps are queued
+    and run, the bits are those of one call per substep."""
+    n = 20
+    sc, x, m = _stack(12, 6)
+    v = np.zeros_like(x)
+    for k in range(12):
+        x[k * m // 12:(k + 1) * m // 12, 1] += 8e-3 * k
+        v[k * m // 12:(k + 1) * m // 12, 1] = -0.1 * k
+
+    def run(step):
+        h = B.Handle(sc)
+        h.set_state(x, v)
+        assert h.step(1)["n_contacts"] == 0
+        few = h.kernels_per_step()
+        counts = step(h)
+        out = h.get_state(), counts, h.kernels_per_step() > few
+        h.close()
+        return out
+
+    ref, counts, _ = run(lambda h: [h.step(1)["n_contacts"] for _ in range(n)])
+    assert max(counts) > 768
+    state, _, launches = run(lambda h: h.step(n))
+    assert launches and all(np.array_equal(p, q) for p, q in zip(state, ref))
+
+    def queued(h):
+        h.step_async(n // 2)
+        for _ in range(n // 2):
+            h.step_async()
+        h.sync()
+
+    state, _, _ = run(queued)
+    assert all(np.array_equal(p, q) for p, q in zip(state, ref))
