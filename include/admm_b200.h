@@ -438,6 +438,10 @@ int  admm_learn_loss_grad(AdmmLearn* L, int K, const float* omega, const float* 
                           float* g_theta);
 int  admm_learn_solve(AdmmLearn* L, const float* b, float* x, double rel_tol, int max_iter, int* iters);
 int  admm_learn_set_residual_weight(AdmmLearn* L, double mu);
+/* Most device memory that the vectors of the samples that admm_learn_loss_grad takes at
+ * once may use (2 GiB by default); one sample at least, and fewer samples at once where
+ * the device has less. */
+int  admm_learn_set_batch_bytes(AdmmLearn* L, size_t bytes);
 
 /* The global-step matrix A of a handle: nnz of the off-diagonal part when start
  * is NULL, else its CSR (start[n_dyn+1], col, val) and diagonal (host). */

@@ -412,7 +412,9 @@ struct AdmmLearn {
     float *gm = nullptr, *gth = nullptr;
     double* coef = nullptr;  // [2 kMaxK] dL/domega_k, dL/dbeta_k interleaved
     double mu = 0.0;         // weight of the residual term
-    // workspaces, grown to the largest call: a batch's vectors; the partials and scalars
+    size_t batch_bytes = (size_t)2 << 30;  // most a batch's vectors may take (one sample at least)
+    // workspaces, one sample's from the start, grown to the largest call: a batch's vectors; the
+    // partials and scalars
     float* work = nullptr;
     size_t work_floats = 0;
     double* dwork = nullptr;
@@ -431,19 +433,27 @@ int lalloc(AdmmLearn* L, T** p, size_t count) {
     return ADMM_OK;
 }
 
-// At least `count` elements at *p (their contents are lost when it grows).
+// At least `count` elements at *p (their contents are lost when it grows); *p stays as it is when
+// they cannot be had.
 template <class T>
 int grow(T** p, size_t* have, size_t count) {
     if (*have >= count) return ADMM_OK;
-    cudaFree(*p);
-    *p = nullptr;
-    *have = 0;
-    if (cudaMalloc((void**)p, count * sizeof(T)) != cudaSuccess) {
+    T* q = nullptr;
+    if (cudaMalloc((void**)&q, count * sizeof(T)) != cudaSuccess) {
         cudaGetLastError();
         return ADMM_ERR_OOM;
     }
+    cudaFree(*p);
+    *p = q;
     *have = count;
     return ADMM_OK;
+}
+
+// Workspace of `samples` samples of K sweeps.
+int grow_batch(AdmmLearn* L, int K, int samples) {
+    const size_t n = L->n, gb = nblk(n, kT), ge = std::min<size_t>(gb, kParts);
+    if (int rc = grow(&L->work, &L->work_floats, samples * ((2 * K + 9) * 3 * n + n))) return rc;
+    return grow(&L->dwork, &L->dwork_doubles, samples * (4 + 4 * ge + 2 * K * gb));
 }
 
 TrainMat matrix_of(const AdmmLearn* L) { return {L->start, L->col, L->val, L->diag, L->n, 3 * (size_t)L->n}; }
@@ -465,7 +475,8 @@ int admm_learn_create(int n, const int32_t* start, const int32_t* col, const flo
     int rc = ADMM_OK;
     if ((rc = lalloc(L, &L->start, n + 1)) || (rc = lalloc(L, &L->col, nnz)) || (rc = lalloc(L, &L->val, nnz)) ||
         (rc = lalloc(L, &L->diag, n)) || (rc = lalloc(L, &L->m, n)) || (rc = lalloc(L, &L->th, n)) ||
-        (rc = lalloc(L, &L->gm, n)) || (rc = lalloc(L, &L->gth, n)) || (rc = lalloc(L, &L->coef, 2 * kMaxK))) {
+        (rc = lalloc(L, &L->gm, n)) || (rc = lalloc(L, &L->gth, n)) || (rc = lalloc(L, &L->coef, 2 * kMaxK)) ||
+        (rc = grow_batch(L, kMaxK, 1))) {
         admm_learn_destroy(L);
         return rc;
     }
@@ -509,11 +520,14 @@ int admm_learn_loss_grad(AdmmLearn* L, int K, const float* omega, const float* b
     const TrainMat M = matrix_of(L);
     const int gb = nblk(n, kT), ge = std::min(gb, kParts);
     cudaStream_t st = L->st;
-    // samples per batch: 2 K + 9 vectors each, at most 2 GiB together (one at least)
+    // samples per batch: 2 K + 9 vectors each, and fewer where the device has no memory for them (the
+    // workspace of one has been there from the start)
     const size_t per = (size_t)(2 * K + 9) * N3 + n;
-    const int most = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nsamp, ((size_t)2 << 30) / (4 * per), 32768}));
-    if (int rc = grow(&L->work, &L->work_floats, per * most)) return rc;
-    if (int rc = grow(&L->dwork, &L->dwork_doubles, (size_t)most * (4 + 4 * (size_t)ge + 2 * (size_t)K * gb))) return rc;
+    int most = (int)std::max<size_t>(1, std::min<size_t>({(size_t)nsamp, L->batch_bytes / (4 * per), 32768}));
+    while (grow_batch(L, K, most) != ADMM_OK) {
+        if (most == 1) return ADMM_ERR_OOM;
+        most /= 2;
+    }
     cudaMemcpyAsync(L->m, m, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     cudaMemcpyAsync(L->th, theta, sizeof(float) * n, cudaMemcpyHostToDevice, st);
     cudaMemsetAsync(L->gm, 0, sizeof(float) * n, st);
@@ -579,6 +593,12 @@ int admm_learn_loss_grad(AdmmLearn* L, int K, const float* omega, const float* b
         for (int k = 0; k < K; k++) g_omega[k] = (float)coef[2 * k];
     if (g_beta)
         for (int k = 0; k < K; k++) g_beta[k] = k > 0 ? (float)coef[2 * k + 1] : 0.f;
+    return ADMM_OK;
+}
+
+int admm_learn_set_batch_bytes(AdmmLearn* L, size_t bytes) {
+    if (!L) return ADMM_ERR_INVALID;
+    L->batch_bytes = bytes;
     return ADMM_OK;
 }
 

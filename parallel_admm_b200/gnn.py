@@ -53,6 +53,7 @@ def _lib():
                                                     _d, _f, _f, _f, _f]),
             "admm_learn_solve": (ctypes.c_int, [vp, _f, _f, ctypes.c_double, ctypes.c_int, _i]),
             "admm_learn_set_residual_weight": (ctypes.c_int, [vp, ctypes.c_double]),
+            "admm_learn_set_batch_bytes": (ctypes.c_int, [vp, ctypes.c_size_t]),
         }
         for name, (res, args) in sig.items():
             fn = getattr(L, name)
@@ -297,9 +298,10 @@ class LearnedPreconditioner:
 
 
 class SweepTrainer:
-    """GPU context of the learned global step's training on one system (learn.cu)."""
+    """GPU context of the learned global step's training on one system (learn.cu).  batch_bytes: most
+    device memory of the samples that loss_grad takes at once (2 GiB by default, one sample at least)."""
 
-    def __init__(self, sysm: System, residual_weight: float = 0.0):
+    def __init__(self, sysm: System, residual_weight: float = 0.0, batch_bytes: Optional[int] = None):
         self.sysm = sysm
         self.L = vp()
         rc = _lib().admm_learn_create(sysm.n, _p(sysm.start, _i), _p(sysm.col, _i), _p(sysm.val, _f),
@@ -310,6 +312,10 @@ class SweepTrainer:
             rc = _lib().admm_learn_set_residual_weight(self.L, float(residual_weight))
             if rc != B.OK:
                 raise B.AdmmError(rc, "admm_learn_set_residual_weight")
+        if batch_bytes is not None:
+            rc = _lib().admm_learn_set_batch_bytes(self.L, batch_bytes)
+            if rc != B.OK:
+                raise B.AdmmError(rc, "admm_learn_set_batch_bytes")
 
     def close(self):
         if self.L:
