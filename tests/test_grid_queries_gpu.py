@@ -51,3 +51,24 @@ def test_grid_query_ranges(case, lanes, semantics):
     assert n == len(ref) and n > 0
     assert sorted(map(tuple, h.contacts()["pairs"].tolist())) == sorted(map(tuple, ref.tolist()))
     h.close()
+
+
+@pytest.mark.parametrize("lanes", [8, 16, 32])
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_non_finite_vertex(value, lanes):
+    """A vertex without a finite position leaves the pairs of the elements that it is no part of as
+    they are when it is far away."""
+    sc, x = _scattered(*CASES["lists"], seed=5)
+    sc.params.query_lanes = lanes
+    sc.params.broad_phase = 2
+    v = 100
+    out = []
+    for p in ((50.0, 50.0, 50.0), (value, value, value), (float(x[v, 0]), value, float(x[v, 2]))):
+        h = B.Handle(sc)
+        y = x.copy()
+        y[v] = p
+        h.detect(y)
+        pairs = h.contacts()["pairs"]
+        out.append(sorted(map(tuple, pairs[(pairs != v).all(1)].tolist())))
+        h.close()
+    assert out[0] and out[1] == out[0] and out[2] == out[0]

@@ -147,3 +147,23 @@ def test_learned_step_before_its_model(sweeps):
         for p, q in zip(a.get_state(), b.get_state()):
             assert np.array_equal(p, q)
     assert a.learned_stats() == b.learned_stats()
+
+
+@pytest.mark.parametrize("tol", [0.0, 1e-4])
+@pytest.mark.parametrize("lanes", [1, 4])
+def test_learned_bodies_bitwise(lanes, tol):
+    """Several bodies in a group: vertex-wise m and theta, and one partial sum per CTA."""
+    from parallel_admm_b200 import gnn
+    SCENES["small bodies"] = lambda: S.batch_bodies(n_bodies=12, seed=3, vmin=100, vmax=600)
+    a, b = _pair("small bodies", lanes, global_solver=3, residual_tol=tol)
+    rng = np.random.default_rng(1)
+    m = (rng.uniform(0.8, 1.1, a.n_dyn) / gnn.system(a).diag).astype(np.float32)
+    theta = rng.uniform(-0.5, 0.5, a.n_dyn).astype(np.float32)
+    for h in (a, b):
+        h.set_learned(np.full(5, 0.9, np.float32), np.full(5, 0.1, np.float32), m, theta)
+    for _ in range(3):
+        for h in (a, b):
+            h.step(1, allow=(B.ERR_CONTACT_OVERFLOW,))
+        for p, q in zip(a.get_state(), b.get_state()):
+            assert np.array_equal(p, q)
+    assert a.learned_stats() == b.learned_stats()
