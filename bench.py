@@ -562,6 +562,14 @@ def main():
         cpu = {"value": rate, "unit": "steps/s", "cores": cores, "kind": "port", "sample": desc}
     tn, gm = h.tuning(), h.global_mode()
     tuned = {"jacobi_lanes": tn["jacobi_lanes"], "rhs_lanes": tn["rhs_lanes"], "global_mode": gm["mode"]}
+    # sweeps in a launch of the probed class: all of a global step in the resident mode (the bytes of
+    # a launch are then those of one pass over the matrix), two over the tiles
+    sweeps, kernel_name = 1, {"learned": "k_lsweep (learned sweep)"}.get(pk, args.probe)
+    if pk in ("jacobi", "learned") and gm["mode"] == "resident":
+        sweeps = int(main_r["info"]["sweeps"]) if pk == "learned" else sc.params.jacobi_iter
+        kernel_name = f"k_resident_{pk}"
+    elif pk == "jacobi" and gm["mode"] == "tiled":
+        sweeps = 2
     cfg = {"workload": CONFIGS[args.config]["workload"], "frames": f"{args.start_frame}..{args.start_frame + args.steps - 1}",
            "n_vert": sc.n_vert, "n_rows": sc.n_rows, "parallelism": f"replicas x{world}",
            "l2": "flushed (256 MiB write) between timed steps", "residual_tol": args.tol,
@@ -579,7 +587,7 @@ def main():
         "dtype": "f32", "data": "synthetic", "config": cfg,
         "e2e": {"value": e2e_value, "unit": "steps/s", "h2d_bytes_per_step": bytes_io, "d2h_bytes_per_step": bytes_io},
         "gpu_launches": main_r["launches"] + (res["jacobi"]["launches"] if args.solver == "learned" else 0),
-        "roofline": {"bound": "hbm", "kernel": {"learned": "k_lsweep (learned sweep)"}.get(pk, args.probe),
+        "roofline": {"bound": "hbm", "kernel": kernel_name, "sweeps_per_launch": sweeps,
                      "achieved": achieved, "peak": peak_gbs,
                      "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": (achieved / peak_gbs) if achieved else None, "traffic": traffic,
