@@ -382,8 +382,8 @@ int  admm_b200_record_global(AdmmB200* h, int iteration, float* b, float* x_cur,
 /* How the global step runs (jacobi_mode): persistent = 1 for the one-kernel
  * global step (blocks = its grid), 3 for two sweeps per launch over row tiles, 4 for
  * all sweeps in one launch with the matrix in shared memory (blocks = its grid),
- * 0 for one kernel per sweep; the autotuner's ms per global step with one
- * kernel per sweep and with the persistent kernel (0 when not timed). */
+ * 0 for one kernel per sweep; ms_sweeps: the autotuner's ms per global step with one
+ * kernel per sweep (0 when not timed); ms_persist: 0 (the persistent kernel is not timed). */
 int  admm_b200_global_mode(AdmmB200* h, int* persistent, int* blocks, float* ms_sweeps, float* ms_persist);
 
 /* --- learned block preconditioner (an addition with no reference counterpart) ---

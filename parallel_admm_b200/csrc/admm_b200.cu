@@ -141,7 +141,7 @@ struct AdmmB200 {
     HostCsr hostA;                  // the global matrix on the host (admm_b200_system)
     std::vector<float> hostAdiag;
     float tune_ms_tiled = 0.f;
-    float tune_ms_persist = 0.f, tune_ms_sweeps = 0.f;  // one global step, both modes
+    float tune_ms_sweeps = 0.f;     // one global step with a kernel per sweep
     // host-buffer stepping
     float* stage = nullptr;    // row-major host rows on their way to or from the device
     size_t stage_floats = 0;
@@ -1090,13 +1090,12 @@ int build_resident_plan(AdmmB200* h, const HostCsr& A, const std::vector<float>&
     return ADMM_OK;
 }
 
-// Milliseconds of one global step (RHS + jac_iter sweeps) in the given mode,
-// timed as a captured graph of 8 global steps (as the substep graph runs them,
+// Milliseconds of one global step (RHS + jac_iter sweeps), with a launch per sweep or two sweeps
+// per launch (tiled), timed as a captured graph of 8 global steps (as the substep graph runs them,
 // with programmatic dependent launch); +inf when the mode cannot be captured.
-int time_global(AdmmB200* h, int mode, float* ms) {
-    const bool keep = h->persist, keep_t = h->tiled;
-    h->persist = mode == 2;
-    h->tiled = mode == 3;
+int time_global(AdmmB200* h, bool tiled, float* ms) {
+    const bool keep_t = h->tiled;
+    h->tiled = tiled;
     h->force_plain = true;
     h->cstream = h->stream;
     constexpr int kReps = 8;
@@ -1109,7 +1108,6 @@ int time_global(AdmmB200* h, int mode, float* ms) {
     }
     ok = ok && cudaGraphInstantiate(&ge, g, 0) == cudaSuccess;
     if (g) cudaGraphDestroy(g);
-    h->persist = keep;
     h->tiled = keep_t;
     h->force_plain = false;
     if (!ok) {
@@ -1125,9 +1123,6 @@ int time_global(AdmmB200* h, int mode, float* ms) {
     CK(cudaEventSynchronize(h->ev1));
     cudaGraphExecDestroy(ge);
     CK(cudaGetLastError());
-    int e[4] = {0, 0, 0, 0};
-    CK(cudaMemcpy(e, h->s.err, sizeof(e), cudaMemcpyDeviceToHost));
-    if (e[3]) return fail(h, ADMM_ERR_TIMEOUT, "persistent global step: a block wait timed out");
     float t = 0.f;
     CK(cudaEventElapsedTime(&t, h->ev0, h->ev1));
     *ms = t / kReps;
@@ -1469,9 +1464,9 @@ int build_step_graph(AdmmB200* h) {
 // next ones with launches 1.4 / 1.9 ms).  So a launch each, too, where the counts of the last
 // kCountRing * kPeaks substeps have not arrived (a long step_async).  Only for scenes of up to
 // kSmallSurface surface vertices: on larger ones the local step, which runs beside the contact step,
-// takes as long as the launches.  Measured per ADMM iteration: 5 contacts 24.6 us with launches.
-// Two thresholds, so that a count near them does not switch graphs back and forth; probed substeps
-// keep what they were captured with.
+// takes as long as the launches.  A 32^2 cloth with few contacts: 0.64 ms per substep of 20 iterations
+// in one block, 0.98 with launches.  Two thresholds, so that a count near them does not switch graphs
+// back and forth; probed substeps keep what they were captured with.
 constexpr int kSmallSurface = 8192, kOneAgain = 512, kCalm = 4;
 
 // peaks: the largest counts of the last kPeaks substeps.
@@ -1994,18 +1989,20 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     h->hostAdiag = as.a_diag;
     h->persist = h->tiled = false;
     if (!h->resident && h->jac_iter >= 2 && (d->global_solver == 0 || d->global_solver == 3)) {
-        if (d->jacobi_mode == 2) TRY(build_persist_plan(h, as.A));  // slower than launches wherever it was timed
+        if (d->jacobi_mode == 2) TRY(build_persist_plan(h, as.A));  // only on request: slower than launches wherever it was timed
+        int sms = 148;
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
         // two sweeps per launch pay while a launch is bound by latency: up to a tile per SM
-        const bool try_tiles = d->jacobi_mode == 0 && s.nd <= 148 * kTileOwnMax;
+        const bool try_tiles = d->jacobi_mode == 0 && s.nd <= sms * kTileOwnMax;
         if (try_tiles || d->jacobi_mode == 3) TRY(build_tiles_dev(h, as.A));
         if (d->jacobi_mode == 2 && h->persist_ok) {
             h->persist = true;
         } else if (d->jacobi_mode == 3) {
             h->tiled = true;
         } else if (d->jacobi_mode == 0) {
-            TRY(time_global(h, 1, &h->tune_ms_sweeps));
+            TRY(time_global(h, false, &h->tune_ms_sweeps));
             h->tune_ms_tiled = 1e30f;
-            if (try_tiles) TRY(time_global(h, 3, &h->tune_ms_tiled));
+            if (try_tiles) TRY(time_global(h, true, &h->tune_ms_tiled));
             h->tiled = h->tune_ms_tiled < h->tune_ms_sweeps;
         }
     }
@@ -2967,7 +2964,7 @@ int admm_b200_global_mode(AdmmB200* h, int* persistent, int* blocks, float* ms_s
     if (persistent) *persistent = h->resident ? 4 : h->persist ? 1 : h->tiled ? 3 : 0;
     if (blocks) *blocks = h->resident ? h->res.groups * h->res.cluster : h->persist ? h->pp.blocks : 0;
     if (ms_sweeps) *ms_sweeps = h->tune_ms_sweeps;
-    if (ms_persist) *ms_persist = h->tune_ms_persist;
+    if (ms_persist) *ms_persist = 0.f;
     return ADMM_OK;
 }
 
