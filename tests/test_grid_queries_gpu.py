@@ -72,3 +72,26 @@ def test_non_finite_vertex(value, lanes):
         out.append(sorted(map(tuple, pairs[(pairs != v).all(1)].tolist())))
         h.close()
     assert out[0] and out[1] == out[0] and out[2] == out[0]
+
+
+@pytest.mark.parametrize("n", [8, 56])
+def test_contact_arrays_one_by_one(n):
+    """Contacts read all at once (records up to 4096 of them, arrays above) and array by array."""
+    import ctypes
+    v, f = scene.grid_cloth(n, 1.0)
+    e = 1.0 / (n - 1)
+    bodies = [scene._Body(v + np.array([0.0, 0.5 + 0.3 * e * k, 0.0]), f, np.zeros((0, 4), np.int32), 0.1, 1e3, 1e-3)
+              for k in range(2)]
+    h = B.Handle(scene.assemble("two", bodies, [], scene.SolverParams(thickness=e, max_contacts=1_000_000)))
+    k = h.detect()
+    assert (k > 4096) == (n == 56)
+    every = h.contacts()
+    names = ["pairs", "bary", "normal", "point", "gap"]
+    cnt = ctypes.c_int32()
+    for ask in [(name,) for name in names] + [("pairs", "point"), ("bary", "normal", "point"), ("pairs", "gap", "point")]:
+        out = {a: np.zeros_like(every[a]) for a in ask}
+        ptr = [out[a].ctypes.data_as(ctypes.POINTER(ctypes.c_int32 if a == "pairs" else ctypes.c_float)) if a in out
+               else None for a in names]
+        assert B.lib().admm_b200_contacts(h.h, *ptr, k, ctypes.byref(cnt)) == B.OK and cnt.value == k
+        assert all(np.array_equal(out[a], every[a]) for a in ask), ask
+    h.close()
