@@ -72,15 +72,14 @@ void* current_context() {
 
 // One Jacobi sweep on CSR (off-diagonal part, JacobiFunctor of the reference's
 // jacobi_solver.cu:52-98): dst_i = (b_i - sum_{j != i} a_ij src_j) / a_ii,
-// row-major n x 3 vectors.  Bound by the chain of dependent loads of a row, not by bytes: four
-// lanes share a row, its first kPre entries per lane are loaded before the dependency wait (the
+// row-major n x 3 vectors.  Bound by the chain of dependent loads of a row, not by bytes: four (or
+// two) lanes share a row, its first kPre entries per lane are loaded before the dependency wait (the
 // sweeps after a call's first one launch while the sweep before them drains; the first one
 // starts after everything before it, so the matrix and b are complete by then).  src and dst are
 // not __restrict__: the sweep before still writes src when this one starts, so src must not be
 // read through the read-only path, nor before the wait.  28 k rows of 11
 // entries, 20 sweeps: 157 us with a thread per row.
-constexpr int kRowLanes = 4, kPre = 4;
-
+template <int kRowLanes, int kPre>  // lanes per row, entries per lane before the wait
 __global__ void __launch_bounds__(128) k_jacobi_csr(int n, const int32_t* __restrict__ start,
                                                     const int32_t* __restrict__ cols, const float* __restrict__ vals,
                                                     const float* __restrict__ diag, const float* __restrict__ b,
@@ -129,6 +128,11 @@ __global__ void __launch_bounds__(128) k_jacobi_csr(int n, const int32_t* __rest
     dst[3 * (size_t)i + 1] = (b1 - ay) / d;
     dst[3 * (size_t)i + 2] = (b2 - az) / d;
 }
+
+// More rows than two lanes each fill the device with at once (148 SMs of 2048 threads) have two: there
+// the rounds of blocks count, and short rows waste four lanes.  262144 rows of 2 / 14 / 40 entries, 20
+// sweeps: 117 / 158 / 548 us with two lanes, 195 / 207 / 404 with four, 124 / 215 / 942 with one.
+constexpr int kFourLaneRows = 148 * 2048 / 2;
 
 // Device address of g_jacobi_scratch in the current context: looked up again on
 // every call outside capture (cheap), taken from the per-context record during
@@ -198,13 +202,14 @@ extern "C" int admm_b200_jacobi_noalloc(int n, const int32_t* row_start, const i
         return ADMM_OK;
     }
     float* buf[2] = {scratch, scratch + (size_t)kNoAllocMaxRows * 3};
-    const int threads = 128, blocks = (n * kRowLanes + threads - 1) / threads;
+    const int lanes = n > kFourLaneRows ? 2 : 4;
+    const int threads = 128, blocks = (n * lanes + threads - 1) / threads;
     for (int k = 0; k < sweeps; k++) {
         const float* src = k == 0 ? x_in : buf[(k - 1) & 1];
         // the last sweep writes x_out directly unless x_out is also its source
         float* dst = (k == sweeps - 1 && src != x_out) ? x_out : buf[k & 1];
-        if (admm::launch_k(k_jacobi_csr, dim3(blocks), dim3(threads), 0, st, k > 0, n, row_start, cols, vals, diag, b,
-                           src, dst) != cudaSuccess)
+        if (admm::launch_k(lanes == 2 ? k_jacobi_csr<2, 6> : k_jacobi_csr<4, 4>, dim3(blocks), dim3(threads), 0, st, k > 0,
+                           n, row_start, cols, vals, diag, b, src, dst) != cudaSuccess)
             return ADMM_ERR_CUDA;
         if (k == sweeps - 1 && dst != x_out &&
             cudaMemcpyAsync(x_out, dst, bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess)

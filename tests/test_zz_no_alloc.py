@@ -171,3 +171,28 @@ def test_noalloc_overlapped_sweeps(n):
         out = torch.full_like(ref, float("nan"))
         sweeps(x[0], out, k)
         assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("n", [151_552, 151_553])
+def test_noalloc_lanes_per_row(n):
+    """One sweep on rows of 0 to 60 entries, with four lanes per row and with two: within the rounding
+    of L products and sums, (L + 3) 2^-24 (|b| + sum |a x|) / d, of the sweep in FP64."""
+    import torch
+    torch.cuda.set_device(0)
+    rng = np.random.default_rng(n)
+    size = rng.choice([0, 1, 2, 5, 12, 13, 16, 17, 30, 60], size=n)
+    start = np.concatenate([[0], np.cumsum(size)])
+    col = rng.integers(0, n, start[-1]).astype(np.int32)
+    val = rng.normal(size=start[-1]).astype(np.float32)
+    diag = rng.uniform(1.0, 2.0, n).astype(np.float32)
+    b, x = (rng.normal(size=(n, 3)).astype(np.float32) for _ in range(2))
+    dev = [torch.from_numpy(np.ascontiguousarray(a)).to("cuda:0") for a in (start.astype(np.int32), col, val, diag, b, x)]
+    out = torch.full_like(dev[5], float("nan"))
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert B.lib().admm_b200_jacobi_noalloc(n, *(_ptr(t) for t in dev), _ptr(out), 1, st) == B.OK
+    terms = val[:, None].astype(np.float64) * x[col]
+    rows = np.repeat(np.arange(n), size)
+    ax, mag = (np.stack([np.bincount(rows, t[:, c], n) for c in range(3)], 1) for t in (terms, np.abs(terms)))
+    d = diag[:, None].astype(np.float64)
+    bound = (size[:, None] + 3) * 2.0 ** -24 * (np.abs(b) + mag) / d
+    assert (np.abs(out.cpu().numpy() - (b - ax) / d) <= bound).all()
