@@ -39,6 +39,9 @@ constexpr int kParts = 592;  // most blocks of the reduction kernels (4 x 148 SM
 // queued past the end 3 us.
 constexpr int kCgChunk = 16;
 constexpr int kCgAhead = 16;  // entries of a row loaded before the dependency wait
+// most blocks of a conjugate-gradient kernel (16 x 148 SMs: every thread the device holds at once;
+// 1.45 M rows, 128 iterations: 23 ms against 28 with kParts)
+constexpr int kCgParts = 2368;
 constexpr int kMaxK = 32;
 
 inline int nblk(size_t n, int t) { return (int)((n + t - 1) / t); }
@@ -291,15 +294,52 @@ __global__ void __launch_bounds__(kT) k_cg_init(TrainMat M, const float* __restr
     block_sum2(acc, 0.0, sh, part + blockIdx.x, nullptr);
 }
 
+// Up to so many rows k_cg_q makes the direction itself: a launch less, but every neighbour's z and p
+// gathered and combined in FP64.  128 iterations on rows of 14 entries, direction in k_cg_q / in k_cg_p:
+// 9 k rows 1.85 / 1.92 ms, 16 k 1.88 / 1.85, 100 k 4.0 / 3.2, 1.45 M 30.7 / 22.7.
+constexpr int kFusedRows = 16384;
+
 // Entry q of the direction z + beta p (p null: z).
 __device__ __forceinline__ float cg_direction(const float* z, const float* p, int q,
                                               double beta) {
     return p ? (float)((double)z[q] + beta * (double)p[q]) : z[q];
 }
 
-// Iteration `it`: rz = the sum of the partials of the last kernel; ends here once rz has dropped
-// by rel_tol^2, or is 0; else p_new = z + (rz / rz_old) p and q = A p_new (the neighbours' p_new
-// computed from their z and p), part = p_new . q.
+// The state at the start of iteration `it`, by every block alike: rz = the sum of the partials of the
+// last kernel; ends here (false) once rz has dropped by rel_tol^2, or is 0; else *beta for the new
+// direction.
+__device__ __forceinline__ bool cg_begin(int nparts, const double* parts_in, double rel_tol2, int it, const CgState* old,
+                                         CgState* cur, double* sh, double* beta) {
+    const CgState s0 = *old;
+    const double rz = s0.done ? s0.rz : parts_sum(parts_in, nparts, sh);
+    const double rz0 = it == 0 ? rz : s0.rz0;
+    const bool done = s0.done || !(rz > rel_tol2 * rz0 && rz > 0.0);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        CgState c = s0;
+        c.rz0 = rz0;
+        c.rz = rz;
+        c.done = done;
+        *cur = c;
+    }
+    *beta = it == 0 ? 0.0 : rz / s0.rz;
+    return !done;
+}
+
+// The direction of iteration `it` on its own, before k_cg_q<false>: p = z + (rz / rz_old) p.
+__global__ void __launch_bounds__(kT) k_cg_p(TrainMat M, const float* z, float* p, int nparts, const double* parts_in,
+                                             double rel_tol2, int it, const CgState* old, CgState* cur) {
+    __shared__ double sh[2 * kT];
+    ADMM_PDL_PROLOGUE();
+    double beta;
+    if (!cg_begin(nparts, parts_in, rel_tol2, it, old, cur, sh, &beta)) return;
+    for (size_t k = blockIdx.x * blockDim.x + threadIdx.x; k < M.n3; k += gridDim.x * blockDim.x)
+        p[k] = it == 0 ? z[k] : (float)((double)z[k] + beta * (double)p[k]);
+}
+
+// Iteration `it`, unless it ends in cg_begin: p_new = z + (rz / rz_old) p and q = A p_new (the
+// neighbours' p_new computed from their z and p), part = p_new . q.  FUSED = false: p_new is z, and
+// the state cur, from k_cg_p.
+template <bool FUSED>
 __global__ void __launch_bounds__(kT) k_cg_q(TrainMat M, const float* z, const float* p,
                                              int nparts, const double* parts_in, double rel_tol2, int it,
                                              const CgState* old, CgState* cur,
@@ -320,20 +360,9 @@ __global__ void __launch_bounds__(kT) k_cg_q(TrainMat M, const float* z, const f
         ahead_val[k] = e0 + k < e1 ? M.val[e0 + k] : 0.f;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const CgState s0 = *old;
-    const double rz = s0.done ? s0.rz : parts_sum(parts_in, nparts, sh);
-    const double rz0 = it == 0 ? rz : s0.rz0;
-    const bool done = s0.done || !(rz > rel_tol2 * rz0 && rz > 0.0);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        CgState c = s0;
-        c.rz0 = rz0;
-        c.rz = rz;
-        c.done = done;
-        *cur = c;
-    }
-    if (done) return;
-    const double beta = it == 0 ? 0.0 : rz / s0.rz;
-    const float* pp = it == 0 ? nullptr : p;
+    double beta = 0.0;
+    if (FUSED ? !cg_begin(nparts, parts_in, rel_tol2, it, old, cur, sh, &beta) : cur->done != 0) return;
+    const float* pp = FUSED && it > 0 ? p : nullptr;
     double acc = 0.0;
     for (int i = first; i < M.n; i += gridDim.x * blockDim.x) {
         const bool ahead = i == first;
@@ -360,7 +389,7 @@ __global__ void __launch_bounds__(kT) k_cg_q(TrainMat M, const float* z, const f
             for (int c = 0; c < 3; c++) a[c] = fmaf(w, cg_direction(z, pp, 3 * j + c, beta), a[c]);
         }
         for (int c = 0; c < 3; c++) {
-            pn[3 * i + c] = pi[c];
+            if (FUSED) pn[3 * i + c] = pi[c];
             q[3 * i + c] = a[c];
             acc += (double)a[c] * (double)pi[c];
         }
@@ -613,7 +642,7 @@ int admm_learn_solve(AdmmLearn* L, const float* b, float* x, double rel_tol, int
     const int n = L->n;
     const size_t N3 = 3 * (size_t)n;
     const TrainMat M = matrix_of(L);
-    const int ge = std::min(nblk(n, kT), kParts);
+    const int ge = std::min(nblk(n, kT), kCgParts);
     cudaStream_t st = L->st;
     if (int rc = grow(&L->work, &L->work_floats, 7 * N3)) return rc;
     constexpr size_t kState = sizeof(CgState) / sizeof(double);
@@ -627,12 +656,20 @@ int admm_learn_solve(AdmmLearn* L, const float* b, float* x, double rel_tol, int
     cudaMemcpyAsync(dx, x, sizeof(float) * N3, cudaMemcpyHostToDevice, st);
     k_cg_init<<<ge, kT, 0, st>>>(M, db, dx, r, z, part[0]);
     CgState now = {};
+    const bool fused = n <= kFusedRows;
     for (int it = 0; it < max_iter && !now.done;) {
         for (const int end = std::min(max_iter, it + kCgChunk); it < end; it++) {
-            admm::launch_k(k_cg_q, ge, kT, 0, st, true, M, z, p[it & 1], ge, part[0], rel_tol * rel_tol, it, state[0],
-                           state[1], p[(it + 1) & 1], q, part[1]);
-            admm::launch_k(k_cg_xr, ge, kT, 0, st, true, M, p[(it + 1) & 1], q, ge, part[1], state[1], state[0], dx, r,
-                           z, part[0]);
+            float* pn = p[fused ? (it + 1) & 1 : 0];
+            if (fused) {
+                admm::launch_k(k_cg_q<true>, ge, kT, 0, st, true, M, z, p[it & 1], ge, part[0], rel_tol * rel_tol, it,
+                               state[0], state[1], pn, q, part[1]);
+            } else {
+                admm::launch_k(k_cg_p, ge, kT, 0, st, true, M, z, pn, ge, part[0], rel_tol * rel_tol, it, state[0],
+                               state[1]);
+                admm::launch_k(k_cg_q<false>, ge, kT, 0, st, true, M, pn, nullptr, ge, part[0], rel_tol * rel_tol, it,
+                               state[0], state[1], nullptr, q, part[1]);
+            }
+            admm::launch_k(k_cg_xr, ge, kT, 0, st, true, M, pn, q, ge, part[1], state[1], state[0], dx, r, z, part[0]);
         }
         if (cudaMemcpyAsync(&now, state[0], sizeof(now), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)

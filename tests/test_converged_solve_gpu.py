@@ -31,3 +31,10 @@ def test_solve_row_shapes(n, side):
     tr.close()
     r = b - sysm.matvec(x.astype(np.float64))
     assert it > 0 and np.linalg.norm(r) <= 1e-5 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n", [16_384, 16_385, 303_105])
+def test_solve_row_counts(n):
+    """The largest system whose iteration takes two launches, the smallest with three, and one more
+    row than the kernels have threads."""
+    test_solve_row_shapes(n, 3)
