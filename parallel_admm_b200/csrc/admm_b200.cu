@@ -58,14 +58,13 @@ struct AdmmB200 {
     // The contact passes run in one block (contact_one.cuh) or with a launch each; the graph of the
     // other choice is kept while it lasts (pick_contact_passes).
     bool contact_one = false, contact_small = false;
-    int calm = 0;                   // looks at the contact counts since the last one with many
-    bool calm_now = true;           // the last one had few
-    // Contact counts of substeps that no status read follows, on their way to the host: sent after
-    // every kPeaks-th substep.
-    static constexpr int kCountRing = 16;
-    cudaEvent_t count_ev[kCountRing] = {};
-    int* count_host = nullptr;      // pinned [kCountRing * kPeaks]
-    int64_t count_sent = 0, count_seen = 0;
+    int calm = 1;                   // looks in a row at the one-block passes' score that found them faster
+    // Scores of substeps that no status read follows, on their way to the host: sent after every
+    // kScores-th substep.
+    static constexpr int kScoreRing = 16;
+    cudaEvent_t score_ev[kScoreRing] = {};
+    int* score_host = nullptr;      // pinned [kScoreRing * kScores]
+    int64_t score_sent = 0, score_seen = 0;
     int unsent = 0;                 // substeps since the last one sent or read
     struct OtherGraph {
         cudaGraphExec_t exec = nullptr;
@@ -254,8 +253,8 @@ int alloc_bvh(AdmmB200* h, BvhDev& t, int n) {
     return ADMM_OK;
 }
 
-constexpr int kPeaks = 4;                       // substeps of nc_peaks
-constexpr int kStatusWords = kPeakWord + kPeaks;  // err[4], nc, nc_raw, -, -, nc_peaks
+constexpr int kScores = 4;                          // substeps of one_score
+constexpr int kStatusWords = kScoreWord + kScores;  // err[4], nc, nc_raw, -, -, one_score
 
 // The captured substep graphs are out of date.
 void drop_graphs(AdmmB200* h) {
@@ -1456,61 +1455,61 @@ int build_step_graph(AdmmB200* h) {
     return build_step_graph_once(h);
 }
 
-// How the contact passes of the next substep run: in one block after kCalm looks at the last kPeaks
-// substeps found few contacts in every detection (a cloth on the ground may go from none to thousands
-// and back from one detection of a substep to the next), else with a launch each; the same bits
-// either way, and a substep that the guess missed is still right, but slower (contact_one_global;
-// the first substep in which a cloth of 64^2 / 88^2 vertices lands on the ground: 1.9 / 3.7 ms, the
-// next ones with launches 1.4 / 1.9 ms).  So a launch each, too, where the counts of the last
-// kCountRing * kPeaks substeps have not arrived (a long step_async).  Only for scenes of up to
-// kSmallSurface surface vertices: on larger ones the local step, which runs beside the contact step,
-// takes as long as the launches.  A 32^2 cloth with few contacts: 0.64 ms per substep of 20 iterations
-// in one block, 0.98 with launches.  Two thresholds, so that a count near them does not switch graphs
-// back and forth; probed substeps keep what they were captured with.
-constexpr int kSmallSurface = 8192, kOneAgain = 512, kCalm = 4;
+// How the contact passes of the next substep run: in one block while that has been faster over the
+// last kScores substeps (one_score: a cloth on the ground goes from none to thousands of contacts and
+// back from one detection of a substep to the next) and, once it has not, again after kCalm looks
+// that found it faster; else with a launch each.  The same bits either way; a substep that the guess
+// misses is still right, but slower (contact_one_global; the first substep in which a cloth of
+// 64^2 / 88^2 vertices lands on the ground: 1.9 / 3.7 ms, the next ones with launches 1.4 / 1.9 ms).
+// So a launch each, too, where the scores of the last kScoreRing * kScores substeps have not arrived
+// (a long step_async).  Only for scenes of up to kSmallSurface surface vertices: on larger ones the
+// local step, which runs beside the contact step, takes as long as the launches.  A 32^2 cloth with
+// few contacts: 0.64 ms per substep of 20 iterations in one block, 0.98 with launches.  Probed
+// substeps keep what they were captured with.
+constexpr int kSmallSurface = 8192, kCalm = 4;
 
-// peaks: the largest counts of the last kPeaks substeps.
-void note_counts(AdmmB200* h, const int* peaks) {
-    const int contacts = *std::max_element(peaks, peaks + kPeaks);
-    h->calm_now = contacts <= kOneContacts;
-    h->calm = contacts <= kOneAgain ? h->calm + 1 : 0;
+// scores: of the last kScores substeps.
+void note_scores(AdmmB200* h, const int* scores) {
+    int64_t sum = 0;
+    for (int k = 0; k < kScores; k++) sum += scores[k];
+    h->calm = sum <= 0 ? h->calm + 1 : 0;
 }
 
-// The counts that have arrived; waits until at most `behind` of those sent have not (< 0: no wait).
-int take_counts(AdmmB200* h, int behind) {
-    for (; h->count_seen < h->count_sent; h->count_seen++) {
-        const int slot = (int)(h->count_seen % AdmmB200::kCountRing);
-        if (behind >= 0 && h->count_sent - h->count_seen > behind) {
-            CK(cudaEventSynchronize(h->count_ev[slot]));
+// The scores that have arrived; waits until at most `behind` of those sent have not (< 0: no wait).
+int take_scores(AdmmB200* h, int behind) {
+    for (; h->score_seen < h->score_sent; h->score_seen++) {
+        const int slot = (int)(h->score_seen % AdmmB200::kScoreRing);
+        if (behind >= 0 && h->score_sent - h->score_seen > behind) {
+            CK(cudaEventSynchronize(h->score_ev[slot]));
         } else {
-            const cudaError_t e = cudaEventQuery(h->count_ev[slot]);
+            const cudaError_t e = cudaEventQuery(h->score_ev[slot]);
             if (e == cudaErrorNotReady) {
                 cudaGetLastError();
                 break;
             }
             CK(e);
         }
-        note_counts(h, h->count_host + slot * kPeaks);
+        note_scores(h, h->score_host + slot * kScores);
     }
     return ADMM_OK;
 }
 
-// Sends the contact counts of the substeps launched, when it is their turn.
-int send_counts(AdmmB200* h) {
-    if (!h->contact_small || ++h->unsent < kPeaks) return ADMM_OK;
+// Sends the scores of the substeps launched, when it is their turn.
+int send_scores(AdmmB200* h) {
+    if (!h->contact_small || ++h->unsent < kScores) return ADMM_OK;
     h->unsent = 0;
-    if (h->count_sent - h->count_seen == AdmmB200::kCountRing) h->count_seen++;  // its slot is written again
-    const int slot = (int)(h->count_sent % AdmmB200::kCountRing);
-    CK(cudaMemcpyAsync(h->count_host + slot * kPeaks, nc_peaks(h->s), sizeof(int) * kPeaks, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaEventRecord(h->count_ev[slot], h->stream));
-    h->count_sent++;
+    if (h->score_sent - h->score_seen == AdmmB200::kScoreRing) h->score_seen++;  // its slot is written again
+    const int slot = (int)(h->score_sent % AdmmB200::kScoreRing);
+    CK(cudaMemcpyAsync(h->score_host + slot * kScores, one_score(h->s), sizeof(int) * kScores, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaEventRecord(h->score_ev[slot], h->stream));
+    h->score_sent++;
     return ADMM_OK;
 }
 
 void pick_contact_passes(AdmmB200* h) {
     if (!h->contact_small || h->probe_kernel != 0) return;
-    const bool known = h->count_sent - h->count_seen < AdmmB200::kCountRing;
-    const bool one = known && (h->contact_one ? h->calm_now : h->calm >= kCalm);
+    const bool known = h->score_sent - h->score_seen < AdmmB200::kScoreRing;
+    const bool one = known && h->calm >= (h->contact_one ? 1 : kCalm);
     if (one == h->contact_one) return;
     h->contact_one = one;
     std::swap(h->step_exec, h->other.exec);
@@ -1917,8 +1916,8 @@ int create_impl(const AdmmB200Desc* d, int device, AdmmB200* h) {
     h->contact_small = h->contact_one = s.contact && !s.cpu_backend && s.nsv <= kSmallSurface;
     if (h->contact_small) {
         CK(cudaFuncSetAttribute(k_contact_one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ContactOneSmem)));
-        for (auto& e : h->count_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        CK(cudaHostAlloc((void**)&h->count_host, sizeof(int) * AdmmB200::kCountRing * kPeaks, cudaHostAllocDefault));
+        for (auto& e : h->score_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        CK(cudaHostAlloc((void**)&h->score_host, sizeof(int) * AdmmB200::kScoreRing * kScores, cudaHostAllocDefault));
     }
     CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking));
@@ -2153,11 +2152,11 @@ int accumulate_timers(AdmmB200* h) {
 }
 
 // n_steps substeps.  wait: the caller waits for them, so this may wait on the way for all but the
-// last 2 kPeaks, for their contact counts.
+// last 2 kScores, for their scores.
 int run_substeps(AdmmB200* h, int n_steps, bool wait) {
     if (n_steps < 0) return fail(h, ADMM_ERR_INVALID, "n_steps");
     CK(cudaSetDevice(h->device));
-    TRY(take_counts(h, -1));
+    TRY(take_scores(h, -1));
     pick_contact_passes(h);
     if (h->profiling) {
         // eager, one substep at a time so that every event pair can be read back
@@ -2176,12 +2175,12 @@ int run_substeps(AdmmB200* h, int n_steps, bool wait) {
     CK(cudaEventRecord(h->ev0, h->stream));
     for (int k = 0; k < n_steps; k++) {
         if (k > 0) {
-            TRY(take_counts(h, wait ? 1 : -1));
+            TRY(take_scores(h, wait ? 1 : -1));
             pick_contact_passes(h);
             TRY(build_step_graph(h));
         }
         TRY(launch_substep(h));
-        if (!wait || k + 1 < n_steps) TRY(send_counts(h));  // else a status read follows
+        if (!wait || k + 1 < n_steps) TRY(send_scores(h));  // else a status read follows
     }
     CK(cudaEventRecord(h->ev1, h->stream));
     h->frame += n_steps;
@@ -2189,12 +2188,12 @@ int run_substeps(AdmmB200* h, int n_steps, bool wait) {
 }
 
 // Waits for the stream; the status of what ran on it (cleared on the device) and, in
-// h->status_host, the contact counts (4: stored, 5: found, from kPeakWord: most found in each of the last kPeaks substeps).
+// h->status_host, the contact counts (4: stored, 5: found; from kScoreWord: one_score).
 int read_status(AdmmB200* h, int* status) {
     int* e = h->status_host;
     CK(cudaMemcpyAsync(e, h->s.err, sizeof(int) * kStatusWords, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    TRY(take_counts(h, 0));
+    TRY(take_scores(h, 0));
     h->unsent = 0;
     if (e[0] || e[1] || e[2] || e[3]) CK(cudaMemset(h->s.err, 0, sizeof(int) * 4));
     // after a timed-out wait the blocks' sweep counters disagree: start them again from 0
@@ -2421,8 +2420,8 @@ void admm_b200_destroy(AdmmB200* h) {
     drop_graphs(h);
     if (h->fail_host) cudaFreeHost(h->fail_host);
     if (h->status_host) cudaFreeHost(h->status_host);
-    if (h->count_host) cudaFreeHost(h->count_host);
-    for (auto e : h->count_ev)
+    if (h->score_host) cudaFreeHost(h->score_host);
+    for (auto e : h->score_ev)
         if (e) cudaEventDestroy(e);
     cudaFree(h->stage);
     for (void* p : h->allocs)
@@ -2459,7 +2458,7 @@ int admm_b200_step(AdmmB200* h, int n_steps, AdmmStepStats* stats) {
     TRY(run_substeps(h, n_steps, true));
     int status = ADMM_OK;
     TRY(read_status(h, &status));
-    if (n_steps > 0) note_counts(h, h->status_host + kPeakWord);
+    if (n_steps > 0) note_scores(h, h->status_host + kScoreWord);
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
     h->last_ms = n_steps > 0 ? ms / n_steps : 0.f;
@@ -2673,6 +2672,7 @@ int admm_b200_detect(AdmmB200* h, int* count) {
     TRY(read_status(h, &status));
     h->peak = std::max(h->peak, h->status_host[4]);
     h->detected = true;
+    if (h->status_host[5] > kOneContacts) h->calm = 0;  // a hint for the next substep
     if (count) *count = h->status_host[5];
     return status;
 }
@@ -2806,7 +2806,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     if (n != h->s.n) return fail(h, ADMM_ERR_INVALID, "n must equal n_vert");
     CK(cudaSetDevice(h->device));
     TRY(grow_stage(h, (size_t)6 * n));
-    TRY(take_counts(h, -1));
+    TRY(take_scores(h, -1));
     pick_contact_passes(h);
     TRY(build_step_graph(h));
     const size_t bytes = sizeof(float) * 3 * (size_t)n;
@@ -2820,7 +2820,7 @@ int admm_b200_step_host(AdmmB200* h, const float* x_in, const float* v_in, float
     h->frame += 1;
     int status = ADMM_OK;
     TRY(read_status(h, &status));
-    note_counts(h, h->status_host + kPeakWord);
+    note_scores(h, h->status_host + kScoreWord);
     return status;
 }
 

@@ -6,7 +6,6 @@
 
 namespace admm {
 
-constexpr int kOneContacts = 768;              // a thread per contact (85 registers each)
 constexpr int kOneVerts = 4 * kOneContacts;
 constexpr int kOneShort = 4;                   // lists of up to so many entries: a thread per vertex
 
@@ -54,8 +53,7 @@ ADMM_DEV float4 contact_short_sum(int b, int len, Entry entry, Du du) {
 }
 
 // More contacts than fit (the host then switches to a launch per pass, see pick_contact_passes):
-// the same passes in global memory, a thread per vertex with a short list, the long lists of a
-// warp's vertices four at a time.
+// the same passes in global memory.
 ADMM_DEV void contact_one_global(const DevScene& s, int nc, int passes) {
     const int lane = threadIdx.x & 31, sub = lane % kGatherLanes, grp = lane / kGatherLanes, ntv = *s.ntv;
     const unsigned gmask = 0xffu << (lane & ~(kGatherLanes - 1));
@@ -72,8 +70,21 @@ ADMM_DEV void contact_one_global(const DevScene& s, int nc, int passes) {
             s.rc[c] = f4(r.x + d.x, r.y + d.y, r.z + d.z);
         }
         __syncthreads();
-        for (int t0 = threadIdx.x - lane; t0 < ntv; t0 += blockDim.x) {
-            const int4 v = t0 + lane < ntv ? s.tvr[t0 + lane] : make_int4(0, 0, 0, 0);
+        if (ntv <= 4 * kOneContacts / kGatherLanes) {  // few turns: a group per vertex
+            for (int t = threadIdx.x / kGatherLanes; t < ntv; t += kOneContacts / kGatherLanes) {
+                const int4 v = s.tvr[t];
+                if (v.x >= s.nd) continue;  // the same in the whole group
+                const float4 a = contact_lane_sum(v.y, v.z, sub, gmask, entry, du);
+                if (sub == 0) s.p[v.x] = add3(s.p[v.x], a);
+            }
+            __syncthreads();
+            continue;
+        }
+        // a thread per vertex with a short list, the long lists of a warp's vertices four at a time
+        for (int t0 = 0; t0 < ntv; t0 += kOneContacts) {
+            // one turn: dealt out over the warps; more: consecutive vertices, read together
+            const int t = ntv <= kOneContacts ? lane * (kOneContacts / 32) + (threadIdx.x >> 5) : t0 + threadIdx.x;
+            const int4 v = t < ntv ? s.tvr[t] : make_int4(0, 0, 0, 0);
             const int len = v.x < s.nd ? v.z - v.y : 0;
             if (len > 0 && len <= kOneShort) s.p[v.x] = add3(s.p[v.x], contact_short_sum(v.y, len, entry, du));
             for (unsigned m = __ballot_sync(~0u, len > kOneShort); m;) {

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kVertThreads) k_pre_integration(DevScene s) {
     ADMM_PDL_PROLOGUE();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.n) return;
-    const int4 peaks = i == 0 ? *nc_peaks(s) : make_int4(0, 0, 0, 0);
+    const int4 score = i == 0 ? *one_score(s) : make_int4(0, 0, 0, 0);
     float4 x0 = s.x0[i], v = s.v[i], x;
     if (s.fixed[i] == 0) {
         if (i < s.nd) {
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kVertThreads) k_pre_integration(DevScene s) {
     s.x[i] = x;
     s.mxt[i] = f4(m * x.x, m * x.y, m * x.z);
     if (i >= s.nd) s.p[i] = v;
-    if (i == 0) *nc_peaks(s) = make_int4(0, peaks.x, peaks.y, peaks.z);  // a substep begins
+    if (i == 0) *one_score(s) = make_int4(0, score.x, score.y, score.z);  // a substep begins
 }
 
 // ---------------------------------------------------------------------------

@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_total(DevScene s, int nt
     ADMM_PDL_PROLOGUE();
     __shared__ int sh[32];
     __shared__ int carry;
-    const int peak = threadIdx.x == 0 ? nc_peaks(s)->x : 0;
+    const int score = threadIdx.x == 0 ? one_score(s)->x : 0;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     for (int base = 0; base < ntiles; base += kScanThreads) {
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kScanThreads) k_count_total(DevScene s, int nt
     if (threadIdx.x == 0) {
         const int raw = carry;
         *s.nc_raw = raw;
-        nc_peaks(s)->x = max(peak, raw);
+        one_score(s)->x = max(min(score + one_cost(raw), 1 << 24), -(1 << 24));
         *s.nc = raw < s.cap ? raw : s.cap;
         if (raw > s.cap) s.err[0] = 1;
         *s.ntv = 0;

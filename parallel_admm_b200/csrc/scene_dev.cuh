@@ -162,9 +162,15 @@ struct DevScene {
     int* done = nullptr;
 };
 
-// Largest unclamped contact count of the detections of each of the last four substeps, the latest
-// first: behind err among the status words.
-constexpr int kPeakWord = 8;
-__host__ __device__ inline int4* nc_peaks(const DevScene& s) { return reinterpret_cast<int4*>(s.err + kPeakWord); }
+// What the one-block contact passes (contact_one.cuh) cost over the launches in each of the last four
+// substeps, the latest first, behind err among the status words: summed over the detections, in units
+// of the 0.026 us per ADMM iteration that a contact adds to passes which do not fit the block
+// (914 contacts 4 us more than with launches, 1984 24, 3646 75, 9099 317); passes that do save some 12 us.
+constexpr int kOneContacts = 768;  // a thread per contact (85 registers each)
+__host__ __device__ inline int one_cost(int contacts) {
+    return contacts <= kOneContacts ? -460 : (contacts < 1 << 20 ? contacts : 1 << 20) - 500;
+}
+constexpr int kScoreWord = 8;
+__host__ __device__ inline int4* one_score(const DevScene& s) { return reinterpret_cast<int4*>(s.err + kScoreWord); }
 
 }  // namespace admm
