@@ -52,7 +52,8 @@ ADMM_DEV float4 contact_short_sum(int b, int len, Entry entry, Du du) {
     return add3(add3(a[0], a[2]), add3(a[1], a[3]));
 }
 
-// More contacts than fit (the host then switches to a launch per pass, see pick_contact_passes):
+// More contacts than fit (the host switches to a launch per pass where that pays, see
+// pick_contact_passes):
 // the same passes in global memory.
 ADMM_DEV void contact_one_global(const DevScene& s, int nc, int passes) {
     const int lane = threadIdx.x & 31, sub = lane % kGatherLanes, grp = lane / kGatherLanes, ntv = *s.ntv;

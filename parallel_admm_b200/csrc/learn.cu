@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kT) k_t_collect(TrainMat M, const double* __re
 }
 
 // ---- conjugate gradients (diag(A) preconditioned) for the converged solution ----
-// Two launches per iteration, the scalars on the device: every block of a kernel sums the
+// Two launches per iteration (three above kFusedRows rows), the scalars on the device: every block of a kernel sums the
 // partials that the kernel before it left.  Once the iteration has ended (done), the kernels
 // still queued do nothing.  The kernels start before their predecessor has ended (programmatic
 // launch) and load what does not change, the matrix and its diagonal, before they wait for it: at
